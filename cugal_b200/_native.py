@@ -38,7 +38,8 @@ class SolveParams(ctypes.Structure):
         ("stream_dtype", c_int), ("max_iterations", c_int), ("threshold", c_double), ("eval_freq", c_int),
         ("momentum_start", c_int), ("fp32_warmup_sweeps", c_int), ("reabsorb_every", c_int),
         ("polish_sweeps", c_int), ("u_out", c_void_p), ("v_out", c_void_p), ("record", c_void_p),
-        ("column_partials", c_void_p), ("column_partial_chunks", ctypes.c_int32), ("column_partial_ld", c_int64),
+        ("column_partials", c_void_p), ("column_partial_chunks", ctypes.c_int32),
+        ("fixed_order", ctypes.c_int32), ("column_partial_ld", c_int64),
     ]
 
 

@@ -96,6 +96,9 @@ class SinkhornPlan(torch.autograd.Function):
     def forward(ctx, C, config, tol, max_iter):
         n = C.shape[0]
         state = SinkhornState(n, config)
+        # the adjoint of a nearly integral plan amplifies the plan's last bits (up to 1e-3 of
+        # dC between two equally exact plans), so its sums keep one order
+        state._solver.fixed_order = True
         state.solve(C.detach().to(torch.float32).contiguous(), config)
         P = state.plan()
         ctx.save_for_backward(P)

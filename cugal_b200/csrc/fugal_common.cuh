@@ -171,15 +171,29 @@ FUGAL_DEVICE bool mbar_try_wait(uint64_t* bar, uint32_t parity, uint32_t hint_ns
         : "memory");
     return ok != 0;
 }
+// The same with CTA scope: for barriers that only this CTA and its bulk copies signal.
+FUGAL_DEVICE bool mbar_try_wait_cta(uint64_t* bar, uint32_t parity, uint32_t hint_ns) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n"
+        " mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2, %3;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(smem_addr(bar)), "r"(parity), "r"(hint_ns)
+        : "memory");
+    return ok != 0;
+}
 // Bounded wait: returns false (and records FUGAL_DEVICE_TIMEOUT) if the phase
-// does not complete within limit_ns (0: kWaitLimitNs).
+// does not complete within limit_ns (0: kWaitLimitNs).  CTA: mbar_try_wait_cta.
+template <bool CTA = false>
 FUGAL_DEVICE bool mbar_wait(uint64_t* bar, uint32_t parity, int* err, uint32_t hint_ns = kSuspendHintNs,
                             uint64_t limit_ns = 0) {
-    if (mbar_try_wait(bar, parity, hint_ns)) return true;
+    auto probe = [&]() { return CTA ? mbar_try_wait_cta(bar, parity, hint_ns) : mbar_try_wait(bar, parity, hint_ns); };
+    if (probe()) return true;
     const uint64_t limit = limit_ns != 0 ? limit_ns : kWaitLimitNs;
     const uint64_t t0 = global_timer_ns();
     for (uint32_t i = 0; i < kMaxPolls; ++i) {
-        if (mbar_try_wait(bar, parity, hint_ns)) return true;
+        if (probe()) return true;
         if (global_timer_ns() - t0 > limit) break;
     }
     report_error(err, FUGAL_DEVICE_TIMEOUT);
@@ -292,44 +306,6 @@ FUGAL_DEVICE void tmem_ld16(uint32_t taddr, float* v) {
         : "memory");
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// Warp-wide: lane i of the warp stores v[0..31] into TMEM lane (lane base + i),
-// columns [col, col + 32) of `taddr` (lane base in bits 31..16, column in 15..0;
-// the warp's lane base is 32 x (warp index mod 4)).
-FUGAL_DEVICE void tmem_st32(uint32_t taddr, const float* v) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-        "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-        "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
-        "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
-        "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])), "r"(__float_as_uint(v[8])),
-        "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
-        "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])),
-        "r"(__float_as_uint(v[15])), "r"(__float_as_uint(v[16])), "r"(__float_as_uint(v[17])),
-        "r"(__float_as_uint(v[18])), "r"(__float_as_uint(v[19])), "r"(__float_as_uint(v[20])),
-        "r"(__float_as_uint(v[21])), "r"(__float_as_uint(v[22])), "r"(__float_as_uint(v[23])),
-        "r"(__float_as_uint(v[24])), "r"(__float_as_uint(v[25])), "r"(__float_as_uint(v[26])),
-        "r"(__float_as_uint(v[27])), "r"(__float_as_uint(v[28])), "r"(__float_as_uint(v[29])),
-        "r"(__float_as_uint(v[30])), "r"(__float_as_uint(v[31]))
-        : "memory");
-}
-// Warp-wide load of the same layout.  The wait for the load is part of the same
-// asm statement, so the registers are valid when it returns.
-FUGAL_DEVICE void tmem_ld32(uint32_t taddr, float* v) {
-    uint32_t r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-        "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 }  // namespace fugal

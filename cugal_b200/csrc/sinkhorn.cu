@@ -21,18 +21,21 @@
 // of per-panel column (max, sum) partials, which the gradient writes with the
 // cost (column_partials) or a pass over the cost computes (column_pass_kernel).
 //
-// Two sweep kernels share this structure.
-//   sweep_kernel (FP32 sweeps, the absorb sweep, and 16-bit sweeps wider than
-//   32768 columns): each cluster of C CTAs owns a contiguous block of rows; CTA
-//   k of the cluster owns column slice k.  Row slices stream HBM -> shared
-//   memory with 1-D bulk copies (cp.async.bulk + mbarrier, several stages in
-//   flight); the per-row (max, sum) partials of the C CTAs are exchanged through
-//   distributed shared memory (remote stores + remote mbarrier arrives,
-//   double-buffered).  Every thread keeps its 16 or 32 columns' running column
-//   sums in registers, so the only global writes are one partial row per cluster.
-//   row_sweep_kernel (16-bit sweeps up to 32768 columns): one 512-thread CTA per
-//   SM owns whole rows, the row normaliser is a CTA barrier, the column sums
-//   live in tensor memory (TMEM); see its own comment below.
+// Three sweep kernels share this structure.
+//   rows_kernel (sinkhorn_rows.cu; FP32 sweeps up to 8192 columns, 16-bit sweeps up
+//   to 24576): one persistent CTA per SM owns whole rows and runs many sweeps in one
+//   launch, the finalize step included.
+//   sweep_kernel (wider FP32 sweeps, the absorb sweep, solves with a fixed order of
+//   sums): each cluster of C CTAs owns a contiguous block of rows; CTA k of the
+//   cluster owns column slice k.  Row slices stream HBM -> shared memory with 1-D
+//   bulk copies (cp.async.bulk + mbarrier, several stages in flight); the per-row
+//   (max, sum) partials of the C CTAs are exchanged through distributed shared memory
+//   (remote stores + remote mbarrier arrives, double-buffered).  Every thread keeps
+//   its 16 or 32 columns' running column sums in registers, so the only global writes
+//   are one partial row per cluster.
+//   row_sweep_kernel (16-bit sweeps of 24577 to 65536 columns): one 512-thread CTA per
+//   SM, or a cluster of two, owns whole rows, the row normaliser is a CTA barrier, the
+//   column sums live in tensor memory (TMEM); see its own comment below.
 //
 // Precision: the cost arrives "absorbed" (cost32 = K + U_i + V_j with the
 // previous solves' duals U, V folded in), so its entries are ~log P and the
@@ -55,75 +58,13 @@
 
 #include "fugal_common.cuh"
 #include "fugal_host.h"
+#include "sinkhorn_rows.h"
+#include "sinkhorn_state.cuh"
 
 namespace fugal {
 
 constexpr int kMaxStages = 8;
 constexpr int kMaxCluster = 16;
-
-struct SolveState {
-    int it;          // index of the next sweep
-    int done;        // set when the current phase has finished
-    int final_it;    // index of the last sweep of the current phase
-    int n_err;
-    unsigned int ticket;
-    int status;      // device-side error code (bounded waits)
-    int max_it;      // phase ends after sweep max_it - 1
-    int check;       // 1: main phase (convergence checks), 0: polish
-    int eval_freq;
-    int momentum_start;
-    int main_final_it;
-    int main_n_err;
-    int polish_count;
-    int exact_next;  // 1: the next sweep reduces rows with the exact (two-barrier) path
-    float max_corr;  // max |log colsum| of the current sweep (as float bits, atomicMax)
-    int pad1;
-    double threshold;
-    double omega;
-    double err_accum;
-    double last_err;
-    double main_last_err;
-    double polish_err;
-    double errors[FUGAL_MAX_RECORDED_ERRORS];
-};
-
-// ------------------------------------------------------------------ device
-
-__device__ double lehmann_momentum(const SolveState* st) {
-    return lehmann_omega(st->errors, st->n_err, st->eval_freq, st->momentum_start);
-}
-
-// End-of-sweep decision (single thread).
-__device__ void decide(SolveState* st, double err) {
-    const int t = st->it;
-    st->last_err = err;
-    bool stop = false;
-    if (st->check) {
-        if (t % st->eval_freq == 0 && t != 0) {
-            if (st->n_err < FUGAL_MAX_RECORDED_ERRORS) st->errors[st->n_err] = err;
-            st->n_err += 1;
-            if (err < st->threshold)
-                stop = true;
-            else
-                st->omega = lehmann_momentum(st);
-        }
-    } else {
-        st->polish_err = err;
-        st->polish_count += 1;
-    }
-    if (!stop && t + 1 >= st->max_it) stop = true;
-    if (st->status != 0) stop = true;  // a bounded wait timed out: end the phase
-    if (stop) {
-        st->done = 1;
-        st->final_it = t;
-        if (st->check) {
-            st->main_final_it = t;
-            st->main_n_err = st->n_err;
-            st->main_last_err = err;
-        }
-    }
-    st->it = t + 1;
-}
 
 struct SweepArgs {
     const void* L;        // cost (element type T), n x ld
@@ -151,10 +92,6 @@ struct SweepArgs {
 };
 
 constexpr int kBarBytes = 128;
-
-// Largest |column correction| (nats) after which the next sweep uses the exact
-// (max-stabilised) row reduction instead of the previous row normaliser.
-constexpr float kFastPathLimit = 30.0f;
 
 // Sum (or max) of one value per lane, the same in every lane.  The sum is lane
 // 0's butterfly result broadcast: every warp that reduces the same inputs then
@@ -226,70 +163,13 @@ __device__ __forceinline__ float slot_sum(const float2* xch, int slot, int C, in
     return lanes_sum(v);
 }
 
-// One 16-byte chunk of T as float pairs (elements 2q, 2q+1 in .x, .y).
-template <typename T> struct Pairs;
-template <> struct Pairs<float> {
-    FUGAL_DEVICE static void unpack(const uint4& r, float2* o) {
-        o[0] = make_float2(__uint_as_float(r.x), __uint_as_float(r.y));
-        o[1] = make_float2(__uint_as_float(r.z), __uint_as_float(r.w));
-    }
-};
-template <> struct Pairs<__nv_bfloat16> {
-    FUGAL_DEVICE static void unpack(const uint4& r, float2* o) {
-        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) o[i] = make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
-    }
-};
-template <> struct Pairs<__half> {
-    FUGAL_DEVICE static void unpack(const uint4& r, float2* o) {
-        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) o[i] = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-    }
-};
-
-FUGAL_DEVICE float2 ex2_pair(float2 x) { return make_float2(ex2(x.x), ex2(x.y)); }
-
-// 2^x for two lanes on the FMA pipe instead of MUFU (Cody-Waite style
-// reduction): k = round(x) by the 1.5 * 2^23 rounding constant, f = x - k in
-// [-1/2, 1/2], 2^f by a degree-6 polynomial, and k added to the result's
-// exponent bits.  The coefficients were fitted for this file by Lawson's
-// iteratively reweighted least squares, minimising the relative error on
-// [-1/2, 1/2]: 1.9e-9 in exact arithmetic, under 8e-8 (about 1 ulp) with FP32
-// Horner steps -- no worse than ex2.approx.  x is clamped to [-127, 127] (so a
-// huge x still gives a huge finite value) and x < -126 gives 0, as
-// ex2.approx.ftz flushes results below 2^-126; -inf gives 0.
-FUGAL_DEVICE float2 ex2_poly_pair(float2 x) {
-    const float2 xc = make_float2(fminf(fmaxf(x.x, -127.f), 127.f), fminf(fmaxf(x.y, -127.f), 127.f));
-    const float2 rnd = make_float2(12582912.f, 12582912.f);  // 1.5 * 2^23
-    const float2 t = __fadd2_rn(xc, rnd);                     // rnd + round(x)
-    const float2 k = __fadd2_rn(t, make_float2(-12582912.f, -12582912.f));
-    const float2 f = __ffma2_rn(k, make_float2(-1.f, -1.f), xc);  // x - k, exact
-    float2 q = make_float2(1.534581242594868e-4f, 1.534581242594868e-4f);
-    q = __ffma2_rn(q, f, make_float2(1.3399930903688073e-3f, 1.3399930903688073e-3f));
-    q = __ffma2_rn(q, f, make_float2(9.618489071726799e-3f, 9.618489071726799e-3f));
-    q = __ffma2_rn(q, f, make_float2(5.550328642129898e-2f, 5.550328642129898e-2f));
-    q = __ffma2_rn(q, f, make_float2(2.4022646248340607e-1f, 2.4022646248340607e-1f));
-    q = __ffma2_rn(q, f, make_float2(6.931471824645996e-1f, 6.931471824645996e-1f));
-    q = __ffma2_rn(q, f, make_float2(1.f, 1.f));
-    // the bits of t are those of rnd plus round(x); rnd's low 9 bits are 0, so
-    // (bits(t) << 23) is round(x) << 23 modulo 2^32: round(x) added to the exponent
-    float2 y;
-    y.x = __int_as_float(__float_as_int(q.x) + (__float_as_int(t.x) << 23));
-    y.y = __int_as_float(__float_as_int(q.y) + (__float_as_int(t.y) << 23));
-    if (x.x < -126.f) y.x = 0.f;
-    if (x.y < -126.f) y.y = 0.f;
-    return y;
-}
-
 // Sweep kernel.  Each thread owns KPT columns of its CTA's slice as KPT/2
 // float pairs and processes R rows per batch; the hot loop runs on Blackwell's
 // packed FP32x2 FMA/ADD (fma.rn.f32x2) with the exponentials on MUFU ex2, in
-// base-2 units (b_s holds the column duals times log2 e).  At most 128
-// registers per thread so two 256-thread CTAs share an SM.
+// base-2 units (b_s holds the column duals times log2 e).  Two CTAs share an SM
+// (at most 128 registers per thread at 256 threads).
 template <typename T, int THREADS, int KPT, int R, bool ABSORB, typename TOUT>
-__global__ void __launch_bounds__(THREADS, (THREADS >= 512 ? 1 : 512 / THREADS)) sweep_kernel(const SweepArgs p) {
+__global__ void __launch_bounds__(THREADS, 2) sweep_kernel(const SweepArgs p) {
     constexpr int V = Vec<T>::N;  // elements per 16-byte chunk
     constexpr int G = KPT / V;    // chunks per thread per row
     constexpr int VP = V / 2;     // pairs per chunk
@@ -663,9 +543,10 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 512 ? 1 : 512 / THREADS))
 }
 
 // ---------------------------------------------------------------------------
-// Row-owned 16-bit sweep (n <= 32768): one 512-thread CTA per SM walks a block
-// of whole rows, so the row normaliser is a CTA barrier instead of a cluster
-// exchange, and each thread keeps the running column sums of its EPT columns
+// Row-owned 16-bit sweep (24576 < n <= 32768, or two CTAs up to 65536): one
+// 512-thread CTA per SM walks a block of whole rows, so the row normaliser is a CTA
+// barrier instead of a cluster exchange, and each thread keeps the running column sums
+// of its 64 columns
 // in tensor memory (TMEM lane 32 (warp % 4) + lane, columns (warp / 4) EPT ..).
 // Rows stream through shared memory in segments of up to 16384 elements
 // (32 KB) with bulk copies.  The column duals (b log2 e) of the thread's
@@ -746,7 +627,6 @@ __global__ void __launch_bounds__(THREADS, 1) row_sweep_kernel(const RowArgs p) 
     __shared__ __align__(8) float2 xs[2];
     __shared__ __align__(16) float red_s[2][kRowWarps];
     __shared__ __align__(16) float red_m[2][kRowWarps];
-    __shared__ __align__(16) float red_grp[2][4][kRowWarps];
     __shared__ uint32_t tmem_slot;
 
     SolveState* st = p.st;
@@ -978,78 +858,6 @@ __global__ void __launch_bounds__(THREADS, 1) row_sweep_kernel(const RowArgs p) 
 
     bool alive = true;
     int r = 0;
-    // Rows in groups of RB = 64 / EPT (one-segment rows, fast path): the group's
-    // exponentials stay in registers, so its rows share one barrier, one read of
-    // the per-warp sums and one pass over the TMEM accumulators.  A group with a
-    // row outside the fast path's range hands the rest of the sweep to the
-    // single-row loop below, which restarts at that group (stages still held).
-    if constexpr (CL == 1 && NSEG == 1 && EPT <= 32) {
-        constexpr int RB = 64 / EPT;  // 2 or 4
-        if (!exact_only) {
-            for (; r < nrows; r += RB) {
-                const int nr = min(RB, nrows - r);
-                const int par = (r / RB) & 1;
-                bool ok = true;
-                float2 yg[RB][H];
-                float part[RB];
-#pragma unroll
-                for (int k = 0; k < RB; ++k) {
-                    float2 sa = make_float2(0.f, 0.f), ta = sa;
-                    if (k < nr) {
-                        row_fast(next_rows(cur, k), yg[k], sa, ta, ok);
-                    } else {
-#pragma unroll
-                        for (int h = 0; h < H; ++h) yg[k][h] = make_float2(0.f, 0.f);
-                    }
-                    const float2 ua = __fadd2_rn(sa, ta);
-                    part[k] = ua.x + ua.y;
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-                    for (int k = 0; k < RB; ++k) part[k] += __shfl_xor_sync(0xffffffffu, part[k], o);
-                }
-                if (lane == 0) {
-#pragma unroll
-                    for (int k = 0; k < RB; ++k) red_grp[par][k][warp] = part[k];
-                }
-                if (!__syncthreads_and(ok)) {
-                    alive = false;
-                    break;
-                }
-                float S[RB], wk[RB];
-                bool in_range = true;
-#pragma unroll
-                for (int k = 0; k < RB; ++k) {
-                    S[k] = sum16(red_grp[par][k]);
-                    if (k < nr && !(S[k] > 1e-30f && S[k] < 1e30f)) in_range = false;
-                }
-                if (!in_range) break;  // uniform
-#pragma unroll
-                for (int k = 0; k < RB; ++k) {
-                    if (k < nr) release(r + k, next_rows(cur, k));
-                    wk[k] = k < nr ? __frcp_rn(S[k]) : 0.f;
-                    if (tid == 0 && k < nr) p.a[row_begin + r + k] = -__log2f(S[k]) * kLn2;
-                }
-#pragma unroll
-                for (int c = 0; c < EPT / 16; ++c) {
-                    float acc[16];
-                    tmem_ld16(tcol + 16 * c, acc);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        float2 a2 = make_float2(acc[2 * q], acc[2 * q + 1]);
-#pragma unroll
-                        for (int k = 0; k < RB; ++k) a2 = __ffma2_rn(yg[k][8 * c + q], make_float2(wk[k], wk[k]), a2);
-                        acc[2 * q] = a2.x;
-                        acc[2 * q + 1] = a2.y;
-                    }
-                    tmem_st16(tcol + 16 * c, acc);
-                }
-                cur = next_rows(cur, nr);
-            }
-        }
-    }
-    if (alive)
     for (; r < nrows; ++r) {
         const int row = row_begin + r;
         const int par = r & 1;
@@ -1207,43 +1015,50 @@ __global__ void __launch_bounds__(THREADS, 1) row_sweep_kernel(const RowArgs p) 
 }
 
 // Reduce the per-cluster column sums (FP64), write log(colsum), decide.
-// Block: 8 warps x 32 lanes; lanes own 4 consecutive columns each (128 per
-// block), warps split the partial rows; one FP64 error sum and one maximum
-// |column correction| per block go to the solve state by atomics.
+// Block: 8 warps x 32 lanes, one column per lane; warps split the partial rows, up
+// to 12 loads in flight per lane (a chain of dependent loads was most of this
+// kernel: 9.1 us at n = 4096 on 293 partial rows with 4 columns per lane and 32
+// blocks).  One FP64 error sum and one maximum |column correction| per block go to
+// the solve state by atomics.
 constexpr int kFinThreads = 256;
-constexpr int kFinCols = 128;
+constexpr int kFinCols = 32;
 
 __global__ void __launch_bounds__(kFinThreads) finalize_kernel(const float* partials, int nparts, long long n_pad,
                                                                int n, float* logcs, SolveState* st) {
-    __shared__ double part[kFinThreads / 32][kFinCols];
+    constexpr int kWarps = kFinThreads / 32;
+    constexpr int U = 12;
+    __shared__ double part[kWarps][kFinCols];
     __shared__ double red[32];
-    __shared__ float red_corr[kFinThreads / 32];
+    __shared__ float red_corr[kWarps];
     if (*reinterpret_cast<volatile int*>(&st->done)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int j0 = blockIdx.x * kFinCols + lane * 4;
-    double cs[4] = {0.0, 0.0, 0.0, 0.0};
-    if (j0 < n) {
-        for (int c = warp; c < nparts; c += kFinThreads / 32) {
-            const float4 v = *reinterpret_cast<const float4*>(partials + static_cast<size_t>(c) * n_pad + j0);
-            cs[0] += v.x; cs[1] += v.y; cs[2] += v.z; cs[3] += v.w;
+    const int j = blockIdx.x * kFinCols + lane;
+    double cs = 0.0;
+    if (j < n) {
+        for (int c0 = warp; c0 < nparts; c0 += U * kWarps) {
+            float v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int c = c0 + u * kWarps;
+                v[u] = c < nparts ? partials[static_cast<size_t>(c) * n_pad + j] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (c0 + u * kWarps < nparts) cs += static_cast<double>(v[u]);
         }
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) part[warp][lane * 4 + q] = cs[q];
+    part[warp][lane] = cs;
     __syncthreads();
     double err = 0.0;
     float corr = 0.f;
-    if (threadIdx.x < kFinCols) {
-        const int j = blockIdx.x * kFinCols + threadIdx.x;
-        if (j < n) {
-            double tot = 0.0;
+    if (warp == 0 && j < n) {
+        double tot = 0.0;
 #pragma unroll
-            for (int w = 0; w < kFinThreads / 32; ++w) tot += part[w][threadIdx.x];
-            err = fabs(tot - 1.0);
-            const float lg = static_cast<float>(log(fmax(tot, 1e-37)));
-            logcs[j] = lg;
-            corr = fabsf(lg);
-        }
+        for (int w = 0; w < kWarps; ++w) tot += part[w][lane];
+        err = fabs(tot - 1.0);
+        const float lg = static_cast<float>(log(fmax(tot, 1e-37)));
+        logcs[j] = lg;
+        corr = fabsf(lg);
     }
     corr = warp_max(corr);
     if (lane == 0) red_corr[warp] = corr;
@@ -1361,6 +1176,7 @@ __global__ void __launch_bounds__(256) column_merge_kernel(const float2* part, i
         st->polish_count = 0;
         st->exact_next = 1;
         st->max_corr = 0.f;
+        st->arrivals = 0;
         st->threshold = ia.threshold;
         st->omega = 1.0;
         st->err_accum = 0.0;
@@ -1492,15 +1308,18 @@ unsigned suspend_hint() {
     return static_cast<unsigned>(v < 0 ? 0 : (v > 1000000 ? 1000000 : v));
 }
 
-// Launch shapes: (threads per CTA, columns per thread).  Rows per batch are
-// 32 / columns-per-thread, so a thread always holds 32 exponentials.
-constexpr int rows_per_batch(int kpt) { return 32 / kpt; }
+// Launch shapes: (threads per CTA, columns per thread).  Rows per batch: 32
+// exponentials a thread at 256 threads; 64 (32 KB of FP32 rows a stage) at 128
+// threads, where two CTAs on an SM are too few warps to hide a batch's exchange and
+// registers are left over.  The rows of a batch do not touch each other, so results
+// do not depend on it.
+constexpr int rows_per_batch(int threads, int kpt) { return (threads == 128 ? 64 : 32) / kpt; }
 
 using KernelFn = void (*)(const SweepArgs);
 
 template <typename T, int THREADS, int KPT, bool ABSORB, typename TOUT>
 KernelFn pick_kernel() {
-    return sweep_kernel<T, THREADS, KPT, rows_per_batch(KPT), ABSORB, TOUT>;
+    return sweep_kernel<T, THREADS, KPT, rows_per_batch(THREADS, KPT), ABSORB, TOUT>;
 }
 
 // kind: 0 = plain sweep over dtype dt, 1 = absorb (fp32 -> bf16), 2 = absorb (fp32 -> fp16)
@@ -1519,7 +1338,7 @@ KernelFn kernel_for(int threads, int kpt, int dt, int kind) {
 }
 
 int header_for(int threads, int R) {
-    if (threads == 128) return R == 2 ? header_bytes_v3<128, 2>() : header_bytes_v3<128, 1>();
+    if (threads == 128) return R == 4 ? header_bytes_v3<128, 4>() : header_bytes_v3<128, 2>();
     return R == 2 ? header_bytes_v3<256, 2>() : header_bytes_v3<256, 1>();
 }
 
@@ -1575,7 +1394,7 @@ constexpr int kSmemTarget = 100 * 1024;
 fugal_status make_plan(int64_t n, int dt, int kind, SweepPlan& pl, bool query_occupancy) {
     FUGAL_TRY(plan_shape(n, pl.threads, pl.kpt, pl.cluster));
     const int es = (kind != 0) ? 4 : elem_size(dt);
-    pl.R = rows_per_batch(pl.kpt);
+    pl.R = rows_per_batch(pl.threads, pl.kpt);
     pl.slice_w = pl.threads * pl.kpt;
     const size_t stage_bytes = static_cast<size_t>(pl.R) * pl.slice_w * es;
     const int sms = sm_count();
@@ -1623,7 +1442,8 @@ fugal_status make_plan(int64_t n, int dt, int kind, SweepPlan& pl, bool query_oc
                 return fail(FUGAL_UNSUPPORTED, "sinkhorn: cluster of %d CTAs cannot be scheduled", pl.cluster);
             clusters = active;
         }
-        const int max_useful = static_cast<int>((n + pl.R - 1) / pl.R);
+        const int min_rows = 32 / pl.kpt;  // rows a cluster should have at least
+        const int max_useful = static_cast<int>((n + min_rows - 1) / min_rows);
         clusters = std::max(1, std::min(clusters, max_useful));
         pl.clusters = clusters;
         pl.rows_per_cluster = static_cast<int>((n + clusters - 1) / clusters);
@@ -1656,8 +1476,7 @@ using RowKernelFn = void (*)(const RowArgs);
 template <typename T, bool BT, int POLY>
 RowKernelFn row_kernel_typed(int ept, int cl) {
     if (cl == 2) return row_sweep_kernel<T, 64, 512, BT, POLY, (BT ? 2 : 1)>;
-    return ept == 16 ? row_sweep_kernel<T, 16, 512, BT, POLY, 1>
-                     : (ept == 32 ? row_sweep_kernel<T, 32, 512, BT, POLY, 1> : row_sweep_kernel<T, 64, 512, BT, POLY, 1>);
+    return row_sweep_kernel<T, 64, 512, BT, POLY, 1>;
 }
 
 template <typename T>
@@ -1710,19 +1529,21 @@ bool row_duals_in_tmem() {
 // made it slower.)
 int row_threads_for(int64_t) { return 512; }
 
+// Row-owned 16-bit sweeps (default); FUGAL_ROW_SWEEP=0 selects the cluster kernel.
+bool row_sweep_on() {
+    const char* e = getenv("FUGAL_ROW_SWEEP");
+    return !(e != nullptr && atoi(e) == 0);
+}
+
 fugal_status make_row_plan(int64_t n, int dt, int64_t n_pad, RowPlan& rp, bool set_attributes) {
     rp = RowPlan{};
     if (dt == FUGAL_F32) return FUGAL_OK;
-    const char* e = getenv("FUGAL_ROW_SWEEP");
-    if (e != nullptr && atoi(e) == 0) return FUGAL_OK;
     rp.bt = row_duals_in_tmem();
     // rows up to 32768 columns: one CTA; up to 65536: a cluster of two (duals in TMEM)
     if (n_pad > (rp.bt ? 65536 : 32768)) return FUGAL_OK;
     rp.threads = row_threads_for(n_pad);
     rp.cl = n_pad > 32768 ? 2 : 1;
-    const int64_t per_cta = (n_pad + rp.cl - 1) / rp.cl;
-    rp.ept = static_cast<int>((per_cta + rp.threads * 16 - 1) / (rp.threads * 16)) * 16;  // 16, 32 or 64
-    if (rp.ept == 48) rp.ept = 64;
+    rp.ept = 64;  // narrower rows take the persistent kernel (sinkhorn_rows.cu)
     const size_t stage_bytes = static_cast<size_t>(rp.threads) * std::min(rp.ept, kRowSeg / rp.threads) * 2;
     rp.poly = rp.bt ? row_poly() : 0;
     // column duals of every covered column, unless they live in TMEM
@@ -1774,10 +1595,13 @@ struct Workspace {
     SolveState* st;
     float* b_buf;     // [2][n_pad]
     float* logcs;     // [n_pad]
+    float* b_next;    // [n_pad]
     float* a;         // [n_pad]
     float* a_snap;    // [2][n_pad]
     float* b_snap;    // [2][n_pad]
     float* partials;  // [max(sweep clusters, 2*column chunks)][n_pad]
+    double* errs;     // [SMs] column errors of the row-owned sweeps' CTAs
+    float* corrs;     // [SMs] their largest corrections
     long long n_pad;
     size_t bytes;
 };
@@ -1796,10 +1620,13 @@ Workspace layout(int64_t n, char* base, int partial_rows) {
     w.st = reinterpret_cast<SolveState*>(take(sizeof(SolveState)));
     w.b_buf = reinterpret_cast<float*>(take(2 * w.n_pad * 4));
     w.logcs = reinterpret_cast<float*>(take(w.n_pad * 4));
+    w.b_next = reinterpret_cast<float*>(take(w.n_pad * 4));
     w.a = reinterpret_cast<float*>(take(w.n_pad * 4));
     w.a_snap = reinterpret_cast<float*>(take(2 * w.n_pad * 4));
     w.b_snap = reinterpret_cast<float*>(take(2 * w.n_pad * 4));
     w.partials = reinterpret_cast<float*>(take(static_cast<size_t>(partial_rows) * w.n_pad * 4));
+    w.errs = reinterpret_cast<double*>(take(static_cast<size_t>(sm_count()) * 8));
+    w.corrs = reinterpret_cast<float*>(take(static_cast<size_t>(sm_count()) * 4));
     w.bytes = off;
     return w;
 }
@@ -1858,8 +1685,22 @@ extern "C" fugal_status fugal_sinkhorn_plan_info(int64_t n, int stream_dtype, in
     if (info == nullptr) return fail(FUGAL_BAD_ARGUMENT, "fugal_sinkhorn_plan_info: null output");
     if (stream_dtype < FUGAL_F32 || stream_dtype > FUGAL_F16)
         return fail(FUGAL_BAD_ARGUMENT, "fugal_sinkhorn_plan_info: bad stream dtype");
+    if (stream_dtype == FUGAL_F32 ? getenv("FUGAL_SWEEP_SHAPE") == nullptr : row_sweep_on()) {
+        RowsPlan rows;
+        FUGAL_TRY(make_rows_plan(n, stream_dtype, rows, false));
+        if (rows.use) {  // row-owned persistent sweeps: one CTA per SM, no cluster
+            info[0] = 512;
+            info[1] = 1;
+            info[2] = rows.ctas;
+            info[3] = rows.stages;
+            info[4] = static_cast<int32_t>(rows.smem);
+            info[5] = rows.streams;
+            return FUGAL_OK;
+        }
+    }
     RowPlan rp;
-    FUGAL_TRY(make_row_plan(n, stream_dtype, static_cast<int64_t>(align_up(static_cast<size_t>(n), 64)), rp, false));
+    if (row_sweep_on())
+        FUGAL_TRY(make_row_plan(n, stream_dtype, static_cast<int64_t>(align_up(static_cast<size_t>(n), 64)), rp, false));
     if (rp.use) {  // row-owned sweep: one CTA per SM, no cluster
         info[0] = rp.threads;
         info[1] = rp.cl;
@@ -1916,14 +1757,20 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
 
     SweepPlan plan32{}, plan16{}, plan_abs{};
     RowPlan rowplan;
-    FUGAL_TRY(make_plan(n, FUGAL_F32, 0, plan32, true));
-    if (use16) FUGAL_TRY(make_row_plan(n, p.stream_dtype, w.n_pad, rowplan, true));
+    RowsPlan rows32, rows16;
+    const char* shape = getenv("FUGAL_SWEEP_SHAPE");
+    if (shape == nullptr && !p.fixed_order) FUGAL_TRY(make_rows_plan(n, FUGAL_F32, rows32, true));
+    if (!rows32.use) FUGAL_TRY(make_plan(n, FUGAL_F32, 0, plan32, true));
+    if (use16 && row_sweep_on() && !p.fixed_order) {
+        FUGAL_TRY(make_rows_plan(n, p.stream_dtype, rows16, true));
+        if (!rows16.use) FUGAL_TRY(make_row_plan(n, p.stream_dtype, w.n_pad, rowplan, true));
+    }
     if (use16) {
-        if (!rowplan.use) FUGAL_TRY(make_plan(n, p.stream_dtype, 0, plan16, true));
+        if (!rows16.use && !rowplan.use) FUGAL_TRY(make_plan(n, p.stream_dtype, 0, plan16, true));
         FUGAL_TRY(make_plan(n, FUGAL_F32, p.stream_dtype == FUGAL_BF16 ? 1 : 2, plan_abs, true));
     }
     if (plan32.clusters > prow || (use16 && (plan16.clusters > prow || plan_abs.clusters > prow)) ||
-        rowplan.groups > prow)
+        rowplan.groups > prow || rows32.parts > prow || rows16.parts > prow)
         return fail(FUGAL_UNSUPPORTED, "fugal_sinkhorn_solve: more clusters than partial rows");
 
     FrameArgs frame{use16 ? 1 : 0, use16 ? p.fp32_warmup_sweeps : 0, use16 ? p.reabsorb_every : 1,
@@ -1982,6 +1829,28 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
         a.st = w.st;
         return a;
     };
+    auto rows_args = [&](int dt, int sweeps) {
+        RowsArgs ra{};
+        ra.L = dt == FUGAL_F32 ? static_cast<const void*>(p.cost32) : p.cost16;
+        ra.ld = dt == FUGAL_F32 ? p.ld32 : p.ld16;
+        ra.n = static_cast<int>(n);
+        const int V = 16 / elem_size(dt);
+        ra.n_copy = static_cast<int>((n + V - 1) / V * V);
+        ra.sweeps = sweeps;
+        ra.suspend_ns = suspend_hint();
+        ra.b_buf = w.b_buf;
+        ra.logcs = w.logcs;
+        ra.b_next = w.b_next;
+        ra.a = w.a;
+        ra.partials = w.partials;
+        ra.errs = w.errs;
+        ra.corrs = w.corrs;
+        ra.n_pad = w.n_pad;
+        ra.st = w.st;
+        ra.wait_limit_ns = test_wait_limit_ns();
+        ra.fault_row = dt == FUGAL_F32 ? -1 : test_fault_row();
+        return ra;
+    };
     const int fin_grid = static_cast<int>((n + kFinCols - 1) / kFinCols);
     auto finalize = [&](int nparts) -> fugal_status {
         LaunchScope scope(FUGAL_KERNEL_FINALIZE, stream);
@@ -2016,10 +1885,18 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
         poll_slot = -1;
         return s;
     };
-    for (int t = 0; t < p.max_iterations && status == FUGAL_OK; ++t) {
+    // One step of this loop is one sweep, or a launch of the row-owned kernel that runs
+    // all sweeps up to the next change of kind (`len` of them).
+    int len = 1;
+    for (int t = 0; t < p.max_iterations && status == FUGAL_OK; t += len) {
+        len = 1;
         const int snap_idx = (!use16 || t < p.fp32_warmup_sweeps) ? -1 : ((t - p.fp32_warmup_sweeps) / p.reabsorb_every);
         const bool absorb = use16 && t >= p.fp32_warmup_sweeps && (t - p.fp32_warmup_sweeps) % p.reabsorb_every == 0;
-        if (!use16 || t < p.fp32_warmup_sweeps) {
+        if (rows32.use && (!use16 || t < p.fp32_warmup_sweeps)) {
+            len = (use16 ? std::min(p.max_iterations, p.fp32_warmup_sweeps) : p.max_iterations) - t;
+            len = std::min(len, kRowsMaxSweeps);
+            status = launch_rows(rows32, rows_args(FUGAL_F32, len), stream, FUGAL_KERNEL_SWEEP_F32);
+        } else if (!use16 || t < p.fp32_warmup_sweeps) {
             SweepArgs a = sweep_args(plan32, p.cost32, p.ld32, nullptr, nullptr);
             status = launch_sweep(plan32, kernel_for(plan32.threads, plan32.kpt, FUGAL_F32, 0), a, stream, FUGAL_KERNEL_SWEEP_F32);
             if (status == FUGAL_OK) status = finalize(plan32.clusters);
@@ -2035,6 +1912,10 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
             status = launch_sweep(plan_abs, kernel_for(plan_abs.threads, plan_abs.kpt, FUGAL_F32, p.stream_dtype == FUGAL_BF16 ? 1 : 2),
                                   a, stream, FUGAL_KERNEL_ABSORB);
             if (status == FUGAL_OK) status = finalize(plan_abs.clusters);
+        } else if (rows16.use) {
+            const int since = (t - p.fp32_warmup_sweeps) % p.reabsorb_every;
+            len = std::min({p.max_iterations - t, p.reabsorb_every - since, kRowsMaxSweeps});
+            status = launch_rows(rows16, rows_args(p.stream_dtype, len), stream, FUGAL_KERNEL_SWEEP);
         } else if (rowplan.use) {
             RowArgs ra{};
             ra.L = p.cost16;
@@ -2088,7 +1969,9 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
             status = read_poll(stop);
             if (status != FUGAL_OK || stop) break;
         }
-        const bool eval_point = (t % p.eval_freq == 0 && t != 0);
+        if (t + len >= p.max_iterations) break;  // nothing left to stop
+        // an evaluation point among sweeps t .. t + len - 1
+        const bool eval_point = (t + len - 1) / p.eval_freq > (t > 0 ? (t - 1) / p.eval_freq : 0);
         if (eval_point) {
             if (poll_slot >= 0) {  // eval_freq < kPollLag: settle the older poll first
                 status = read_poll(stop);
@@ -2100,7 +1983,7 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
                                 "sinkhorn: poll copy");
             if (status == FUGAL_OK) status = cuda_check(cudaEventRecord(ev[slot], stream), "sinkhorn: poll event");
             poll_slot = slot;
-            poll_t = t;
+            poll_t = t + len - 1;
         }
     }
     if (status != FUGAL_OK) {
@@ -2117,6 +2000,11 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
                                                           static_cast<int>(n), frame);
             status = launch_check("sinkhorn: polish begin");
         }
+        if (rows32.use) {
+            for (int k = 0; k < p.polish_sweeps && status == FUGAL_OK; k += kRowsMaxSweeps)
+                status = launch_rows(rows32, rows_args(FUGAL_F32, std::min(p.polish_sweeps - k, kRowsMaxSweeps)), stream,
+                                     FUGAL_KERNEL_SWEEP_F32);
+        } else
         for (int k = 0; k < p.polish_sweeps && status == FUGAL_OK; ++k) {
             SweepArgs a = sweep_args(plan32, p.cost32, p.ld32, nullptr, nullptr);
             status = launch_sweep(plan32, kernel_for(plan32.threads, plan32.kpt, FUGAL_F32, 0), a, stream, FUGAL_KERNEL_SWEEP_F32);

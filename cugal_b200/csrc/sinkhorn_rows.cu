@@ -1,0 +1,855 @@
+// Row-owned, persistent log-domain Sinkhorn sweeps (see sinkhorn.cu for what a
+// sweep is): one launch runs up to args.sweeps iteration boundaries.
+//
+// One 512-thread CTA per SM owns a block of whole rows.  Its 16 warps form
+// `GR` row streams of 512 / GR threads; stream g takes rows g, g + GR, ... of the
+// block, EPT columns per thread, so the row normaliser is a barrier of one
+// stream and the streams hide part of each other's reduction and barrier latency.
+// Running column sums and the column duals (b log2 e) of a thread's columns are
+// registers up to EPT = 32, tensor memory above.  A row's exponentials stay in
+// registers until the next row of the stream overwrites them chunk by chunk, each
+// 16-column chunk being added into the column sums right before.  Rows stream
+// through a ring of whole-row stages in shared memory (bulk copies); the cost does
+// not depend on the duals, so the ring already fills with the next sweep's first rows
+// while the CTAs exchange column sums.  When all rows of a CTA fit the ring they are
+// copied once and stay.
+//
+// What bounds it: small n, the two grid exchanges (about 6 us a sweep, of which 1.3 us
+// are each barrier and 2.5 us the FP64 column sums); from n = 3000 on the per-row
+// chain of a stream (wait, exponentials, shuffles, barrier, reciprocal: about 1.5 us
+// with 32 columns a thread) against MUFU and HBM.  Time per iteration, FP32, this
+// kernel against a cluster sweep and a finalize kernel per iteration: n = 1000 8.2
+// against 23.5 us, 4096 20.0 against 45.7, 8192 51.3 against 77.5 (41 us at the copy
+// peak); BF16: 4096 19.3 against 37.6, 8192 43.7 against 62.1, 16384 120 against 158,
+// 20011 217 against 275.  One exponential pair in 8 on the FMA pipe, worth 1.5% in the
+// 64-column kernel, costs 2 to 7% here (instruction issue) and is not used.
+//
+// End of a sweep: every CTA writes its column sums; grid barrier; each CTA
+// adds up its share of the columns in FP64 and writes log(colsum), its error and
+// its largest correction; grid barrier; every CTA sums the errors in the same
+// order and takes the same decision on its own copy of the solve state, which CTA
+// 0 writes back when the launch ends.  The launch is cooperative, so all CTAs are
+// resident; every wait is bounded, and a timed-out one ends the kernel with
+// FUGAL_DEVICE_TIMEOUT in the state.
+#include <algorithm>
+#include <type_traits>
+
+#include "fugal_common.cuh"
+#include "sinkhorn_rows.h"
+#include "sinkhorn_state.cuh"
+
+namespace fugal {
+
+constexpr int kRowsThreads = 512;
+// The streams' column sums meet in shared memory, unless two streams of more than 32
+// columns per thread need it for their stages (each then writes a partial row).
+constexpr bool rows_dump(int streams, int ept) { return streams > 1 && ept <= 32; }
+constexpr int kRowsWarps = kRowsThreads / 32;
+constexpr int kRowsMaxRows = 256;      // rows per CTA the row-dual staging holds
+constexpr int kRowsStatic = 24 * 1024; // shared memory kept for the static arrays
+
+// Barrier over the GT threads of stream g; true if every thread voted true.
+template <int GT>
+FUGAL_DEVICE bool stream_and(bool ok, int g) {
+    if constexpr (GT == kRowsThreads) {
+        return __syncthreads_and(ok) != 0;
+    } else {
+        uint32_t out;
+        asm volatile(
+            "{\n .reg .pred p, q;\n"
+            " setp.ne.u32 q, %1, 0;\n"
+            " barrier.cta.red.and.aligned.pred p, %2, %3, q;\n"
+            " selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(out)
+            : "r"(static_cast<uint32_t>(ok)), "r"(g + 1), "n"(GT)
+            : "memory");
+        return out != 0;
+    }
+}
+
+// Sum of GW per-warp values in a fixed pairwise order.
+template <int GW>
+FUGAL_DEVICE float sum_warps(const float* r) {
+    if constexpr (GW == 2) {
+        const float2 a = *reinterpret_cast<const float2*>(r);
+        return a.x + a.y;
+    } else {
+        float s[GW / 4];
+#pragma unroll
+        for (int i = 0; i < GW / 4; ++i) {
+            const float4 a = reinterpret_cast<const float4*>(r)[i];
+            s[i] = (a.x + a.y) + (a.z + a.w);
+        }
+        if constexpr (GW == 4) return s[0];
+        else if constexpr (GW == 8) return s[0] + s[1];
+        else return (s[0] + s[1]) + (s[2] + s[3]);
+    }
+}
+
+// 16 elements of a staged row (chunk c of this thread) as 8 float pairs.
+template <typename T, int GT>
+FUGAL_DEVICE void load16(const T* stage, int c, int gt, float2* v) {
+    constexpr int V = Vec<T>::N;
+#pragma unroll
+    for (int i = 0; i < 16 / V; ++i)
+        Pairs<T>::unpack(*reinterpret_cast<const uint4*>(stage + ((c * (16 / V) + i) * GT + gt) * V), v + i * V / 2);
+}
+
+// Grid-wide barrier (thread 0 of every CTA arrives and waits, bounded).  The
+// arrival counter is a multiple of the grid whenever no barrier is in progress;
+// `target` is its value when this barrier is complete.
+FUGAL_DEVICE bool grid_barrier(SolveState* st, bool ok, unsigned target, unsigned long long limit_ns) {
+    __shared__ int passed;
+    if (!__syncthreads_and(ok)) return false;
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->arrivals) : "memory");
+        const uint64_t limit = limit_ns != 0 ? limit_ns : kWaitLimitNs;
+        uint64_t t0 = 0;
+        int good = 0;
+        for (uint32_t i = 0; i < kMaxPolls; ++i) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&st->arrivals) : "memory");
+            if (static_cast<int>(v - target) >= 0) {
+                good = 1;
+                break;
+            }
+            if ((i & 63u) == 63u) {
+                const uint64_t now = global_timer_ns();
+                if (t0 == 0) t0 = now;
+                if (now - t0 > limit || *reinterpret_cast<volatile int*>(&st->status) != 0) break;
+            }
+        }
+        if (!good) report_error(&st->status, FUGAL_DEVICE_TIMEOUT);
+        passed = good;
+    }
+    __syncthreads();
+    return passed != 0;
+}
+
+// Column sums and column duals (b log2 e) of a thread's EPT columns: in registers
+// up to 32 columns, else in tensor memory, 16 columns per access.
+template <int EPT, bool REG = (EPT <= 32)>
+struct ColumnState;
+
+template <int EPT>
+struct ColumnState<EPT, true> {
+    static constexpr uint32_t kTmemColumns = 0;
+    float2 sum[EPT / 2], dual[EPT / 2];
+    FUGAL_DEVICE void start(uint32_t, int) {}
+    // 16 duals b of chunk c; their sums start at 0
+    FUGAL_DEVICE void set(int c, const float* b) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            dual[8 * c + q] = make_float2(b[2 * q], b[2 * q + 1]);
+            sum[8 * c + q] = make_float2(0.f, 0.f);
+        }
+    }
+    FUGAL_DEVICE void ready() {}
+    FUGAL_DEVICE void duals(int c, float2* b) const {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) b[q] = dual[8 * c + q];
+    }
+    // adds the pending row's chunk y (weight w) to the sums of chunk c
+    FUGAL_DEVICE void add(int c, const float2* y, float w) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) sum[8 * c + q] = __ffma2_rn(y[q], make_float2(w, w), sum[8 * c + q]);
+    }
+    FUGAL_DEVICE void total(int c, const float2* y, float w, float* out) {
+        add(c, y, w);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            out[2 * q] = sum[8 * c + q].x;
+            out[2 * q + 1] = sum[8 * c + q].y;
+        }
+    }
+};
+
+template <int EPT>
+struct ColumnState<EPT, false> {
+    static constexpr uint32_t kTmemColumns = 512;  // 4 warps per lane quarter x (sums + duals) x EPT <= 64
+    uint32_t tsum, tdual;
+    FUGAL_DEVICE void start(uint32_t base, int warp) {
+        tsum = base + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + static_cast<uint32_t>((warp >> 2) * EPT);
+        tdual = tsum + static_cast<uint32_t>((kRowsThreads / 128) * EPT);
+    }
+    FUGAL_DEVICE void set(int c, const float* b) {
+        float z[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) z[k] = 0.f;
+        tmem_st16(tdual + 16 * c, b);
+        tmem_st16(tsum + 16 * c, z);
+    }
+    FUGAL_DEVICE void ready() { tmem_wait_st(); }
+    FUGAL_DEVICE void duals(int c, float2* b) const {
+        float v[16];
+        tmem_ld16(tdual + 16 * c, v);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) b[q] = make_float2(v[2 * q], v[2 * q + 1]);
+    }
+    FUGAL_DEVICE void total(int c, const float2* y, float w, float* out) {
+        tmem_ld16(tsum + 16 * c, out);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const float2 a2 = __ffma2_rn(y[q], make_float2(w, w), make_float2(out[2 * q], out[2 * q + 1]));
+            out[2 * q] = a2.x;
+            out[2 * q + 1] = a2.y;
+        }
+    }
+    FUGAL_DEVICE void add(int c, const float2* y, float w) {
+        float acc[16];
+        total(c, y, w, acc);
+        tmem_st16(tsum + 16 * c, acc);
+    }
+};
+
+// This CTA's share of the columns: FP64 sums over the partial rows, log(colsum),
+// the CTA's error and largest correction.  Lanes of a warp: cgp column quads (a
+// power of two) x the rest over partial rows.  (Not inlined: its registers would
+// be live across the row loop.)
+__device__ __noinline__ void reduce_columns(const RowsArgs& p, int t, int parts) {
+    __shared__ double colred[kRowsWarps][128];
+    __shared__ double errred[kRowsWarps];
+    __shared__ float corred[kRowsWarps];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n = p.n;
+    const int quads = (n + 3) / 4;
+    const int per = (quads + gridDim.x - 1) / gridDim.x;
+    int cgp = 1;
+    while (cgp < per) cgp <<= 1;
+    const int cg = tid & (cgp - 1);
+    const int q0 = blockIdx.x * per;
+    const bool mine = cg < per && q0 + cg < quads;
+    const int j0 = (q0 + cg) * 4;
+    const int step = kRowsThreads / cgp;
+    double cs[4] = {0.0, 0.0, 0.0, 0.0};
+    // all of a thread's loads in flight (they come from L2): at most 4 up to 8192
+    // columns on 148 SMs, 10 per round above
+    const float* src = p.partials + j0;
+    auto add_rows = [&](auto unroll) {
+        constexpr int U = decltype(unroll)::value;
+        for (int k0 = tid / cgp; k0 < parts; k0 += U * step) {
+            float4 v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int k = k0 + u * step;
+                v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (mine && k < parts)
+                    v[u] = __ldcg(reinterpret_cast<const float4*>(src + static_cast<size_t>(k) * p.n_pad));
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (k0 + u * step < parts) {
+                    cs[0] += v[u].x;
+                    cs[1] += v[u].y;
+                    cs[2] += v[u].z;
+                    cs[3] += v[u].w;
+                }
+            }
+        }
+    };
+    if (parts <= 4 * step) add_rows(std::integral_constant<int, 4>{});
+    else add_rows(std::integral_constant<int, 10>{});
+    for (int o = cgp; o < 32; o <<= 1) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cs[q] += __shfl_xor_sync(0xffffffffu, cs[q], o);
+    }
+    // cgp <= 32: lane l < cgp of every warp holds quad l; cgp = 64: warps alternate quads 0..31, 32..63
+    if (lane < cgp) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) colred[warp][lane * 4 + q] = cs[q];
+    }
+    float b_now = 0.f;
+    if (tid < per * 4 && q0 * 4 + tid < n) b_now = __ldcg(p.b_buf + (t & 1) * p.n_pad + q0 * 4 + tid);
+    __syncthreads();
+    double err = 0.0;
+    float corr = 0.f;
+    if (tid < per * 4) {
+        const int j = q0 * 4 + tid;
+        if (j < n) {
+            // pairwise over the warps (the upper half is empty at cgp = 64)
+            double h[kRowsWarps];
+#pragma unroll
+            for (int w = 0; w < kRowsWarps; ++w)
+                h[w] = cgp <= 32 ? colred[w][tid]
+                                 : (w < kRowsWarps / 2 ? colred[2 * w + (tid >> 7)][tid & 127] : 0.0);
+#pragma unroll
+            for (int o = kRowsWarps / 2; o > 0; o >>= 1) {
+#pragma unroll
+                for (int w = 0; w < o; ++w) h[w] += h[w + o];
+            }
+            const double tot = h[0];
+            err = fabs(tot - 1.0);
+            const float lg = static_cast<float>(log(fmax(tot, 1e-37)));
+            p.logcs[j] = lg;
+            p.b_next[j] = b_now - lg;  // the next sweep's dual without momentum
+            corr = fabsf(lg);
+        }
+    }
+    const int used = (per * 4 + 31) / 32;  // warps that hold columns
+    if (warp < used) {
+        err = warp_sum(err);
+        corr = warp_max(corr);
+        if (used == 1) {
+            if (lane == 0) {
+                p.errs[blockIdx.x] = err;
+                p.corrs[blockIdx.x] = corr;
+            }
+        } else if (lane == 0) {
+            errred[warp] = err;
+            corred[warp] = corr;
+        }
+    }
+    if (used > 1) {
+        __syncthreads();
+        if (tid == 0) {
+            double e = 0.0;
+            float c = 0.f;
+            for (int w = 0; w < used; ++w) {
+                e += errred[w];
+                c = fmaxf(c, corred[w]);
+            }
+            p.errs[blockIdx.x] = e;
+            p.corrs[blockIdx.x] = c;
+        }
+    }
+}
+
+// The decision at the end of a sweep, the same in every CTA (warp 0).
+__device__ __noinline__ void take_decision(const RowsArgs& p, SolveState* ss) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == 0) {
+        double e = 0.0;
+        float c = 0.f;
+        constexpr int U = 8;  // 256 CTAs per round, all loads in flight
+        const int ctas = static_cast<int>(gridDim.x);
+        for (int k0 = lane; k0 < ctas; k0 += 32 * U) {
+            double ev[U];
+            float cv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int k = k0 + 32 * u;
+                ev[u] = k < ctas ? __ldcg(p.errs + k) : 0.0;
+                cv[u] = k < ctas ? __ldcg(p.corrs + k) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                e += ev[u];
+                c = fmaxf(c, cv[u]);
+            }
+        }
+        e = warp_sum(e);
+        c = warp_max(c);
+        if (lane == 0) {
+            decide(ss, e);
+            // the next sweep may use the previous row normaliser as its reference
+            // only if no column moves by more than kFastPathLimit nats
+            ss->exact_next = (c * static_cast<float>(ss->omega) > kFastPathLimit || ss->omega != 1.0) ? 1 : 0;
+        }
+    }
+}
+
+template <typename T, int EPT, int GR>
+__global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_constant__ RowsArgs p) {
+    constexpr int V = Vec<T>::N;                // elements per 16 bytes
+    constexpr int GT = kRowsThreads / GR;       // threads per stream
+    constexpr int GW = GT / 32;
+    constexpr int COVER = GT * EPT;             // columns a stream covers
+    constexpr int NCH = EPT / 16;
+    constexpr int H = EPT / 2;
+    constexpr bool F32 = sizeof(T) == 4;
+    constexpr bool DUMP = rows_dump(GR, EPT);
+    constexpr uint32_t TCOLS = ColumnState<EPT>::kTmemColumns;
+    static_assert(EPT <= 64, "column sums and duals of every thread fit the tensor memory");
+    static_assert(COVER * sizeof(T) <= 64 * 1024, "a stage holds one row");
+    extern __shared__ __align__(128) unsigned char ring[];
+    float* dump = reinterpret_cast<float*>(ring + static_cast<size_t>(p.stages) * COVER * sizeof(T));  // DUMP
+    __shared__ uint64_t full[kRowsMaxStages];
+    __shared__ __align__(16) float red_s[GR][2][GW];
+    __shared__ __align__(16) float red_m[GR][2][GW];
+    __shared__ float a_s[kRowsMaxRows];
+    __shared__ SolveState ss;
+    __shared__ int newest[kRowsMaxStages];  // phase of the newest copy into a stage (-1: none)
+    __shared__ uint32_t tmem_slot;
+
+    if (*reinterpret_cast<volatile int*>(&p.st->done)) return;  // uniform: written by an earlier kernel
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = tid / GT, gt = tid % GT, gw = warp % GW;
+    const int n = p.n;
+    const int row_begin = blockIdx.x * p.rows_per_cta;
+    const int nrows = max(0, min(n, row_begin + p.rows_per_cta) - row_begin);
+    const int NST = p.stages;
+    const float2 log2e2 = make_float2(kLog2e, kLog2e);
+
+    // this CTA's copy of the solve state, row duals, barriers, finite stage memory
+    // (columns past n_copy are never copied), tensor memory
+    for (int k = tid; k < static_cast<int>(sizeof(SolveState) / 4); k += kRowsThreads)
+        reinterpret_cast<int*>(&ss)[k] = reinterpret_cast<const int*>(p.st)[k];
+    for (int i = tid; i < nrows; i += kRowsThreads) a_s[i] = p.a[row_begin + i];
+    {
+        const int tail = COVER - p.n_copy;
+        for (int s = 0; s < NST; ++s) {
+            T* row = reinterpret_cast<T*>(ring) + static_cast<size_t>(s) * COVER;
+            for (int j = tid; j < tail; j += kRowsThreads) row[p.n_copy + j] = from_float<T>(0.f);
+        }
+    }
+    if (tid == 0) {
+        for (int s = 0; s < NST; ++s) {
+            mbar_init(&full[s], 1);
+            newest[s] = -1;
+        }
+        fence_mbarrier_init();
+    }
+    if constexpr (TCOLS > 0) {
+        if (warp == 0) {
+            tmem_alloc(&tmem_slot, TCOLS);
+            tmem_relinquish();
+        }
+        tmem_fence_before_sync();
+    }
+    __syncthreads();
+    ColumnState<EPT> cols;
+    if constexpr (TCOLS > 0) {
+        tmem_fence_after_sync();
+        cols.start(tmem_slot, warp);
+    }
+
+    // Ring of whole rows.  Unit u (row u mod nrows of sweep u / nrows) sits in stage
+    // u mod NST; the stream that consumed it refills the stage with unit u + NST, which
+    // within a sweep is that stream's own (NST is a multiple of GR) and in a later sweep
+    // is waited for only after a barrier of the whole CTA: no wait is ever more than one
+    // phase ahead of its barrier.
+    const int sweeps = min(p.sweeps, ss.max_it - ss.it);
+    const int units = p.resident ? nrows : nrows * sweeps;  // at most 256 kRowsMaxSweeps
+    const uint32_t row_bytes = static_cast<uint32_t>(p.n_copy) * sizeof(T);
+    auto issue = [&](int row, int s, uint32_t phase, bool first) {
+        const uint32_t unmet = (first && blockIdx.x == 0 && row == p.fault_row) ? 16u : 0u;
+        newest[s] = static_cast<int>(phase);
+        mbar_arrive_expect_tx(&full[s], row_bytes + unmet);
+        bulk_load(ring + static_cast<size_t>(s) * COVER * sizeof(T),
+                  static_cast<const T*>(p.L) +
+                      static_cast<unsigned long long>(static_cast<unsigned>(row_begin + row)) *
+                          static_cast<unsigned>(p.ld),
+                  row_bytes, &full[s]);
+    };
+    if (tid == 0) {
+        fence_proxy_async_smem();  // the fill above precedes the copies
+        const int first = min(units, NST);
+        for (int u = 0; u < first; ++u) issue(u % nrows, u, 0u, u < nrows);
+    }
+    int ubase = 0;  // units consumed by finished sweeps
+    int sbase = 0;        // their stage and phase: unit ubase + r sits in stage (sbase + r) mod NST
+    uint32_t phbase = 0u;
+    const int ahead = NST % max(1, nrows);  // row of unit u + NST, from u's row
+
+    // The duals of this thread's columns; up to 32 columns they are fetched while warp
+    // 0 still takes the decision of the sweep before.
+    constexpr bool PREFETCH = EPT <= 32;
+    float4 b_raw[PREFETCH ? EPT / 4 : 4];
+    auto column_of = [&](int e) { return ((e / V) * GT + gt) * V + e % V; };
+    // duals of sweep t before scaling: b_prev - omega logcs, or b_next, which the sweep
+    // before wrote for omega = 1
+    auto load_duals = [&](int e, int t, bool next, float omega) -> float4 {
+        const int j = column_of(e);
+        if (j >= n) return make_float4(0.f, 0.f, 0.f, 0.f);  // the vectors are n_pad long, a multiple of 64
+        if (next) return __ldcg(reinterpret_cast<const float4*>(p.b_next + j));
+        const float4 bp = __ldcg(reinterpret_cast<const float4*>(p.b_buf + ((t - 1) & 1) * p.n_pad + j));
+        const float4 lc = __ldcg(reinterpret_cast<const float4*>(p.logcs + j));
+        return make_float4(bp.x - omega * lc.x, bp.y - omega * lc.y, bp.z - omega * lc.z, bp.w - omega * lc.w);
+    };
+    const bool plain = ss.momentum_start < 0;  // omega stays 1
+
+    unsigned arrivals = ss.arrivals - ss.arrivals % gridDim.x;  // a first barrier may already be filling
+    bool alive = true;
+    for (int sw = 0; sw < sweeps; ++sw) {
+        const int t = ss.it;
+        const float omega = static_cast<float>(ss.omega);
+        const bool momentum = omega != 1.0f;
+        const bool exact_only = ss.exact_next != 0 || momentum;  // uniform
+        // ---- column duals of this sweep: b = b_prev - w log(colsum_prev), kept as b log2 e;
+        //      -inf past n, so those columns contribute exactly 0
+        {
+            const bool next = plain && sw > 0;
+            float* b_out = p.b_buf + (t & 1) * p.n_pad;
+#pragma unroll
+            for (int c = 0; c < NCH; ++c) {
+                float bb[16];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (!PREFETCH) b_raw[k] = load_duals(16 * c + 4 * k, t, next, omega);
+                    else if (!next) b_raw[4 * c + k] = load_duals(16 * c + 4 * k, t, false, omega);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int j = column_of(16 * c + 4 * k);
+                    const float4 b = b_raw[(PREFETCH ? 4 * c : 0) + k];
+                    if (blockIdx.x == 0 && g == 0 && j < n) *reinterpret_cast<float4*>(b_out + j) = b;
+                    const float b4[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) bb[4 * k + w] = j + w < n ? b4[w] * kLog2e : -INFINITY;
+                }
+                cols.set(c, bb);
+            }
+            cols.ready();
+        }
+
+        float2 y[H];     // exponentials of the stream's last row, not yet in the column sums
+        float wp = 0.f;  // and its weight 1 / (row sum)
+#pragma unroll
+        for (int h = 0; h < H; ++h) y[h] = make_float2(0.f, 0.f);
+        int s_cur = sbase + g;
+        uint32_t ph = phbase;
+        while (s_cur >= NST) {
+            s_cur -= NST;
+            ph ^= 1u;
+        }
+        int par = 0;
+        for (int r = g; r < nrows; r += GR, par ^= 1) {
+            const int s = s_cur;
+            const T* stage = reinterpret_cast<const T*>(ring) + static_cast<size_t>(s) * COVER;
+            // a resident row is waited for once per launch
+            bool ok = (p.resident && sw > 0) ||
+                      mbar_wait<true>(&full[s], p.resident ? 0u : ph, &p.st->status, p.suspend_ns, p.wait_limit_ns);
+            auto release = [&]() {
+                // (every thread of the stream has read the stage before the barrier just passed)
+                if (gt == 0 && ubase + r + NST < units) {
+                    int row = r + ahead;
+                    if (row >= nrows) row -= nrows;
+                    issue(row, s, ph ^ 1u, false);
+                }
+            };
+            float anew = 0.f, wr = 0.f;
+            bool fast_ok = false;
+            if (!exact_only) {
+                // ---- fast path: y = 2^(L log2e + b [+ a_old log2e]), against the absorbed frame
+                //      (16-bit) or the previous row normaliser (FP32)
+                float2 s2 = make_float2(0.f, 0.f), t2 = make_float2(0.f, 0.f);
+                const float ref = F32 ? a_s[r] * kLog2e : 0.f;
+                const float2 ref2 = make_float2(ref, ref);
+#pragma unroll
+                for (int c = 0; c < NCH; ++c) {
+                    cols.add(c, y + 8 * c, wp);
+                    float2 bb[8];
+                    cols.duals(c, bb);
+#pragma unroll
+                    for (int i = 0; i < 16 / V; ++i) {
+                        float2 v2[V / 2];
+                        Pairs<T>::unpack(
+                            *reinterpret_cast<const uint4*>(stage + ((c * (16 / V) + i) * GT + gt) * V), v2);
+#pragma unroll
+                        for (int h = 0; h < V / 2; ++h) {
+                            const int q = i * (V / 2) + h;
+                            float2 b2 = bb[q];
+                            if (F32) b2 = __fadd2_rn(b2, ref2);
+                            const float2 x = __ffma2_rn(v2[h], log2e2, b2);
+                            const float2 e = ex2_pair(x);
+                            y[8 * c + q] = e;
+                            if (q & 1)
+                                t2 = __fadd2_rn(t2, e);
+                            else
+                                s2 = __fadd2_rn(s2, e);
+                        }
+                    }
+                }
+                const float2 u2 = __fadd2_rn(s2, t2);
+                const float part = warp_sum(u2.x + u2.y);
+                if (lane == 0) red_s[g][par][gw] = part;
+                if (!stream_and<GT>(ok, g)) {
+                    alive = false;
+                    break;
+                }
+                const float S = sum_warps<GW>(red_s[g][par]);
+                fast_ok = S > 1e-30f && S < 1e30f;  // uniform over the stream
+                if (fast_ok) {
+                    release();
+                    if (gt == GT - 32) anew = (F32 ? a_s[r] : 0.f) - __log2f(S) * kLn2;
+                    wr = __frcp_rn(S);
+                }
+            }
+            if (!fast_ok) {
+                // ---- exact path: row maximum, then the exponentials relative to it (the previous
+                //      row dual is read before the barriers that precede its update)
+                const float a_old = momentum ? a_s[r] : 0.f;
+                if (exact_only) {  // the pending row (the fast path above has already added it)
+#pragma unroll
+                    for (int c = 0; c < NCH; ++c) cols.add(c, y + 8 * c, wp);
+                }
+                float mx = -INFINITY;
+#pragma unroll
+                for (int c = 0; c < NCH; ++c) {
+                    float2 bb[8];
+                    cols.duals(c, bb);
+                    float2 v2[8];
+                    load16<T, GT>(stage, c, gt, v2);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const float2 x = __ffma2_rn(v2[q], log2e2, bb[q]);
+                        y[8 * c + q] = x;
+                        mx = fmaxf(mx, fmaxf(x.x, x.y));
+                    }
+                }
+                mx = warp_max(mx);
+                if (lane == 0) red_m[g][par][gw] = mx;
+                if (!stream_and<GT>(ok, g)) {
+                    alive = false;
+                    break;
+                }
+                float M2 = -INFINITY;
+#pragma unroll
+                for (int w = 0; w < GW; ++w) M2 = fmaxf(M2, red_m[g][par][w]);
+                const float base = (M2 == -INFINITY) ? 0.f : M2;
+                const float2 nb = make_float2(-base, -base);
+                float2 ssum = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    y[h] = ex2_pair(__fadd2_rn(y[h], nb));
+                    ssum = __fadd2_rn(ssum, y[h]);
+                }
+                const float part = warp_sum(ssum.x + ssum.y);
+                if (lane == 0) red_s[g][par][gw] = part;
+                stream_and<GT>(true, g);
+                release();
+                const float S = sum_warps<GW>(red_s[g][par]);
+                const float lse = (M2 + log2f(S)) * kLn2;
+                anew = momentum ? (1.f - omega) * a_old - omega * lse : -lse;
+                wr = (M2 == -INFINITY) ? 0.f : ex2(M2 + anew * kLog2e);
+            }
+            if (gt == GT - 32) {  // not the warp that refills the stage
+                a_s[r] = anew;
+                p.a[row_begin + r] = anew;
+            }
+            wp = wr;
+            s_cur += GR;
+            while (s_cur >= NST) {
+                s_cur -= NST;
+                ph ^= 1u;
+            }
+        }
+
+        // ---- this CTA's column sums: the streams' sums (the pending rows included) meet in
+        //      shared memory, so that the grid exchanges one row per CTA
+        {
+            float* prow = p.partials + static_cast<size_t>(blockIdx.x * (DUMP ? 1 : GR) + (DUMP ? 0 : g)) * p.n_pad;
+            float* mine = DUMP ? dump + static_cast<size_t>(g) * COVER : prow;
+#pragma unroll
+            for (int c = 0; c < NCH; ++c) {
+                float acc[16];
+                cols.total(c, y + 8 * c, wp, acc);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int j = column_of(16 * c + 4 * k);
+                    if (j < n)  // partial rows are n_pad wide, a multiple of 64 columns
+                        *reinterpret_cast<float4*>(mine + j) =
+                            make_float4(acc[4 * k], acc[4 * k + 1], acc[4 * k + 2], acc[4 * k + 3]);
+                }
+            }
+            if constexpr (DUMP) {
+                __syncthreads();
+                for (int j = tid * 4; j < n; j += kRowsThreads * 4) {
+                    float4 v[GR];
+#pragma unroll
+                    for (int k = 0; k < GR; ++k) v[k] = *reinterpret_cast<const float4*>(dump + k * COVER + j);
+#pragma unroll
+                    for (int o = 1; o < GR; o <<= 1) {  // neighbours first
+#pragma unroll
+                        for (int k = 0; k < GR; k += 2 * o) {
+                            v[k].x += v[k + o].x;
+                            v[k].y += v[k + o].y;
+                            v[k].z += v[k + o].z;
+                            v[k].w += v[k + o].w;
+                        }
+                    }
+                    *reinterpret_cast<float4*>(prow + j) = v[0];
+                }
+            }
+        }
+        arrivals += gridDim.x;
+        if (!grid_barrier(p.st, alive, arrivals, p.wait_limit_ns)) {  // the same in every thread of the CTA
+            alive = false;
+            break;
+        }
+        reduce_columns(p, t, gridDim.x * (DUMP ? 1 : GR));
+        arrivals += gridDim.x;
+        if (!grid_barrier(p.st, true, arrivals, p.wait_limit_ns)) {
+            alive = false;
+            break;
+        }
+        if (PREFETCH && plain) {
+#pragma unroll
+            for (int k = 0; k < (PREFETCH ? EPT / 4 : 0); ++k) b_raw[k] = load_duals(4 * k, t + 1, true, 1.f);
+        }
+        take_decision(p, &ss);
+        ubase += nrows;
+        if (!p.resident) {
+            sbase += nrows;
+            while (sbase >= NST) {
+                sbase -= NST;
+                phbase ^= 1u;
+            }
+        }
+        __syncthreads();
+        if (ss.done) break;
+    }
+
+    // Copies may be in flight (stages refilled ahead, or a timed-out wait): wait for
+    // the newest copy of every stage (bounded) before its shared memory is released;
+    // one that never completes does not hide the others.
+    __syncthreads();
+    if (tid == 0) {
+        for (int s = 0; s < NST; ++s)
+            if (newest[s] >= 0)
+                mbar_wait<true>(&full[s], static_cast<uint32_t>(newest[s]), &p.st->status, p.suspend_ns,
+                                p.wait_limit_ns);
+        if (!alive) {
+            p.st->done = 1;
+            p.st->final_it = ss.it;
+            if (ss.check) {
+                p.st->main_final_it = ss.it;
+                p.st->main_n_err = ss.n_err;
+            }
+            p.st->it = ss.it + 1;
+        }
+    }
+    if (alive && blockIdx.x == 0) {
+        // write the state back (not the error word and the barrier, which the CTAs share)
+        SolveState* st = p.st;
+        if (tid == 0) {
+            st->it = ss.it;
+            st->done = ss.done;
+            st->final_it = ss.final_it;
+            st->n_err = ss.n_err;
+            st->main_final_it = ss.main_final_it;
+            st->main_n_err = ss.main_n_err;
+            st->polish_count = ss.polish_count;
+            st->exact_next = ss.exact_next;
+            st->omega = ss.omega;
+            st->last_err = ss.last_err;
+            st->main_last_err = ss.main_last_err;
+            st->polish_err = ss.polish_err;
+        }
+        for (int k = tid; k < min(ss.n_err, FUGAL_MAX_RECORDED_ERRORS); k += kRowsThreads) st->errors[k] = ss.errors[k];
+    }
+    if constexpr (TCOLS > 0) {
+        tmem_fence_before_sync();
+        __syncthreads();
+        tmem_fence_after_sync();
+        if (warp == 0) tmem_dealloc(tmem_slot, TCOLS);
+    }
+}
+
+namespace {
+
+using RowsFn = void (*)(const RowsArgs);
+
+template <typename T>
+RowsFn rows_fn(int ept, int streams) {
+    switch (streams * 100 + ept) {
+        case 816: return rows_kernel<T, 16, 8>;
+        case 832: return rows_kernel<T, 32, 8>;
+        case 432: return rows_kernel<T, 32, 4>;
+        case 448: return rows_kernel<T, 48, 4>;
+    }
+    if constexpr (sizeof(T) == 2) {
+        switch (streams * 100 + ept) {
+            case 464: return rows_kernel<T, 64, 4>;
+            case 248: return rows_kernel<T, 48, 2>;
+            case 264: return rows_kernel<T, 64, 2>;
+            default: return rows_kernel<T, 48, 1>;
+        }
+    } else {
+        return rows_kernel<T, 32, 2>;
+    }
+}
+
+RowsFn rows_fn(const RowsPlan& pl) {
+    if (pl.dt == FUGAL_F32) return rows_fn<float>(pl.ept, pl.streams);
+    return pl.dt == FUGAL_BF16 ? rows_fn<__nv_bfloat16>(pl.ept, pl.streams) : rows_fn<__half>(pl.ept, pl.streams);
+}
+
+// (streams, columns per thread) in the order of the columns they cover,
+// 512 / streams * ept: the narrowest that covers n.  Measured per iteration: BF16 at
+// n = 8192 43.7 us as {4, 64}, 51.2 as {2, 32}; n = 6000 29.6 as {4, 48}, 39.1 as
+// {2, 32}; n = 4096 19.3 as {4, 32}, 25.5 as {8, 64}.  FP32 rows of 6145 to 8192
+// columns take two streams, so that two stages of 32 KB are left for each.  Wider
+// rows: FP32 sweeps are at 85% of the copy peak in the cluster kernel; 16-bit ones of
+// more than 24576 columns have too few stages left here (469 against 454 us at 32768).
+struct RowsShape {
+    int streams, ept;
+};
+constexpr RowsShape kShapes16[] = {{8, 16}, {8, 32}, {4, 32}, {4, 48}, {4, 64}, {2, 48}, {2, 64}, {1, 48}};
+constexpr RowsShape kShapes32[] = {{8, 16}, {8, 32}, {4, 32}, {4, 48}, {2, 32}};
+
+RowsShape rows_shape(int64_t n, int dt) {
+    auto covers = [n](const RowsShape& sh) { return static_cast<int64_t>(kRowsThreads / sh.streams) * sh.ept >= n; };
+    if (dt == FUGAL_F32) {
+        for (const RowsShape& sh : kShapes32)
+            if (covers(sh)) return sh;
+    } else {
+        for (const RowsShape& sh : kShapes16)
+            if (covers(sh)) return sh;
+    }
+    return RowsShape{0, 0};
+}
+
+}  // namespace
+
+fugal_status make_rows_plan(int64_t n, int dt, RowsPlan& pl, bool device) {
+    pl = RowsPlan{};
+    pl.dt = dt;
+    const int es = dt == FUGAL_F32 ? 4 : 2;
+    const RowsShape shape = rows_shape(n, dt);
+    if (shape.streams == 0) return FUGAL_OK;
+    pl.streams = shape.streams;
+    pl.ept = shape.ept;
+    const int sms = sm_count();
+    const int want = static_cast<int>(std::min<int64_t>(sms, n));
+    pl.rows_per_cta = static_cast<int>((n + want - 1) / want);
+    if (pl.rows_per_cta > kRowsMaxRows) return FUGAL_OK;
+    pl.ctas = static_cast<int>((n + pl.rows_per_cta - 1) / pl.rows_per_cta);
+    const size_t stage = static_cast<size_t>(kRowsThreads / pl.streams) * pl.ept * es;
+    const size_t dump = rows_dump(pl.streams, pl.ept) ? static_cast<size_t>(kRowsThreads) * pl.ept * 4 : 0;
+    pl.parts = pl.ctas * (dump > 0 ? 1 : pl.streams);
+    const size_t room = 227 * 1024 - kRowsStatic - dump;
+    pl.stages = static_cast<int>(std::min<size_t>({room / stage, static_cast<size_t>(kRowsMaxStages),
+                                                   static_cast<size_t>(pl.rows_per_cta)}));
+    pl.resident = pl.stages >= pl.rows_per_cta;
+    // A stage that is refilled within a sweep has to go back to the stream that emptied
+    // it: a stream waiting for a copy two phases ahead of the stage's barrier would take
+    // the phase before as its own (mbarrier waits see one parity bit).
+    if (!pl.resident) pl.stages -= pl.stages % pl.streams;
+    if (pl.stages < 1) return FUGAL_OK;
+    pl.smem = stage * pl.stages + dump;
+    if (device) {
+        int dev = 0, coop = 0, blocks = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return FUGAL_OK;
+        RowsFn fn = rows_fn(pl);
+        FUGAL_TRY(cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem),
+                             "sinkhorn rows: shared memory"));
+        FUGAL_TRY(cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, kRowsThreads, pl.smem),
+                             "sinkhorn rows: occupancy"));
+        if (blocks < 1) return FUGAL_OK;
+    }
+    pl.use = true;
+    return FUGAL_OK;
+}
+
+fugal_status launch_rows(const RowsPlan& pl, RowsArgs args, cudaStream_t stream, int family) {
+    args.rows_per_cta = pl.rows_per_cta;
+    args.stages = pl.stages;
+    args.resident = pl.resident;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(pl.ctas, 1, 1);
+    cfg.blockDim = dim3(kRowsThreads, 1, 1);
+    cfg.dynamicSmemBytes = pl.smem;
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    LaunchScope scope(family, stream);
+    return cuda_check(cudaLaunchKernelEx(&cfg, rows_fn(pl), args), "sinkhorn rows: launch");
+}
+
+}  // namespace fugal

@@ -42,6 +42,7 @@ class SinkhornSolver:
             raise ValueError(f"unsupported stream_dtype {config.stream_dtype}")
         ws = N.workspace_size("fugal_sinkhorn_workspace_size", n, self.stream_dtype)
         self.workspace = torch.empty(ws, dtype=torch.uint8, device=self.device)
+        self.fixed_order = False  # see fugal_solve_params.fixed_order
         self.ld16 = padded_ld(n)
         self.cost16 = None
         if self.stream_dtype != N.FUGAL_F32:
@@ -67,6 +68,7 @@ class SinkhornSolver:
         p.u_out = u_out.data_ptr()
         p.v_out = v_out.data_ptr()
         p.record = record_ptr
+        p.fixed_order = int(self.fixed_order)
         if column_partials is not None:
             # (chunks, 2 ld) float32 = chunks x ld (max, sum) pairs
             p.column_partials = column_partials.data_ptr()

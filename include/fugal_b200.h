@@ -334,6 +334,9 @@ typedef struct {
      * float pairs, merged into the first column update. */
     const float* column_partials;
     int32_t column_partial_chunks;
+    /* 1: the FP32 and 16-bit sweeps sum in the order of the cluster kernel at every size
+     * (for a caller that differentiates the plan); 0: the fastest kernel for the size. */
+    int32_t fixed_order;
     int64_t column_partial_ld;
 } fugal_solve_params;
 
