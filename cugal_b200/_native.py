@@ -24,6 +24,7 @@ LAP_GREEDY, LAP_DOUBLE_GREEDY, LAP_PARALLEL_GREEDY, LAP_ORDERED = 0, 1, 2, 3
  KERNEL_UPDATE, KERNEL_OTHER) = range(8)
 KERNEL_FAMILY_NAMES = ["sweep16", "sweep32", "absorb", "finalize", "column_pass", "gradient", "update", "other"]
 MAX_RECORDED_ERRORS = 256
+ADJOINT_SOLVE_MAX_N = 16384
 
 STREAM_DTYPES = {None: FUGAL_F32, torch.float32: FUGAL_F32, torch.bfloat16: FUGAL_BF16, torch.float16: FUGAL_F16}
 
@@ -90,6 +91,8 @@ SIGNATURES = {
     "fugal_plan_matvec_workspace_size": (_INT, [_I64, POINTER(c_size_t)]),
     "fugal_plan_matvec": (_INT, [_P, _I64, _P, _I64, _I64, _P, _P, _P, _P, _P, _SZ, _P]),
     "fugal_sinkhorn_adjoint": (_INT, [_P, _I64, _P, _I64, _I64, _P, _P, _D, _P, _I64, _P]),
+    "fugal_sinkhorn_adjoint_solve_workspace_size": (_INT, [_I64, POINTER(c_size_t)]),
+    "fugal_sinkhorn_adjoint_solve": (_INT, [_P, _I64, _I64, _P, _P, _D, _INT, _P, _P, _P, _P, _SZ, _P]),
     "fugal_sinkhorn_unrolled_step_backward": (_INT, [_P, _I64, _I64, _P, _P, _P, _INT, _P, _I64, _P, _P, _SZ, _P]),
     "fugal_sinkhorn_workspace_size": (_INT, [_I64, _INT, POINTER(c_size_t)]),
     "fugal_sinkhorn_plan_info": (_INT, [_I64, _INT, _P]),

@@ -8,8 +8,9 @@ implicit-function adjoint at the converged potentials, on the device:
     a = (G o P) 1,  b = (G o P)^T 1,   [I P; P^T I][alpha; beta] = [a; b]   (CG),
     dL/dC = -(1/reg) P o (G - alpha 1^T - 1 beta^T).
 
-Each CG iteration is one pass over P (``fugal_plan_matvec`` forms P y and
-P^T x together); the O(n) vector arithmetic runs in FP64.  The reference has no
+Each CG iteration is one pass over P (P y and P^T x are formed together); the
+O(n) vector arithmetic runs in FP64.  Up to n = 16384 all iterations are one
+launch (``fugal_sinkhorn_adjoint_solve``), above one ``fugal_plan_matvec`` each.  The reference has no
 backward pass; its torch ``solve_log`` differentiated by autograd is the check
 (tests/test_gpu_adjoint.py), with central finite differences of the FP64 oracle.
 
@@ -48,15 +49,26 @@ class _Matvec:
         return Ptx, Py
 
 
-def sinkhorn_adjoint(P: torch.Tensor, G: torch.Tensor, reg: float, tol: float = 1e-7, max_iter: int = 2000):
-    """dL/dC for the converged plan P (n x n FP32 CUDA) and G = dL/dP; returns
-    (dC FP32, CG iterations, final relative residual)."""
-    N.require_cuda(P, "P", torch.float32)
-    G = G.to(torch.float32).contiguous()
+def _solve_on_device(P, a, b, tol: float, max_iter: int):
+    """(alpha, beta, iterations, relative residual) of the adjoint's system, all iterations in one launch."""
     n = P.shape[0]
-    mv = _Matvec(n, P.device)
-    ones = torch.ones(n, dtype=torch.float64, device=P.device)
-    b, a = mv(P, ones, ones, W=G)          # b = (P o G)^T 1, a = (P o G) 1
+    alpha, beta = torch.empty_like(a), torch.empty_like(b)
+    info = torch.empty(3, dtype=torch.float64, device=P.device)
+    ws = torch.empty(N.workspace_size("fugal_sinkhorn_adjoint_solve_workspace_size", n), dtype=torch.uint8,
+                     device=P.device)
+    N.call("fugal_sinkhorn_adjoint_solve", P.data_ptr(), N.matrix_ld(P, "P"), n, a.data_ptr(), b.data_ptr(),
+           float(tol), int(max_iter), alpha.data_ptr(), beta.data_ptr(), info.data_ptr(), ws.data_ptr(), ws.numel(),
+           N.stream_handle(P.device))
+    it, rel, status = info.tolist()
+    if status != 0:
+        raise N.NativeError(f"fugal_sinkhorn_adjoint_solve: device status {int(status)} (bounded wait timed out)")
+    return alpha, beta, int(it), rel
+
+
+def _solve_by_launches(mv: _Matvec, P, a, b, tol: float, max_iter: int):
+    """The same with one matvec launch per iteration, for sizes whose vectors do not fit shared memory
+    (an iteration's pass over P is then long against its launches)."""
+    n = P.shape[0]
     rhs = torch.cat([a, b])
 
     def apply(z):
@@ -82,7 +94,22 @@ def sinkhorn_adjoint(P: torch.Tensor, G: torch.Tensor, reg: float, tol: float = 
                 break
             p = r + (rs_new / rs) * p
             rs = rs_new
-    alpha_v, beta_v = z[:n].contiguous(), z[n:].contiguous()
+    return z[:n].contiguous(), z[n:].contiguous(), it, rel
+
+
+def sinkhorn_adjoint(P: torch.Tensor, G: torch.Tensor, reg: float, tol: float = 1e-7, max_iter: int = 2000):
+    """dL/dC for the converged plan P (n x n FP32 CUDA) and G = dL/dP; returns
+    (dC FP32, CG iterations, final relative residual)."""
+    N.require_cuda(P, "P", torch.float32)
+    G = G.to(torch.float32).contiguous()
+    n = P.shape[0]
+    mv = _Matvec(n, P.device)
+    ones = torch.ones(n, dtype=torch.float64, device=P.device)
+    b, a = mv(P, ones, ones, W=G)          # b = (P o G)^T 1, a = (P o G) 1
+    if n <= N.ADJOINT_SOLVE_MAX_N:
+        alpha_v, beta_v, it, rel = _solve_on_device(P, a, b, tol, max_iter)
+    else:
+        alpha_v, beta_v, it, rel = _solve_by_launches(mv, P, a, b, tol, max_iter)
     dC = torch.empty((n, n), dtype=torch.float32, device=P.device)
     N.call("fugal_sinkhorn_adjoint", P.data_ptr(), N.matrix_ld(P, "P"), G.data_ptr(), N.matrix_ld(G, "G"), n,
            alpha_v.data_ptr(), beta_v.data_ptr(), -1.0 / reg, dC.data_ptr(), n, N.stream_handle(P.device))

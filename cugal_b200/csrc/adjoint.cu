@@ -15,7 +15,8 @@
 //   plan_kernel        P = exp(L + u_i + v_j) from the absorbed cost and duals;
 //   matvec_part_kernel tiles of 64 rows x 1024 columns: row partials of P y and
 //                      column partials of P^T x (P optionally weighted by G);
-//   matvec_merge_*     FP64 sums of the partials;
+//   merge_add_kernel   FP64 sums of the partials;
+//   cg_kernel          the whole conjugate-gradient solve in one launch;
 //   adjoint_kernel     out = scale * P o (G - alpha_i - beta_j).
 #include <cuda_runtime.h>
 
@@ -92,14 +93,6 @@ __global__ void __launch_bounds__(kMvThreads) matvec_part_kernel(const float* __
         if (j0 + q < n) col_part[static_cast<size_t>(blockIdx.y) * n + j0 + q] = cs[q];
 }
 
-__global__ void matvec_merge_kernel(const double* part, int parts, int n, double* out) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int p = 0; p < parts; ++p) s += part[static_cast<size_t>(p) * n + k];
-        out[k] = s;
-    }
-}
-
 __global__ void adjoint_kernel(const float* __restrict__ P, long long ldp, const float* __restrict__ G,
                                long long ldg, int n, const double* __restrict__ alpha,
                                const double* __restrict__ beta, double scale, float* __restrict__ out,
@@ -119,18 +112,22 @@ __global__ void adjoint_kernel(const float* __restrict__ P, long long ldp, const
 //     gK_ij -= g_i E_ij,   g_other_j -= sum_i g_i E_ij        (column partials)
 // axis 0 (column half, out_j = -LSE_i(K_ij + other_i)): E_ij = exp(K_ij + other_i + out_j),
 //     gK_ij -= g_j E_ij,   g_other_i -= sum_j g_j E_ij        (row partials)
+// A block covers kUnRows rows x 1024 columns (4 consecutive columns per thread): at
+// n = 1024 128 blocks, where blocks of 64 rows made 16 (89 us a half step, bound by
+// their FP64 exponentials; 10 us here).
+constexpr int kUnRows = 8;
 __global__ void __launch_bounds__(kMvThreads) unrolled_step_kernel(const float* __restrict__ K, long long ldk, int n,
                                                                    const float* __restrict__ out_dual,
                                                                    const float* __restrict__ other_dual,
                                                                    const double* __restrict__ g, int axis,
                                                                    float* __restrict__ gK, long long ldg,
                                                                    double* row_part, double* col_part) {
-    __shared__ double red[kMvThreads / 32][kMvRows];
+    __shared__ double red[kMvThreads / 32][kUnRows];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int r0 = blockIdx.y * kMvRows;
+    const int r0 = blockIdx.y * kUnRows;
     const int j0 = blockIdx.x * kMvCols + threadIdx.x * 4;
     double cs[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int r = 0; r < kMvRows; ++r) {
+    for (int r = 0; r < kUnRows; ++r) {
         const int i = r0 + r;
         double rs = 0.0;
         if (i < n) {
@@ -161,7 +158,7 @@ __global__ void __launch_bounds__(kMvThreads) unrolled_step_kernel(const float* 
     }
     if (axis == 0) {
         __syncthreads();
-        if (threadIdx.x < kMvRows) {
+        if (threadIdx.x < kUnRows) {
             const int i = r0 + threadIdx.x;
             double s = 0.0;
 #pragma unroll
@@ -175,11 +172,275 @@ __global__ void __launch_bounds__(kMvThreads) unrolled_step_kernel(const float* 
     }
 }
 
-__global__ void merge_add_kernel(const double* part, int parts, int n, double* out) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+// out[k] += sum of the parts of column k (add), or = it: 32 columns per block, the
+// parts over its 8 warps, eight loads in flight per lane.
+__global__ void __launch_bounds__(256) merge_add_kernel(const double* __restrict__ part, int parts, int n, double* out,
+                                                        int add) {
+    __shared__ double red[8][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int k = blockIdx.x * 32 + lane;
+    double s = 0.0;
+    if (k < n) {
+        for (int p0 = warp; p0 < parts; p0 += 64) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = p0 + 8 * u < parts ? part[static_cast<size_t>(p0 + 8 * u) * n + k] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += v[u];
+        }
+    }
+    red[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && k < n) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += red[w][lane];
+        out[k] = add ? out[k] + t : t;
+    }
+}
+
+// Conjugate gradients on [I P; P^T I] [alpha; beta] = [a; b] (alpha, beta from 0)
+// in one persistent, cooperative launch: one 512-thread CTA per SM owns a block of
+// rows (its entries of alpha) and a block of columns (its entries of beta).  Per
+// iteration:
+//   matvec   P y (complete for the CTA's rows) and the CTA's partial of P^T x, from
+//            one read of its rows of P; the search direction's column half y sits in
+//            every CTA's shared memory.  Grid barrier.
+//   columns  the CTA's columns of P^T x, <p, A p>.  Grid barrier.
+//   update   alpha/beta and the residual of the CTA's rows and columns, <r, r>.  Grid
+//            barrier; every CTA then forms the new y itself from the residual.
+// All vectors, sums and scalars are FP64, sums in a fixed order.  As a loop of
+// launches an iteration was one matvec (38 us at n = 4096), 16 vector launches and a
+// host round trip for the residual, 145 us; here about 20 us, bound by the L2 reads
+// of P (67 MB) and the FP32 -> FP64 conversions (16 a clock per SM).
+constexpr int kCgThreads = 512;
+constexpr int kCgWarps = kCgThreads / 32;
+constexpr int kCgRows = 8;         // rows in flight per thread
+constexpr int kCgMaxN = 16384;     // y (8 bytes a column) fits the shared memory
+constexpr int kCgMaxOwn = 128;     // rows and columns a CTA owns at most
+
+struct CgArgs {
+    const float* P;
+    long long ldp;
+    int n;
+    int own;             // rows (and columns) per CTA
+    const double* a;     // [n]
+    const double* b;     // [n]
+    double tol;
+    int max_iter;
+    double* alpha;       // [n]
+    double* beta;        // [n]
+    double* info;        // iterations, relative residual, status
+    double* colpart;     // [CTAs][n]
+    double* r_cols;      // [n] residual of the column half
+    double* dots;        // [2][CTAs]
+    unsigned* arrivals;
+    int* status;
+};
+
+// Sums of 8 values over the 32 lanes of a warp: on return lane l holds the sum of
+// value (l >> 2) in the low two bits' group (all four lanes alike).
+FUGAL_DEVICE double warp_sum8(const double (&v)[8]) {
+    const int lane = threadIdx.x & 31;
+    double w4[4], w2[2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double send = (lane & 16) ? v[k] : v[k + 4];
+        const double keep = (lane & 16) ? v[k + 4] : v[k];
+        w4[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const double send = (lane & 8) ? w4[k] : w4[k + 2];
+        const double keep = (lane & 8) ? w4[k + 2] : w4[k];
+        w2[k] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+    }
+    const double send = (lane & 4) ? w2[0] : w2[1];
+    double w = ((lane & 4) ? w2[1] : w2[0]) + __shfl_xor_sync(0xffffffffu, send, 4);
+    w += __shfl_xor_sync(0xffffffffu, w, 2);
+    w += __shfl_xor_sync(0xffffffffu, w, 1);
+    return w;
+}
+
+// The sum of one value per CTA, the same in every thread of every CTA.
+FUGAL_DEVICE double grid_total(const double* per_cta, double* scratch) {
+    __syncthreads();  // scratch is free
+    if (threadIdx.x < 32) {
         double s = 0.0;
-        for (int p = 0; p < parts; ++p) s += part[static_cast<size_t>(p) * n + k];
-        out[k] += s;
+        const int ctas = static_cast<int>(gridDim.x);
+        for (int k0 = threadIdx.x; k0 < ctas; k0 += 256) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = k0 + 32 * u < ctas ? __ldcg(per_cta + k0 + 32 * u) : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += v[u];
+        }
+        s = warp_sum(s);
+        if (threadIdx.x == 0) scratch[0] = s;
+    }
+    __syncthreads();
+    return scratch[0];
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(kCgThreads, 1) cg_kernel(const __grid_constant__ CgArgs p) {
+    extern __shared__ __align__(16) double y_s[];  // [n rounded up to 2048]
+    __shared__ double x_s[kCgMaxOwn], rx_s[kCgMaxOwn], zx_s[kCgMaxOwn], apx_s[kCgMaxOwn];
+    __shared__ double ry_s[kCgMaxOwn], zy_s[kCgMaxOwn], apy_s[kCgMaxOwn];
+    __shared__ double red[kCgWarps][kCgMaxOwn];
+    __shared__ double scratch[32];
+    constexpr int SPAN = kCgThreads * 4;  // columns a CTA covers at once
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n = p.n;
+    const int o0 = blockIdx.x * p.own;
+    const int own = max(0, min(n, o0 + p.own) - o0);
+    const int span_n = (n + SPAN - 1) / SPAN * SPAN;
+    unsigned arrivals = 0;
+    auto barrier = [&]() {
+        arrivals += gridDim.x;
+        return grid_barrier(p.arrivals, p.status, true, arrivals, 0);
+    };
+    // column q of this thread in the span starting at c0
+    auto column = [&](int c0, int q) { return VEC ? c0 + tid * 4 + q : c0 + q * kCgThreads + tid; };
+    auto give_up = [&]() {  // a wait ran out: no result
+        for (int k = tid; k < own; k += kCgThreads) p.alpha[o0 + k] = p.beta[o0 + k] = NAN;
+        if (blockIdx.x == 0 && tid == 0) p.info[2] = FUGAL_DEVICE_TIMEOUT;
+    };
+
+    for (int j = tid; j < span_n; j += kCgThreads) y_s[j] = j < n ? p.b[j] : 0.0;
+    double rr = 0.0;
+    for (int k = tid; k < own; k += kCgThreads) {
+        x_s[k] = rx_s[k] = p.a[o0 + k];
+        ry_s[k] = p.b[o0 + k];
+        zx_s[k] = zy_s[k] = 0.0;
+        rr += rx_s[k] * rx_s[k] + ry_s[k] * ry_s[k];
+    }
+    rr = block_sum(rr, scratch);
+    if (tid == 0) p.dots[blockIdx.x] = rr;
+    if (!barrier()) return give_up();
+    double rs = grid_total(p.dots, scratch);
+    const double norm = sqrt(rs);
+    double rel = 0.0;
+    int it = 0;
+    if (norm > 0.0) {
+        while (it < p.max_iter) {
+            ++it;
+            // ---- P y for the CTA's rows, partial P^T x
+            for (int c0 = 0; c0 < n; c0 += SPAN) {
+                double yq[4], cs[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) yq[q] = y_s[column(c0, q)];
+                for (int r0 = 0; r0 < own; r0 += kCgRows) {
+                    float4 m[kCgRows];
+#pragma unroll
+                    for (int r = 0; r < kCgRows; ++r) {
+                        m[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (r0 + r < own) {
+                            const float* row = p.P + static_cast<size_t>(o0 + r0 + r) * p.ldp;
+                            if (VEC) {  // n is a multiple of 4
+                                if (column(c0, 0) < n) m[r] = __ldg(reinterpret_cast<const float4*>(row + column(c0, 0)));
+                            } else {
+                                if (column(c0, 0) < n) m[r].x = __ldg(row + column(c0, 0));
+                                if (column(c0, 1) < n) m[r].y = __ldg(row + column(c0, 1));
+                                if (column(c0, 2) < n) m[r].z = __ldg(row + column(c0, 2));
+                                if (column(c0, 3) < n) m[r].w = __ldg(row + column(c0, 3));
+                            }
+                        }
+                    }
+                    double rsum[kCgRows];
+#pragma unroll
+                    for (int r = 0; r < kCgRows; ++r) {
+                        const double x = r0 + r < own ? x_s[r0 + r] : 0.0;
+                        const double d0 = m[r].x, d1 = m[r].y, d2 = m[r].z, d3 = m[r].w;
+                        rsum[r] = fma(d3, yq[3], fma(d2, yq[2], fma(d1, yq[1], d0 * yq[0])));
+                        cs[0] = fma(d0, x, cs[0]);
+                        cs[1] = fma(d1, x, cs[1]);
+                        cs[2] = fma(d2, x, cs[2]);
+                        cs[3] = fma(d3, x, cs[3]);
+                    }
+                    const double s = warp_sum8(rsum);
+                    const int r = r0 + (lane >> 2);
+                    if ((lane & 3) == 0 && r < own) red[warp][r] = (c0 == 0 ? 0.0 : red[warp][r]) + s;
+                }
+                double* cp = p.colpart + static_cast<size_t>(blockIdx.x) * n;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (column(c0, q) < n) cp[column(c0, q)] = cs[q];
+            }
+            if (!barrier()) return give_up();
+            // ---- A p on the CTA's rows and columns, <p, A p>
+            double dot = 0.0;
+            for (int k = tid; k < own; k += kCgThreads) {
+                double s = 0.0;
+#pragma unroll
+                for (int w = 0; w < kCgWarps; ++w) s += red[w][k];
+                apx_s[k] = x_s[k] + s;
+                dot += x_s[k] * apx_s[k];
+            }
+            __syncthreads();  // red is read
+            for (int k0 = 0; k0 < own; k0 += 32) {
+                const int k = k0 + lane;
+                const int ctas = static_cast<int>(gridDim.x);
+                double s = 0.0;
+                if (k < own) {
+                    for (int c0 = warp; c0 < ctas; c0 += 10 * kCgWarps) {
+                        double v[10];
+#pragma unroll
+                        for (int u = 0; u < 10; ++u) {
+                            const int c = c0 + u * kCgWarps;
+                            v[u] = c < ctas ? __ldcg(p.colpart + static_cast<size_t>(c) * n + o0 + k) : 0.0;
+                        }
+#pragma unroll
+                        for (int u = 0; u < 10; ++u) s += v[u];
+                    }
+                    red[warp][k] = s;
+                }
+            }
+            __syncthreads();
+            for (int k = tid; k < own; k += kCgThreads) {
+                double s = 0.0;
+#pragma unroll
+                for (int w = 0; w < kCgWarps; ++w) s += red[w][k];
+                const double yk = y_s[o0 + k];
+                apy_s[k] = s + yk;
+                dot += yk * apy_s[k];
+            }
+            dot = block_sum(dot, scratch);
+            if (tid == 0) p.dots[gridDim.x + blockIdx.x] = dot;
+            if (!barrier()) return give_up();
+            const double step = rs / grid_total(p.dots + gridDim.x, scratch);
+            // ---- solution and residual
+            rr = 0.0;
+            for (int k = tid; k < own; k += kCgThreads) {
+                zx_s[k] += step * x_s[k];
+                zy_s[k] += step * y_s[o0 + k];
+                const double rx = rx_s[k] - step * apx_s[k], ry = ry_s[k] - step * apy_s[k];
+                rx_s[k] = rx;
+                ry_s[k] = ry;
+                p.r_cols[o0 + k] = ry;
+                rr += rx * rx + ry * ry;
+            }
+            rr = block_sum(rr, scratch);
+            if (tid == 0) p.dots[blockIdx.x] = rr;
+            if (!barrier()) return give_up();
+            const double rs_new = grid_total(p.dots, scratch);
+            rel = sqrt(rs_new) / norm;
+            if (rel < p.tol) break;
+            const double ratio = rs_new / rs;
+            rs = rs_new;
+            for (int k = tid; k < own; k += kCgThreads) x_s[k] = rx_s[k] + ratio * x_s[k];
+            for (int j = tid; j < n; j += kCgThreads) y_s[j] = __ldcg(p.r_cols + j) + ratio * y_s[j];
+            __syncthreads();
+        }
+    }
+    for (int k = tid; k < own; k += kCgThreads) {
+        p.alpha[o0 + k] = zx_s[k];
+        p.beta[o0 + k] = zy_s[k];
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+        p.info[0] = it;
+        p.info[1] = rel;
+        p.info[2] = 0.0;
     }
 }
 
@@ -206,7 +467,9 @@ extern "C" fugal_status fugal_sinkhorn_plan(const float* cost32, int64_t ld32, i
 extern "C" fugal_status fugal_plan_matvec_workspace_size(int64_t n, size_t* bytes) {
     if (bytes == nullptr) return fail(FUGAL_BAD_ARGUMENT, "fugal_plan_matvec_workspace_size: null output");
     if (n <= 0 || n > (1ll << 30)) return fail(FUGAL_BAD_SHAPE, "fugal_plan_matvec_workspace_size: bad n");
-    const int64_t cb = (n + kMvCols - 1) / kMvCols, rb = (n + kMvRows - 1) / kMvRows;
+    // row partials of every column block, column partials of every row block (the
+    // unrolled step's blocks are the smaller ones)
+    const int64_t cb = (n + kMvCols - 1) / kMvCols, rb = (n + kUnRows - 1) / kUnRows;
     *bytes = static_cast<size_t>((cb + rb) * n) * 8 + 256;
     return FUGAL_OK;
 }
@@ -233,9 +496,9 @@ extern "C" fugal_status fugal_plan_matvec(const float* P, int64_t ldp, const flo
     }
     {
         LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-        const int blocks = static_cast<int>(std::min<int64_t>((n + 255) / 256, 4 * sm_count()));
-        matvec_merge_kernel<<<blocks, 256, 0, stream>>>(row_part, cb, nn, Py);
-        matvec_merge_kernel<<<blocks, 256, 0, stream>>>(col_part, rb, nn, Ptx);
+        const unsigned blocks = static_cast<unsigned>((n + 31) / 32);
+        merge_add_kernel<<<blocks, 256, 0, stream>>>(row_part, cb, nn, Py, 0);
+        merge_add_kernel<<<blocks, 256, 0, stream>>>(col_part, rb, nn, Ptx, 0);
         FUGAL_TRY(launch_check("fugal_plan_matvec: merge"));
     }
     return FUGAL_OK;
@@ -251,6 +514,78 @@ extern "C" fugal_status fugal_sinkhorn_adjoint(const float* P, int64_t ldp, cons
     LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
     adjoint_kernel<<<ew2d(n), 256, 0, stream>>>(P, ldp, G, ldg, static_cast<int>(n), alpha, beta, scale, out, ldo);
     return launch_check("fugal_sinkhorn_adjoint");
+}
+
+namespace {
+int cg_ctas(int64_t n) { return static_cast<int>(std::min<int64_t>(sm_count(), n)); }
+}  // namespace
+
+extern "C" fugal_status fugal_sinkhorn_adjoint_solve_workspace_size(int64_t n, size_t* bytes) {
+    if (bytes == nullptr)
+        return fail(FUGAL_BAD_ARGUMENT, "fugal_sinkhorn_adjoint_solve_workspace_size: null output");
+    if (n <= 0 || n > FUGAL_ADJOINT_SOLVE_MAX_N)
+        return fail(FUGAL_BAD_SHAPE, "fugal_sinkhorn_adjoint_solve_workspace_size: n must be in [1, %d]",
+                    FUGAL_ADJOINT_SOLVE_MAX_N);
+    // barrier and status words, dot products, column residual, column partials
+    *bytes = 256 + static_cast<size_t>(2 * cg_ctas(n) + n + cg_ctas(n) * n) * 8;
+    return FUGAL_OK;
+}
+
+extern "C" fugal_status fugal_sinkhorn_adjoint_solve(const float* P, int64_t ldp, int64_t n, const double* a,
+                                                     const double* b, double tol, int max_iter, double* alpha,
+                                                     double* beta, double* info, void* workspace,
+                                                     size_t workspace_bytes, fugal_stream_t stream_) {
+    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+    const char* who = "fugal_sinkhorn_adjoint_solve";
+    static_assert(kCgMaxN == FUGAL_ADJOINT_SOLVE_MAX_N, "the header's limit");
+    size_t need = 0;
+    FUGAL_TRY(fugal_sinkhorn_adjoint_solve_workspace_size(n, &need));
+    if (P == nullptr || a == nullptr || b == nullptr || alpha == nullptr || beta == nullptr || info == nullptr ||
+        workspace == nullptr)
+        return fail(FUGAL_BAD_ARGUMENT, "%s: null argument", who);
+    if (ldp < n) return fail(FUGAL_BAD_SHAPE, "%s: ldp < n", who);
+    if (workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 7u) != 0)
+        return fail(FUGAL_WORKSPACE_TOO_SMALL, "%s: workspace %zu < %zu bytes", who, workspace_bytes, need);
+    CgArgs args{};
+    args.P = P;
+    args.ldp = ldp;
+    args.n = static_cast<int>(n);
+    int ctas = cg_ctas(n);
+    args.own = static_cast<int>((n + ctas - 1) / ctas);
+    if (args.own > kCgMaxOwn) return fail(FUGAL_UNSUPPORTED, "%s: too few SMs for n = %lld", who, (long long)n);
+    ctas = static_cast<int>((n + args.own - 1) / args.own);
+    args.a = a;
+    args.b = b;
+    args.tol = tol;
+    args.max_iter = max_iter;
+    args.alpha = alpha;
+    args.beta = beta;
+    args.info = info;
+    char* w = static_cast<char*>(workspace);
+    args.arrivals = reinterpret_cast<unsigned*>(w);
+    args.status = reinterpret_cast<int*>(w + 8);
+    args.dots = reinterpret_cast<double*>(w + 256);
+    args.r_cols = args.dots + 2 * cg_ctas(n);
+    args.colpart = args.r_cols + n;
+    FUGAL_TRY(cuda_check(cudaMemsetAsync(w, 0, 256, stream), who));
+    // float4 rows: aligned, and whole quads (else one column per lane and load)
+    const bool vec = (n % 4) == 0 && (ldp % 4) == 0 && aligned16(P);
+    void (*fn)(CgArgs) = vec ? cg_kernel<true> : cg_kernel<false>;
+    const size_t span = kCgThreads * 4;
+    const size_t smem = (static_cast<size_t>(n) + span - 1) / span * span * 8;
+    FUGAL_TRY(cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), who));
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(ctas, 1, 1);
+    cfg.blockDim = dim3(kCgThreads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
+    return cuda_check(cudaLaunchKernelEx(&cfg, fn, args), who);
 }
 
 extern "C" fugal_status fugal_sinkhorn_unrolled_step_backward(const float* K, int64_t ldk, int64_t n,
@@ -269,7 +604,7 @@ extern "C" fugal_status fugal_sinkhorn_unrolled_step_backward(const float* K, in
     if (workspace_bytes < need)
         return fail(FUGAL_WORKSPACE_TOO_SMALL, "fugal_sinkhorn_unrolled_step_backward: workspace too small");
     const int nn = static_cast<int>(n);
-    const int cb = static_cast<int>((n + kMvCols - 1) / kMvCols), rb = static_cast<int>((n + kMvRows - 1) / kMvRows);
+    const int cb = static_cast<int>((n + kMvCols - 1) / kMvCols), rb = static_cast<int>((n + kUnRows - 1) / kUnRows);
     double* row_part = static_cast<double*>(workspace);
     double* col_part = row_part + static_cast<size_t>(cb) * n;
     {
@@ -280,11 +615,11 @@ extern "C" fugal_status fugal_sinkhorn_unrolled_step_backward(const float* K, in
     }
     {
         LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-        const int blocks = static_cast<int>(std::min<int64_t>((n + 255) / 256, 4 * sm_count()));
+        const unsigned blocks = static_cast<unsigned>((n + 31) / 32);
         if (axis == 0)
-            merge_add_kernel<<<blocks, 256, 0, stream>>>(row_part, cb, nn, g_other);
+            merge_add_kernel<<<blocks, 256, 0, stream>>>(row_part, cb, nn, g_other, 1);
         else
-            merge_add_kernel<<<blocks, 256, 0, stream>>>(col_part, rb, nn, g_other);
+            merge_add_kernel<<<blocks, 256, 0, stream>>>(col_part, rb, nn, g_other, 1);
         FUGAL_TRY(launch_check("fugal_sinkhorn_unrolled_step_backward: merge"));
     }
     return FUGAL_OK;

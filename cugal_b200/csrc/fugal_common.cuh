@@ -200,6 +200,39 @@ FUGAL_DEVICE bool mbar_wait(uint64_t* bar, uint32_t parity, int* err, uint32_t h
     return false;
 }
 
+// Grid-wide barrier of a cooperative launch (thread 0 of every CTA arrives and
+// waits, bounded; false in every thread of a CTA whose wait ran out or where a
+// thread passed ok = false).  The
+// arrival counter is a multiple of the grid whenever no barrier is in progress;
+// `target` is its value when this barrier is complete.
+FUGAL_DEVICE bool grid_barrier(unsigned* arrivals, int* status, bool ok, unsigned target, uint64_t limit_ns) {
+    __shared__ int passed;
+    if (!__syncthreads_and(ok)) return false;
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrivals) : "memory");
+        const uint64_t limit = limit_ns != 0 ? limit_ns : kWaitLimitNs;
+        uint64_t t0 = 0;
+        int good = 0;
+        for (uint32_t i = 0; i < kMaxPolls; ++i) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrivals) : "memory");
+            if (static_cast<int>(v - target) >= 0) {
+                good = 1;
+                break;
+            }
+            if ((i & 63u) == 63u) {
+                const uint64_t now = global_timer_ns();
+                if (t0 == 0) t0 = now;
+                if (now - t0 > limit || *reinterpret_cast<volatile int*>(status) != 0) break;
+            }
+        }
+        if (!good) report_error(status, FUGAL_DEVICE_TIMEOUT);
+        passed = good;
+    }
+    __syncthreads();
+    return passed != 0;
+}
+
 // 1-D bulk copy global -> this CTA's shared memory, completing on `bar`.
 // Both addresses 16-byte aligned, bytes a multiple of 16.
 FUGAL_DEVICE void bulk_load(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {

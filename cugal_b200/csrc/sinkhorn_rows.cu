@@ -95,37 +95,6 @@ FUGAL_DEVICE void load16(const T* stage, int c, int gt, float2* v) {
         Pairs<T>::unpack(*reinterpret_cast<const uint4*>(stage + ((c * (16 / V) + i) * GT + gt) * V), v + i * V / 2);
 }
 
-// Grid-wide barrier (thread 0 of every CTA arrives and waits, bounded).  The
-// arrival counter is a multiple of the grid whenever no barrier is in progress;
-// `target` is its value when this barrier is complete.
-FUGAL_DEVICE bool grid_barrier(SolveState* st, bool ok, unsigned target, unsigned long long limit_ns) {
-    __shared__ int passed;
-    if (!__syncthreads_and(ok)) return false;
-    if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->arrivals) : "memory");
-        const uint64_t limit = limit_ns != 0 ? limit_ns : kWaitLimitNs;
-        uint64_t t0 = 0;
-        int good = 0;
-        for (uint32_t i = 0; i < kMaxPolls; ++i) {
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&st->arrivals) : "memory");
-            if (static_cast<int>(v - target) >= 0) {
-                good = 1;
-                break;
-            }
-            if ((i & 63u) == 63u) {
-                const uint64_t now = global_timer_ns();
-                if (t0 == 0) t0 = now;
-                if (now - t0 > limit || *reinterpret_cast<volatile int*>(&st->status) != 0) break;
-            }
-        }
-        if (!good) report_error(&st->status, FUGAL_DEVICE_TIMEOUT);
-        passed = good;
-    }
-    __syncthreads();
-    return passed != 0;
-}
-
 // Column sums and column duals (b log2 e) of a thread's EPT columns: in registers
 // up to 32 columns, else in tensor memory, 16 columns per access.
 template <int EPT, bool REG = (EPT <= 32)>
@@ -664,13 +633,13 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
             }
         }
         arrivals += gridDim.x;
-        if (!grid_barrier(p.st, alive, arrivals, p.wait_limit_ns)) {  // the same in every thread of the CTA
+        if (!grid_barrier(&p.st->arrivals, &p.st->status, alive, arrivals, p.wait_limit_ns)) {  // the same in every thread of the CTA
             alive = false;
             break;
         }
         reduce_columns(p, t, gridDim.x * (DUMP ? 1 : GR));
         arrivals += gridDim.x;
-        if (!grid_barrier(p.st, true, arrivals, p.wait_limit_ns)) {
+        if (!grid_barrier(&p.st->arrivals, &p.st->status, true, arrivals, p.wait_limit_ns)) {
             alive = false;
             break;
         }

@@ -226,6 +226,16 @@ fugal_status fugal_plan_matvec(const float* P, int64_t ldp, const float* W, int6
 fugal_status fugal_sinkhorn_adjoint(const float* P, int64_t ldp, const float* G, int64_t ldg, int64_t n,
                                     const double* alpha, const double* beta, double scale, float* out, int64_t ldo,
                                     fugal_stream_t stream);
+/* The implicit adjoint's linear system [I P; P^T I] [alpha; beta] = [a; b] by
+ * conjugate gradients from zero (all of it on the device, FP64 vectors), until the
+ * residual is below tol * |[a; b]| or max_iter iterations.  info (DEVICE, 3
+ * doubles): iterations, relative residual, status (FUGAL_OK or
+ * FUGAL_DEVICE_TIMEOUT, alpha and beta then NaN).  No counterpart in the reference. */
+#define FUGAL_ADJOINT_SOLVE_MAX_N 16384
+fugal_status fugal_sinkhorn_adjoint_solve_workspace_size(int64_t n, size_t* bytes);
+fugal_status fugal_sinkhorn_adjoint_solve(const float* P, int64_t ldp, int64_t n, const double* a, const double* b,
+                                          double tol, int max_iter, double* alpha, double* beta, double* info,
+                                          void* workspace, size_t workspace_bytes, fugal_stream_t stream);
 /* Unrolled backward of one half step of the log-domain iteration (no momentum),
  * for the checkpointed unrolled adjoint.  axis 1: out = -LSE_j(K_ij + other_j)
  * (row update); axis 0: out = -LSE_i(K_ij + other_i) (column update).  With
