@@ -596,7 +596,55 @@ __global__ void __launch_bounds__(kStructThreads, 4) gradient_structural_kernel(
     }
 }
 
-// out^T[j][i] = sign * sum_{k in N(i)} Q[j][k]  (M = Q^T operand of the reference's adjacency_matmul)
+// out^T[j][i] = sign * sum_{k in N(i)} Q[j][k]  (M = Q^T operand of the reference's
+// adjacency_matmul).  A CTA keeps R rows of Q in shared memory, interleaved (the R
+// values of column k side by side), and walks the nodes i: one read of a column index
+// and one shared-memory access of 4 R bytes serve R outputs, each summed in CSR order.
+// With one row of Q per block and its values gathered from L1 the column indices were
+// read once per output row: 3.32 ms at n = 8192, mean degree 12, against 0.28 ms for
+// the other operand layout.  R = 4 up to 14000 columns, 2 and 1 up to 57000, by what
+// shared memory holds; wider rows gather from global memory.
+constexpr int kTransposedThreads = 1024;
+template <int R>
+__global__ void __launch_bounds__(kTransposedThreads) spmm_transposed_rows_kernel(
+    const int* __restrict__ rp, const int* __restrict__ col, const float* __restrict__ Q, long long ldq, int n,
+    float* __restrict__ outT, long long ldo, float sign) {
+    extern __shared__ __align__(16) float q_s[];  // [n][R]
+    const int j0 = blockIdx.x * R;
+    for (int k = threadIdx.x; k < n; k += kTransposedThreads) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) q_s[static_cast<size_t>(k) * R + r] = j0 + r < n ? Q[row_offset(j0 + r, ldq) + k] : 0.f;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kTransposedThreads) {
+        float acc[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r] = 0.f;
+        const int e1 = rp[i + 1];
+#pragma unroll 4
+        for (int e = rp[i]; e < e1; ++e) {
+            const float* q = q_s + static_cast<size_t>(__ldg(col + e)) * R;
+            if constexpr (R == 4) {
+                const float4 v = *reinterpret_cast<const float4*>(q);
+                acc[0] += v.x;
+                acc[1] += v.y;
+                acc[2] += v.z;
+                acc[3] += v.w;
+            } else if constexpr (R == 2) {
+                const float2 v = *reinterpret_cast<const float2*>(q);
+                acc[0] += v.x;
+                acc[1] += v.y;
+            } else {
+                acc[0] += *q;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (j0 + r < n) outT[row_offset(j0 + r, ldo) + i] = sign * acc[r];
+    }
+}
+
+// The same with Q gathered from global memory (rows wider than shared memory).
 __global__ void spmm_transposed_operand_kernel(const int* __restrict__ rp, const int* __restrict__ col,
                                                const float* __restrict__ Q, long long ldq, int n,
                                                float* __restrict__ outT, long long ldo, float sign) {
@@ -607,6 +655,18 @@ __global__ void spmm_transposed_operand_kernel(const int* __restrict__ rp, const
     const float* qrow = Q + static_cast<size_t>(j) * ldq;
     for (int e = rp[i]; e < rp[i + 1]; ++e) acc += qrow[col[e]];
     outT[static_cast<size_t>(j) * ldo + i] = sign * acc;
+}
+
+template <int R>
+fugal_status launch_transposed_rows(int64_t n, const int* rp, const int* col, const float* Q, int64_t ldq, float* outT,
+                                    int64_t ldo, float sign, cudaStream_t stream) {
+    const size_t smem = static_cast<size_t>(n) * R * sizeof(float);
+    FUGAL_TRY(cuda_check(cudaFuncSetAttribute(spmm_transposed_rows_kernel<R>,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+                         "fugal_adjacency_matmul: shared memory"));
+    spmm_transposed_rows_kernel<R><<<static_cast<unsigned>((n + R - 1) / R), kTransposedThreads, smem, stream>>>(
+        rp, col, Q, ldq, static_cast<int>(n), outT, ldo, sign);
+    return launch_check("fugal_adjacency_matmul");
 }
 
 // Launch-shape knobs of the gradient kernels.  FUGAL_GATHER_UNROLL: gathers in
@@ -668,6 +728,13 @@ extern "C" fugal_status fugal_adjacency_matmul(const int32_t* col_indices, const
             spmm_kernel<false><<<grid, kSpmmThreads, 0, stream>>>(row_pointers, col_indices, M, ldm,
                                                                    static_cast<int>(n), out, ldo, 0, sign);
     } else {
+        constexpr int64_t kRoom = 224 * 1024 / sizeof(float);  // floats of Q a CTA can hold
+        if (n * 4 <= kRoom)
+            return launch_transposed_rows<4>(n, row_pointers, col_indices, M, ldm, out, ldo, sign, stream);
+        if (n * 2 <= kRoom)
+            return launch_transposed_rows<2>(n, row_pointers, col_indices, M, ldm, out, ldo, sign, stream);
+        if (n <= kRoom)
+            return launch_transposed_rows<1>(n, row_pointers, col_indices, M, ldm, out, ldo, sign, stream);
         dim3 grid(static_cast<unsigned>(n), static_cast<unsigned>((n + 127) / 128));
         spmm_transposed_operand_kernel<<<grid, 128, 0, stream>>>(row_pointers, col_indices, M, ldm,
                                                                  static_cast<int>(n), out, ldo, sign);

@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <initializer_list>
 
 #include "fugal_common.cuh"
 #include "fugal_host.h"
@@ -18,12 +19,6 @@
 namespace fugal {
 
 constexpr int kEwThreads = 256;
-
-// Grid over (row, 1024-column chunk): blockIdx.x = row, blockIdx.y = chunk;
-// each thread handles 4 consecutive columns.
-inline dim3 ew_grid(int64_t n) {
-    return dim3(static_cast<unsigned>(n), static_cast<unsigned>((n + kEwThreads * 4 - 1) / (kEwThreads * 4)));
-}
 
 // Where the update records the plan's nonzero entries (fugal_fw_update_collect):
 // per row k, counts[k] entries (column, q) at entries[k * slots ...] in no
@@ -107,116 +102,279 @@ __global__ void commit_duals_kernel(const float* u, const float* v, double* U, d
     }
 }
 
+// The reference-compatible elementwise kernels walk rows grid-strided, a thread
+// taking 4 consecutive columns with one 16-byte access each (VEC: aligned rows of
+// whole quads), else one column per access (coalesced either way).  With 4 scalar
+// accesses of stride 16 bytes per thread and one block per 1024 columns they ran at
+// 23 to 70% of the copy peak at n = 8192 (update 177 us, regularize 326, distance 544).
+constexpr int kEwCols = kEwThreads * 4;
+inline dim3 ew_blocks(int64_t n) {
+    const int64_t chunks = (n + kEwCols - 1) / kEwCols;
+    const int64_t rows = std::max<int64_t>(1, std::min<int64_t>(n, (static_cast<int64_t>(sm_count()) * 32) / chunks));
+    return dim3(static_cast<unsigned>(chunks), static_cast<unsigned>(rows));
+}
+// Column q (of 4) of this thread, and the access to its four columns of a row.
+template <bool VEC>
+FUGAL_DEVICE int ew_column(int q) {
+    return VEC ? static_cast<int>(blockIdx.x) * kEwCols + static_cast<int>(threadIdx.x) * 4 + q
+               : static_cast<int>(blockIdx.x) * kEwCols + q * kEwThreads + static_cast<int>(threadIdx.x);
+}
+template <bool VEC>
+FUGAL_DEVICE void ew_load(const float* row, int n, float (&v)[4]) {
+    if (VEC) {
+        const int c = ew_column<true>(0);
+        const float4 x = c < n ? *reinterpret_cast<const float4*>(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int c = ew_column<false>(q);
+            v[q] = c < n ? row[c] : 0.f;
+        }
+    }
+}
+template <bool VEC>
+FUGAL_DEVICE void ew_store(float* row, int n, const float (&v)[4]) {
+    if (VEC) {
+        const int c = ew_column<true>(0);
+        if (c < n) *reinterpret_cast<float4*>(row + c) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int c = ew_column<false>(q);
+            if (c < n) row[c] = v[q];
+        }
+    }
+}
+
 // Reference form: scaled = exp(K + v_c + u_r); gap += (scaled - P)(K * -reg); P += (scaled - P) alpha.
+template <bool VEC>
 __global__ void __launch_bounds__(kEwThreads) update_log_kernel(float* __restrict__ P, long long ldp,
                                                                 const float* __restrict__ K, long long ldk,
                                                                 const float* __restrict__ u,
                                                                 const float* __restrict__ v, int n, float alpha,
                                                                 float reg, double* gap) {
     __shared__ double red[32];
-    const int i = blockIdx.x;
-    const int j0 = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     double g = 0.0;
-    for (int j = j0; j < min(n, j0 + 4); ++j) {
-        const float k = K[static_cast<size_t>(i) * ldk + j];
-        float& p = P[static_cast<size_t>(i) * ldp + j];
-        const float scaled = expf(k + v[j] + u[i]);
-        const float diff = scaled - p;
-        g += static_cast<double>(diff) * static_cast<double>(k * -reg);
-        p = __fadd_rn(p, __fmul_rn(diff, alpha));
+    float vv[4];
+    ew_load<VEC>(v, n, vv);
+    for (int i = blockIdx.y; i < n; i += gridDim.y) {
+        float k[4], p[4];
+        ew_load<VEC>(K + static_cast<size_t>(i) * ldk, n, k);
+        ew_load<VEC>(P + static_cast<size_t>(i) * ldp, n, p);
+        const float ui = u[i];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (ew_column<VEC>(q) >= n) continue;
+            const float scaled = expf(k[q] + vv[q] + ui);
+            const float diff = scaled - p[q];
+            g += static_cast<double>(diff) * static_cast<double>(k[q] * -reg);
+            p[q] = __fadd_rn(p[q], __fmul_rn(diff, alpha));
+        }
+        ew_store<VEC>(P + static_cast<size_t>(i) * ldp, n, p);
     }
     g = block_sum(g, red);
     if (threadIdx.x == 0) atomicAdd(gap, g);
 }
 
 // gradient += it - (2 it) * P, unfused IEEE operations in the reference's order.
-__global__ void regularize_kernel(float* G, long long ldg, const float* P, long long ldp, int n, int it) {
-    const int i = blockIdx.x;
-    const int j0 = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
-    for (int j = j0; j < min(n, j0 + 4); ++j) {
-        float& g = G[static_cast<size_t>(i) * ldg + j];
-        const float t = __fmul_rn(static_cast<float>(it * 2), P[static_cast<size_t>(i) * ldp + j]);
-        g = __fadd_rn(g, __fsub_rn(static_cast<float>(it), t));
+template <bool VEC>
+__global__ void __launch_bounds__(kEwThreads) regularize_kernel(float* G, long long ldg, const float* P, long long ldp,
+                                                                int n, int it) {
+    for (int i = blockIdx.y; i < n; i += gridDim.y) {
+        float g[4], p[4];
+        ew_load<VEC>(G + static_cast<size_t>(i) * ldg, n, g);
+        ew_load<VEC>(P + static_cast<size_t>(i) * ldp, n, p);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float t = __fmul_rn(static_cast<float>(it * 2), p[q]);
+            g[q] = __fadd_rn(g[q], __fsub_rn(static_cast<float>(it), t));
+        }
+        ew_store<VEC>(G + static_cast<size_t>(i) * ldg, n, g);
     }
 }
 
 // out[x][y] += sqrtf(sum_i (s[x][i] - t[y][i])^2), squares of FP32 differences summed in double
 // (the reference accumulates into `auto sum = 0.0`).
-__global__ void add_distance_kernel(const float* s, const float* t, int n, float* out, long long ldo) {
-    const int x = blockIdx.x;
-    const int y0 = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
-    const float a0 = s[4 * x], a1 = s[4 * x + 1], a2 = s[4 * x + 2], a3 = s[4 * x + 3];
-    for (int y = y0; y < min(n, y0 + 4); ++y) {
-        double sum = 0.0;
-        const float d0 = a0 - t[4 * y], d1 = a1 - t[4 * y + 1], d2 = a2 - t[4 * y + 2], d3 = a3 - t[4 * y + 3];
-        sum += __fmul_rn(d0, d0);
-        sum += __fmul_rn(d1, d1);
-        sum += __fmul_rn(d2, d2);
-        sum += __fmul_rn(d3, d3);
-        out[static_cast<size_t>(x) * ldo + y] += sqrtf(static_cast<float>(sum));
+template <bool VEC>
+__global__ void __launch_bounds__(kEwThreads) add_distance_kernel(const float* s, const float* t, int n, float* out,
+                                                                  long long ldo) {
+    float f[4][4];  // features of this thread's columns
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int y = ew_column<VEC>(q);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) f[q][k] = y < n ? t[4 * static_cast<size_t>(y) + k] : 0.f;
+    }
+    for (int x = blockIdx.y; x < n; x += gridDim.y) {
+        float o[4], a[4];
+        ew_load<VEC>(out + static_cast<size_t>(x) * ldo, n, o);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) a[k] = s[4 * static_cast<size_t>(x) + k];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            double sum = 0.0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float d = a[k] - f[q][k];
+                sum += __fmul_rn(d, d);
+            }
+            o[q] += sqrtf(static_cast<float>(sum));
+        }
+        ew_store<VEC>(out + static_cast<size_t>(x) * ldo, n, o);
     }
 }
 
+// A row of up to 8192 elements in registers: quad k of thread t starts
+// at column 4 (256 k + t) with float4 loads (VEC), else column q 256 + t of each 1024.
+constexpr int kRowThreads = 256;
+template <bool VEC>
+FUGAL_DEVICE int row_column(int k, int q) {
+    return VEC ? (k * kRowThreads + static_cast<int>(threadIdx.x)) * 4 + q
+               : (k * 4 + q) * kRowThreads + static_cast<int>(threadIdx.x);
+}
+template <bool VEC>
+FUGAL_DEVICE float4 row_quad(const float* row, int k, int cols, float fill) {
+    if (VEC) {  // cols is a multiple of 4
+        const int c = row_column<true>(k, 0);
+        return c < cols ? *reinterpret_cast<const float4*>(row + c) : make_float4(fill, fill, fill, fill);
+    }
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int c = row_column<false>(k, q);
+        v[q] = c < cols ? row[c] : fill;
+    }
+    return make_float4(v[0], v[1], v[2], v[3]);
+}
+
 // out[r] = (1-w) out[r] - w LSE_c(K[r,c] + add[c]) (w == 1 within 1e-4: out[r] = -LSE).
-__global__ void __launch_bounds__(256) log_step_kernel(const float* K, long long ldk, int cols, const float* add,
-                                                       float* out, float w) {
-    __shared__ float sm_m[32], sm_s[32];
+// One block per row, the row read once: QUADS float4 per thread stay in registers
+// between the maximum and the exponentials (rows up to
+// 8192), and longer rows (LONG) keep a running (max, sum) over pieces of 8192.
+// Bound by HBM: 172 us with two scalar passes over a row, 57 us here at n = 8192 (268
+// MB, 41 us at the copy peak).
+template <int QUADS, bool VEC, bool LONG>
+__global__ void __launch_bounds__(kRowThreads) log_step_kernel(const float* K, long long ldk, int cols,
+                                                               const float* add, float* out, float w) {
+    __shared__ float sm_m[kRowThreads / 32], sm_s[kRowThreads / 32];
     const int r = blockIdx.x;
-    const float* row = K + static_cast<size_t>(r) * ldk;
-    float m = -INFINITY;
-    for (int c = threadIdx.x; c < cols; c += blockDim.x) m = fmaxf(m, row[c] + add[c]);
-    m = warp_max(m);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (lane == 0) sm_m[warp] = m;
-    __syncthreads();
-    float M = -INFINITY;
-    for (int q = 0; q < nw; ++q) M = fmaxf(M, sm_m[q]);
-    const float base = (M == -INFINITY) ? 0.f : M;
-    float s = 0.f;
-    for (int c = threadIdx.x; c < cols; c += blockDim.x) s += expf(row[c] + add[c] - base);
-    s = warp_sum(s);
-    if (lane == 0) sm_s[warp] = s;
-    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float M = -INFINITY, S = 0.f;
+    constexpr int PIECE = QUADS * 4 * kRowThreads;
+    for (int c0 = 0; c0 < (LONG ? cols : 1); c0 += PIECE) {
+        const float* row = K + static_cast<size_t>(r) * ldk + c0;
+        const float* ad = add + c0;
+        const int left = cols - c0;
+        float4 x[QUADS];
+#pragma unroll
+        for (int k = 0; k < QUADS; ++k) x[k] = row_quad<VEC>(row, k, left, -INFINITY);
+        float m = -INFINITY;
+#pragma unroll
+        for (int k = 0; k < QUADS; ++k) {
+            const float4 a4 = row_quad<VEC>(ad, k, left, 0.f);
+            x[k] = make_float4(x[k].x + a4.x, x[k].y + a4.y, x[k].z + a4.z, x[k].w + a4.w);
+            m = fmaxf(m, fmaxf(fmaxf(x[k].x, x[k].y), fmaxf(x[k].z, x[k].w)));
+        }
+        m = warp_max(m);
+        if (lane == 0) sm_m[warp] = m;
+        __syncthreads();
+        float Mp = M;
+#pragma unroll
+        for (int q = 0; q < kRowThreads / 32; ++q) Mp = fmaxf(Mp, sm_m[q]);
+        const float base = (Mp == -INFINITY) ? 0.f : Mp;
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < QUADS; ++k)
+            s += (expf(x[k].x - base) + expf(x[k].y - base)) + (expf(x[k].z - base) + expf(x[k].w - base));
+        s = warp_sum(s);
+        if (lane == 0) sm_s[warp] = s;
+        __syncthreads();
+        float piece = 0.f;
+#pragma unroll
+        for (int q = 0; q < kRowThreads / 32; ++q) piece += sm_s[q];
+        S = (LONG && c0 > 0 && M != -INFINITY ? S * expf(M - base) : 0.f) + piece;
+        M = Mp;
+        if (LONG) __syncthreads();  // the next piece writes sm_m, sm_s
+    }
     if (threadIdx.x == 0) {
-        float S = 0.f;
-        for (int q = 0; q < nw; ++q) S += sm_s[q];
         const float lse = M + logf(S);
         out[r] = (fabsf(w - 1.0f) < 1e-4f) ? -lse : (1.0f - w) * out[r] - w * lse;
     }
 }
 
-__global__ void __launch_bounds__(256) marginal_rows_kernel(const float* K, long long ldk, int n, const float* u,
-                                                            const float* v, double* result) {
+template <bool VEC>
+void launch_log_step(int64_t rows, const float* K, int64_t ldk, int cols, const float* add, float* out, float w,
+                     cudaStream_t stream) {
+    const unsigned grid = static_cast<unsigned>(rows);
+    if (cols <= 1024)
+        log_step_kernel<1, VEC, false><<<grid, kRowThreads, 0, stream>>>(K, ldk, cols, add, out, w);
+    else if (cols <= 2048)
+        log_step_kernel<2, VEC, false><<<grid, kRowThreads, 0, stream>>>(K, ldk, cols, add, out, w);
+    else if (cols <= 4096)
+        log_step_kernel<4, VEC, false><<<grid, kRowThreads, 0, stream>>>(K, ldk, cols, add, out, w);
+    else if (cols <= 8192)
+        log_step_kernel<8, VEC, false><<<grid, kRowThreads, 0, stream>>>(K, ldk, cols, add, out, w);
+    else
+        log_step_kernel<8, VEC, true><<<grid, kRowThreads, 0, stream>>>(K, ldk, cols, add, out, w);
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(kRowThreads) marginal_rows_kernel(const float* K, long long ldk, int n,
+                                                                    const float* u, const float* v, double* result) {
     __shared__ double red[32];
     const int r = blockIdx.x;
     const float* row = K + static_cast<size_t>(r) * ldk;
+    const float ur = u[r];
     double s = 0.0;
-    for (int c = threadIdx.x; c < n; c += blockDim.x) s += static_cast<double>(expf(row[c] + u[r] + v[c]));
+    const int quads = (n + 4 * kRowThreads - 1) / (4 * kRowThreads);
+#pragma unroll 4
+    for (int k = 0; k < quads; ++k) {
+        const float4 x = row_quad<VEC>(row, k, n, 0.f), a = row_quad<VEC>(v, k, n, 0.f);
+        const float e[4] = {x.x + ur + a.x, x.y + ur + a.y, x.z + ur + a.z, x.w + ur + a.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (row_column<VEC>(k, q) < n) s += static_cast<double>(expf(e[q]));
+    }
     s = block_sum(s, red);
     if (threadIdx.x == 0) atomicAdd(result, fabs(s - 1.0));
 }
 
-__global__ void __launch_bounds__(256) marginal_cols_kernel(const float* K, long long ldk, int n, const float* u,
-                                                            const float* v, double* result) {
-    __shared__ double red[32];
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    double dev = 0.0;
+// 32 columns per block (one per lane), 32 warps over the rows: enough loads in flight
+// for few columns (153 us at n = 1024 with one thread per column).
+__global__ void __launch_bounds__(1024) marginal_cols_kernel(const float* K, long long ldk, int n, const float* u,
+                                                             const float* v, double* result) {
+    __shared__ double part[32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c = blockIdx.x * 32 + lane;
+    double s = 0.0;
     if (c < n) {
-        double s = 0.0;
-        for (int r = 0; r < n; ++r) s += static_cast<double>(expf(K[static_cast<size_t>(r) * ldk + c] + u[r] + v[c]));
-        dev = fabs(s - 1.0);
+        const float vc = v[c];
+#pragma unroll 8
+        for (int r = warp; r < n; r += 32) s += static_cast<double>(expf(K[static_cast<size_t>(r) * ldk + c] + u[r] + vc));
     }
-    dev = block_sum(dev, red);
-    if (threadIdx.x == 0) atomicAdd(result, dev);
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < 32; ++w) t += part[w][lane];
+        const double dev = warp_sum(c < n ? fabs(t - 1.0) : 0.0);
+        if (lane == 0) atomicAdd(result, dev);
+    }
 }
 
-__global__ void count_le_kernel(const float* P, long long ldp, int n, float thr, unsigned long long* count) {
-    const int i = blockIdx.x;
-    const int j0 = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
-    int c = 0;
-    for (int j = j0; j < min(n, j0 + 4); ++j) c += (P[static_cast<size_t>(i) * ldp + j] <= thr) ? 1 : 0;
+template <bool VEC>
+__global__ void __launch_bounds__(kEwThreads) count_le_kernel(const float* P, long long ldp, int n, float thr,
+                                                              unsigned long long* count) {
+    int c = 0;  // at most 4 n per thread
+    for (int i = blockIdx.y; i < n; i += gridDim.y) {
+        float p[4];
+        ew_load<VEC>(P + static_cast<size_t>(i) * ldp, n, p);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+        for (int q = 0; q < 4; ++q) c += (ew_column<VEC>(q) < n && p[q] <= thr) ? 1 : 0;
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, static_cast<unsigned long long>(c));
 }
 
@@ -225,6 +383,18 @@ fugal_status check_square(const void* p, int64_t ld, int64_t n, const char* who,
     if (n <= 0 || n > (1ll << 30)) return fail(FUGAL_BAD_SHAPE, "%s: bad n", who);
     if (ld < n) return fail(FUGAL_BAD_SHAPE, "%s: leading dimension of %s < n", who, what);
     return FUGAL_OK;
+}
+
+// 16-byte accesses: whole quads in every row of every operand.
+struct EwRows {
+    const void* p;
+    int64_t ld;
+};
+bool ew_vec(int64_t n, std::initializer_list<EwRows> rows) {
+    if ((n % 4) != 0) return false;
+    for (const EwRows& r : rows)
+        if ((r.ld % 4) != 0 || !aligned16(r.p)) return false;
+    return true;
 }
 
 }  // namespace fugal
@@ -304,8 +474,11 @@ extern "C" fugal_status fugal_update_quasi_permutation_log(float* P, int64_t ldp
     if (u == nullptr || v == nullptr || gap == nullptr) return fail(FUGAL_BAD_ARGUMENT, "%s: null argument", who);
     FUGAL_TRY(cuda_check(cudaMemsetAsync(gap, 0, sizeof(double), stream), who));
     LaunchScope scope(FUGAL_KERNEL_UPDATE, stream);
-    update_log_kernel<<<ew_grid(n), kEwThreads, 0, stream>>>(P, ldp, K, ldk, u, v, static_cast<int>(n), alpha,
-                                                              regularization, gap);
+    const int ni = static_cast<int>(n);
+    if (ew_vec(n, {{P, ldp}, {K, ldk}, {v, 4}}))
+        update_log_kernel<true><<<ew_blocks(n), kEwThreads, 0, stream>>>(P, ldp, K, ldk, u, v, ni, alpha, regularization, gap);
+    else
+        update_log_kernel<false><<<ew_blocks(n), kEwThreads, 0, stream>>>(P, ldp, K, ldk, u, v, ni, alpha, regularization, gap);
     return launch_check(who);
 }
 
@@ -315,7 +488,10 @@ extern "C" fugal_status fugal_regularize(float* gradient, int64_t ldg, const flo
     FUGAL_TRY(check_square(gradient, ldg, n, "fugal_regularize", "gradient"));
     FUGAL_TRY(check_square(P, ldp, n, "fugal_regularize", "P"));
     LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-    regularize_kernel<<<ew_grid(n), kEwThreads, 0, stream>>>(gradient, ldg, P, ldp, static_cast<int>(n), iteration);
+    if (ew_vec(n, {{gradient, ldg}, {P, ldp}}))
+        regularize_kernel<true><<<ew_blocks(n), kEwThreads, 0, stream>>>(gradient, ldg, P, ldp, static_cast<int>(n), iteration);
+    else
+        regularize_kernel<false><<<ew_blocks(n), kEwThreads, 0, stream>>>(gradient, ldg, P, ldp, static_cast<int>(n), iteration);
     return launch_check("fugal_regularize");
 }
 
@@ -325,7 +501,10 @@ extern "C" fugal_status fugal_add_distance(const float* source, const float* tar
     FUGAL_TRY(check_square(out, ldo, n, "fugal_add_distance", "out"));
     if (source == nullptr || target == nullptr) return fail(FUGAL_BAD_ARGUMENT, "fugal_add_distance: null features");
     LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-    add_distance_kernel<<<ew_grid(n), kEwThreads, 0, stream>>>(source, target, static_cast<int>(n), out, ldo);
+    if (ew_vec(n, {{out, ldo}}))
+        add_distance_kernel<true><<<ew_blocks(n), kEwThreads, 0, stream>>>(source, target, static_cast<int>(n), out, ldo);
+    else
+        add_distance_kernel<false><<<ew_blocks(n), kEwThreads, 0, stream>>>(source, target, static_cast<int>(n), out, ldo);
     return launch_check("fugal_add_distance");
 }
 
@@ -338,8 +517,11 @@ extern "C" fugal_status fugal_sinkhorn_log_step(const float* K, int64_t rows, in
     if (rows <= 0 || cols <= 0 || ldk < cols || rows > (1ll << 31) - 1)
         return fail(FUGAL_BAD_SHAPE, "fugal_sinkhorn_log_step: bad shape");
     LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-    log_step_kernel<<<static_cast<unsigned>(rows), 256, 0, stream>>>(K, ldk, static_cast<int>(cols), add, out,
-                                                                      momentum);
+    // float4 rows need whole, aligned quads in K and add
+    if ((cols % 4) == 0 && (ldk % 4) == 0 && aligned16(K) && aligned16(add))
+        launch_log_step<true>(rows, K, ldk, static_cast<int>(cols), add, out, momentum, stream);
+    else
+        launch_log_step<false>(rows, K, ldk, static_cast<int>(cols), add, out, momentum, stream);
     return launch_check("fugal_sinkhorn_log_step");
 }
 
@@ -353,11 +535,14 @@ extern "C" fugal_status fugal_sinkhorn_log_marginal(const float* K, int64_t n, i
     if (axis != 0 && axis != 1) return fail(FUGAL_BAD_ARGUMENT, "fugal_sinkhorn_log_marginal: axis must be 0 or 1");
     FUGAL_TRY(cuda_check(cudaMemsetAsync(result, 0, sizeof(double), stream), "fugal_sinkhorn_log_marginal"));
     LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-    if (axis == 1)
-        marginal_rows_kernel<<<static_cast<unsigned>(n), 256, 0, stream>>>(K, ldk, static_cast<int>(n), u, v, result);
+    const unsigned rows = static_cast<unsigned>(n);
+    if (axis == 1 && (n % 4) == 0 && (ldk % 4) == 0 && aligned16(K) && aligned16(v))
+        marginal_rows_kernel<true><<<rows, kRowThreads, 0, stream>>>(K, ldk, static_cast<int>(n), u, v, result);
+    else if (axis == 1)
+        marginal_rows_kernel<false><<<rows, kRowThreads, 0, stream>>>(K, ldk, static_cast<int>(n), u, v, result);
     else
-        marginal_cols_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(K, ldk, static_cast<int>(n),
-                                                                                           u, v, result);
+        marginal_cols_kernel<<<static_cast<unsigned>((n + 31) / 32), 1024, 0, stream>>>(K, ldk, static_cast<int>(n), u,
+                                                                                         v, result);
     return launch_check("fugal_sinkhorn_log_marginal");
 }
 
@@ -368,7 +553,10 @@ extern "C" fugal_status fugal_count_le(const float* P, int64_t ldp, int64_t n, f
     if (count == nullptr) return fail(FUGAL_BAD_ARGUMENT, "fugal_count_le: null count");
     FUGAL_TRY(cuda_check(cudaMemsetAsync(count, 0, sizeof(int64_t), stream), "fugal_count_le"));
     LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-    count_le_kernel<<<ew_grid(n), kEwThreads, 0, stream>>>(P, ldp, static_cast<int>(n), threshold,
-                                                            reinterpret_cast<unsigned long long*>(count));
+    unsigned long long* total = reinterpret_cast<unsigned long long*>(count);
+    if (ew_vec(n, {{P, ldp}}))
+        count_le_kernel<true><<<ew_blocks(n), kEwThreads, 0, stream>>>(P, ldp, static_cast<int>(n), threshold, total);
+    else
+        count_le_kernel<false><<<ew_blocks(n), kEwThreads, 0, stream>>>(P, ldp, static_cast<int>(n), threshold, total);
     return launch_check("fugal_count_le");
 }

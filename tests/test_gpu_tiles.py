@@ -26,6 +26,73 @@ def _csr_graph(lengths, n, seed):
     return torch.from_numpy(rng.permutation(e)).cuda()
 
 
+@pytest.mark.parametrize("ld_pad,offset", [(0, 0), (3, 0), (0, 1)])
+@pytest.mark.parametrize("cols", [1, 3, 1023, 1024, 1028, 2052, 4100, 8192, 8196, 20001])
+def test_log_step_widths(cols, ld_pad, offset):
+    """Rows in registers (up to 8192 columns) and in pieces, 16-byte and scalar access: relative error of
+    the FP32 LSE, at most a few ulp of the largest term plus the summation's sqrt(cols) 2^-24."""
+    from cugal_b200 import _native as N
+    rows, g = 37, _gen(cols)
+    buf = torch.randn(offset + rows * (cols + ld_pad), generator=g, device="cuda") * 5
+    K = buf[offset:].view(rows, cols + ld_pad)[:, :cols]
+    add, out = torch.randn(cols, generator=g, device="cuda"), torch.randn(rows, generator=g, device="cuda")
+    add[cols // 2:cols // 2 + 1] = float("-inf") if cols > 1 else 0.0
+    old = out.clone()
+    for w in (1.0, 0.6):
+        out.copy_(old)
+        N.call("fugal_sinkhorn_log_step", K.data_ptr(), rows, cols, K.stride(0), add.data_ptr(), out.data_ptr(), w,
+               N.stream_handle())
+        lse = torch.logsumexp(K.double() + add.double(), 1)
+        ref = -lse if w == 1.0 else (1 - w) * old.double() - w * lse
+        assert (out.double() - ref).abs().max() < 4e-6 * max(1.0, float(lse.abs().max()))
+
+
+@pytest.mark.parametrize("n,ld_pad", [(1, 0), (3, 1), (1000, 0), (1000, 3), (1025, 0), (2052, 4)])
+def test_elementwise_access(n, ld_pad):
+    """regularize, add_distance, the log update, count_le and the marginals with whole 16-byte rows and
+    without: the FP32 operations of the reference, bit for bit where it fixes them."""
+    from cugal_b200 import _native as N
+    from cugal_b200 import cuda_kernels as ck
+    g = _gen(n + ld_pad)
+    new = lambda s: (torch.randn((n, n + ld_pad), generator=g, device="cuda") * s)[:, :n]
+    G, P, K = new(1.0), new(0.1).abs(), new(2.0) - 6
+    fs, ft = (torch.rand((n, 4), generator=g, device="cuda") * 9 for _ in range(2))
+    u, v = (torch.randn(n, generator=g, device="cuda") for _ in range(2))
+    ref = G + (3.0 - 6.0 * P)
+    ck.regularize(G, P, 3)
+    assert torch.equal(G, ref)
+    d = (fs[:, None, :] - ft[None, :, :]).square().double().sum(2).float().sqrt()
+    out = G.clone()
+    ck.add_distance(fs, ft, out)
+    assert torch.equal(out, G + d)
+    count = torch.zeros(1, dtype=torch.int64, device="cuda")
+    N.call("fugal_count_le", P.data_ptr(), P.stride(0), n, 0.05, count.data_ptr(), N.stream_handle())
+    assert int(count.item()) == int((P <= 0.05).sum())
+    q = torch.exp(K.double() + v.double() + u.double()[:, None])
+    assert abs(ck.sinkhorn_log_marginal(K, u, v) - float((q.sum(1) - 1).abs().sum())) < 1e-5 * float(q.sum() + n)
+    err = torch.zeros(1, dtype=torch.float64, device="cuda")
+    N.call("fugal_sinkhorn_log_marginal", K.data_ptr(), n, K.stride(0), u.data_ptr(), v.data_ptr(), 0, err.data_ptr(),
+           N.stream_handle())
+    assert abs(float(err.item()) - float((q.sum(0) - 1).abs().sum())) < 1e-5 * float(q.sum() + n)
+    P2 = P.clone()
+    gap = ck.update_quasi_permutation_log(P2, K, u, v, 0.3, 0.5)
+    assert torch.allclose(P2.double(), P.double() + 0.3 * (q - P.double()), rtol=2e-6, atol=1e-7)
+    terms = (q - P.double()) * K.double() * -0.5
+    assert abs(gap - abs(float(terms.sum()))) < 1e-5 * float(terms.abs().sum())
+
+
+@pytest.mark.parametrize("n", [1, 7, 1000, 14336, 14337, 28673])
+def test_transposed_operand_rows(n):
+    """4, 2 and 1 rows of the operand per CTA: the sums of the plain operand's kernel, in the same order."""
+    from cugal_b200.adjacency import Adjacency
+    A = Adjacency.from_edges(_csr_graph([], n, n), n)
+    M = torch.rand((n, n), generator=_gen(n), device="cuda")
+    expect = A.mul(M, negate_lhs=True)
+    rows = torch.randint(0, n, (50,), device="cuda")
+    got = A.mul(M.T.contiguous().T, negate_lhs=True)
+    assert torch.equal(got[rows], expect[rows]) and torch.equal(got[:, rows], expect[:, rows])
+
+
 @pytest.mark.parametrize("n", [1, 5, 149, 1000, 1001, 2049, 4100])
 def test_adjoint_solve_matches_fp64(n):
     """The one-launch conjugate gradients (whole quads and odd rows) against a dense FP64 solve: the
