@@ -4,12 +4,12 @@
 //   fugal_average_neighbor_features   cuda_kernels/feature_extraction.cu:86-125
 //
 // Triangle counts are integer and exact: t(v) = sum over u in N(v) of
-// |N(v) & N(u)|, one warp per vertex with lanes over the neighbours and a
-// binary search of the shorter sorted list in the longer one (a hub's list is
-// searched, never merged element by element by a single thread, so BA hubs do
-// not serialise a warp).  The clustering ratio uses the IEEE-rounded FP32
-// division.  Neighbour averages keep the reference's sequential FP32 sum in CSR
-// order (one thread per vertex), so they are bit-reproducible.
+// |N(v) & N(u)|, one warp per 32 consecutive CSR edges (v, u) whatever rows they
+// belong to, so a hub's edges spread over many warps; the lanes share each
+// intersection (the elements of the shorter list, searched in the longer one).
+// The clustering ratio uses the IEEE-rounded FP32 division.  Neighbour averages
+// keep the reference's sequential FP32 sum in CSR order (one warp per vertex, the
+// values fetched by its lanes), so they are bit-reproducible.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,8 +31,86 @@ __device__ __forceinline__ int lower_bound(const int* __restrict__ col, int lo, 
     return lo;
 }
 
+// Adds to tri[v] the common neighbours of the edges (v, u) of one chunk of 32 edges.
+// Count: 64-bit counts (long long) or, where they cannot overflow, 32-bit ones.  Lists
+// of up to 32 entries are intersected in registers (five shuffles a binary search);
+// longer ones are searched in memory by lanes that share the shorter list.  One warp
+// per vertex, lanes over its neighbours, left a power-law graph's hubs to single
+// warps: 904 us at 65536 vertices of mean degree 16.
+template <typename Count>
+__global__ void __launch_bounds__(256) triangle_kernel(const int* __restrict__ col, const int* __restrict__ rp, int n,
+                                                       Count* tri) {
+    const int lane = threadIdx.x & 31;
+    const int nnz = rp[n];
+    const long long chunk = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const long long chunks = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
+    for (long long ch = chunk; ch * 32 < nnz; ch += chunks) {
+        const int e0 = static_cast<int>(ch * 32), e1 = min(nnz, e0 + 32);
+        // this lane's edge: its neighbour and the neighbour's list
+        const int u = e0 + lane < e1 ? col[e0 + lane] : 0;
+        const int us = e0 + lane < e1 ? rp[u] : 0, ue = e0 + lane < e1 ? rp[u + 1] : 0;
+        int v = lower_bound(rp, 0, n + 1, e0 + 1) - 1;  // the row of edge e0 (rp[v] <= e0 < rp[v + 1])
+        int e = e0;
+        while (e < e1) {
+            const int s = rp[v], t = rp[v + 1];
+            if (t <= e) {
+                ++v;
+                continue;
+            }
+            const int d = t - s;
+            const int a = (d <= 32 && lane < d) ? col[s + lane] : INT_MAX;
+            const int stop = min(t, e1);
+            Count count = 0;
+            for (; e < stop; ++e) {
+                const int bs = __shfl_sync(0xffffffffu, us, e - e0), be = __shfl_sync(0xffffffffu, ue, e - e0);
+                const int db = be - bs;
+                if (d <= 32 && db <= 32) {
+                    const int b = lane < db ? col[bs + lane] : INT_MAX;
+                    const int x = db < d ? b : a, hay = db < d ? a : b;  // shorter in longer, INT_MAX past the end
+                    int pos = 0;                                         // entries of hay below x
+#pragma unroll
+                    for (int step = 16; step > 0; step >>= 1) {
+                        const int y = __shfl_sync(0xffffffffu, hay, pos + step - 1);
+                        if (y < x) pos += step;
+                    }
+                    const int y = __shfl_sync(0xffffffffu, hay, pos);
+                    count += (x != INT_MAX && y == x) ? 1 : 0;
+                } else {
+                    int ss = s, st = t, ls = bs, lt = be;  // shorter, longer
+                    if (db < d) {
+                        ss = bs; st = be; ls = s; lt = t;
+                    }
+                    for (int k = ss + lane; k < st; k += 32) {
+                        const int x = col[k];
+                        const int q = lower_bound(col, ls, lt, x);
+                        count += (q < lt && col[q] == x) ? 1 : 0;
+                    }
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
+            if (lane == 0 && count) atomicAdd(&tri[v], count);
+            ++v;
+        }
+    }
+}
+
+template <typename Count>
+__global__ void clustering_kernel(const int* __restrict__ rp, int n, const Count* tri, float* clustering,
+                                  float* degrees, int* degree_counts) {
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const int d = rp[v + 1] - rp[v];
+        const long long t = static_cast<long long>(tri[v]);
+        degrees[v] = static_cast<float>(d);
+        if (degree_counts) degree_counts[v] = d;
+        const float denom = static_cast<float>(static_cast<long long>(d) * (d - 1));
+        clustering[v] = (t == 0 || d < 2) ? 0.0f : __fdiv_rn(static_cast<float>(t), denom);
+    }
+}
+
+// Counts without a buffer of 64-bit ones and vertices whose count may pass 32 bits.
 __global__ void graph_features_kernel(const int* __restrict__ col, const int* __restrict__ rp, int n,
-                                      float* clustering, float* degrees, int* degree_counts, long long* tri_counts) {
+                                      float* clustering, float* degrees, int* degree_counts) {
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
     for (int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
@@ -59,21 +137,35 @@ __global__ void graph_features_kernel(const int* __restrict__ col, const int* __
         if (lane == 0) {
             degrees[v] = static_cast<float>(d);
             if (degree_counts) degree_counts[v] = d;
-            if (tri_counts) tri_counts[v] = t;
             const float denom = static_cast<float>(static_cast<long long>(d) * (d - 1));
             clustering[v] = (t == 0 || d < 2) ? 0.0f : __fdiv_rn(static_cast<float>(t), denom);
         }
     }
 }
 
+// One warp per vertex: lanes fetch 32 neighbours' values (the next 32 already in
+// flight), then every lane adds them in CSR order.
 __global__ void average_neighbor_kernel(const int* __restrict__ col, const int* __restrict__ rp, int n,
                                         const float* __restrict__ f, float* avg) {
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    for (int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
         const int s = rp[v], e = rp[v + 1];
         float sum = 0.0f;
-        for (int k = s; k < e; ++k) sum = __fadd_rn(sum, f[col[k]]);
+        float x = s + lane < e ? f[col[s + lane]] : 0.0f;
+        for (int k = s; k < e; k += 32) {
+            const float next = k + 32 + lane < e ? f[col[k + 32 + lane]] : 0.0f;
+            const int cnt = min(32, e - k);
+            if (cnt == 32) {
+#pragma unroll
+                for (int q = 0; q < 32; ++q) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, x, q));
+            } else {
+                for (int q = 0; q < cnt; ++q) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, x, q));
+            }
+            x = next;
+        }
         const int d = e - s;
-        avg[v] = d == 0 ? 0.0f : __fdiv_rn(sum, static_cast<float>(d));
+        if (lane == 0) avg[v] = d == 0 ? 0.0f : __fdiv_rn(sum, static_cast<float>(d));
     }
 }
 
@@ -90,45 +182,59 @@ __global__ void count_rows_kernel(const int* edges, long long m, int n, int* cou
     }
 }
 
-// Exclusive scan of counts[0..n) into rp[0..n] by one block (carry across chunks).
-__global__ void __launch_bounds__(1024) scan_rows_kernel(const int* counts, int n, int* rp, int* cursor) {
-    __shared__ int warp_tot[32];
-    __shared__ int carry_s;
-    if (threadIdx.x == 0) carry_s = 0;
-    __syncthreads();
+// Exclusive scan of counts[0..n) into rp[0..n], 1024 counts per block; a block first
+// adds up all counts before its own (up to kScanBlocks blocks: at most 1 MB each, read
+// by all SMs at once).  51 us at n = 65536 when one block walked all counts.
+constexpr int kScanBlocks = 256;
+
+// Inclusive scan of one value per thread over a 1024-thread block; returns the block's total in `total`.
+__device__ __forceinline__ int block_scan_1024(int x, int* warp_tot, int& total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int base = 0; base < n; base += blockDim.x) {
-        const int i = base + threadIdx.x;
-        const int x = i < n ? counts[i] : 0;
-        int incl = x;
+    int incl = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) warp_tot[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        int w = warp_tot[lane];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
+            const int y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
         }
-        if (lane == 31) warp_tot[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            int w = lane < (blockDim.x >> 5) ? warp_tot[lane] : 0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= o) w += y;
-            }
-            warp_tot[lane] = w;  // inclusive over warps
-        }
-        __syncthreads();
-        const int carry = carry_s;
-        const int excl = carry + (warp > 0 ? warp_tot[warp - 1] : 0) + incl - x;
-        if (i < n) {
+        warp_tot[lane] = w;  // inclusive over warps
+    }
+    __syncthreads();
+    total = warp_tot[31];
+    incl += warp > 0 ? warp_tot[warp - 1] : 0;
+    __syncthreads();  // warp_tot is read
+    return incl;
+}
+
+__global__ void __launch_bounds__(1024) scan_rows_kernel(const int* counts, int n, int* rp, int* cursor) {
+    __shared__ int warp_tot[32];
+    const int per = (n + gridDim.x - 1) / gridDim.x;  // counts per block: 1024 unless there are too many
+    const int begin = min(n, static_cast<int>(blockIdx.x) * per), end = min(n, begin + per);
+    int sum = 0;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < begin; i += 1024) sum += counts[i];
+    int carry = 0;
+    block_scan_1024(sum, warp_tot, carry);
+    for (int base = begin; base < end; base += 1024) {
+        const int i = base + threadIdx.x;
+        const int x = i < end ? counts[i] : 0;
+        int total = 0;
+        const int excl = carry + block_scan_1024(x, warp_tot, total) - x;
+        if (i < end) {
             rp[i] = excl;
             cursor[i] = excl;
         }
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry_s = excl + x;
-        __syncthreads();
+        carry += total;
     }
-    if (threadIdx.x == 0) rp[n] = carry_s;
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) rp[n] = carry;
 }
 
 __global__ void scatter_cols_kernel(const int* edges, long long m, int n, int* cursor, int* col) {
@@ -140,15 +246,43 @@ __global__ void scatter_cols_kernel(const int* edges, long long m, int n, int* c
     }
 }
 
-// Sort each row's columns ascending: bitonic sort in shared memory, one block
-// per row, rows up to kMaxSortRow entries (longer rows raise a flag).
+// Sort each row's columns ascending.  Rows of up to 32 entries: one warp each, every
+// entry stored at its rank (entries below it, ties by position); a 512-thread block
+// per such row was 303 us at 65536 rows of mean length 16.
+__global__ void __launch_bounds__(256) sort_short_rows_kernel(const int* rp, int n, int* col) {
+    const int lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += warps) {
+        const int s = rp[r], d = rp[r + 1] - s;
+        if (d <= 1 || d > 32) continue;
+        const int x = lane < d ? col[s + lane] : INT_MAX;
+        int rank = 0;
+        for (int k = 0; k < d; ++k) {
+            const int y = __shfl_sync(0xffffffffu, x, k);
+            rank += (y < x || (y == x && k < lane)) ? 1 : 0;
+        }
+        if (lane < d) col[s + rank] = x;
+    }
+}
+
+// Longer rows: bitonic sort in shared memory, one block per row, rows up to
+// kMaxSortRow entries (longer rows raise a flag).
 constexpr int kMaxSortRow = 8192;
 
 __global__ void __launch_bounds__(512) sort_rows_kernel(const int* rp, int n, int* col, int* bad) {
     __shared__ int buf[kMaxSortRow];
-    for (int r = blockIdx.x; r < n; r += gridDim.x) {
+    __shared__ int found[512], nfound;
+    // 512 rows at a time, strided over the blocks (hubs are often neighbours): the long ones
+    for (long long base = blockIdx.x; base < n; base += 512ll * gridDim.x) {
+      if (threadIdx.x == 0) nfound = 0;
+      __syncthreads();
+      const long long mine = base + static_cast<long long>(threadIdx.x) * gridDim.x;
+      if (mine < n && rp[mine + 1] - rp[mine] > 32) found[atomicAdd(&nfound, 1)] = static_cast<int>(mine);
+      __syncthreads();
+      const int rows = nfound;
+      for (int q = 0; q < rows; ++q) {
+        const int r = found[q];
         const int s = rp[r], e = rp[r + 1], d = e - s;
-        if (d <= 1) continue;
         if (d > kMaxSortRow) {
             if (threadIdx.x == 0) atomicExch(bad, 2);
             continue;
@@ -175,6 +309,8 @@ __global__ void __launch_bounds__(512) sort_rows_kernel(const int* rp, int n, in
         }
         for (int i = threadIdx.x; i < d; i += blockDim.x) col[s + i] = buf[i];
         __syncthreads();
+      }
+      __syncthreads();  // found is read
     }
 }
 
@@ -190,11 +326,42 @@ extern "C" fugal_status fugal_graph_features(const int32_t* col_indices, const i
         return fail(FUGAL_BAD_ARGUMENT, "fugal_graph_features: null argument");
     if (n <= 0 || n > INT_MAX - 1) return fail(FUGAL_BAD_SHAPE, "fugal_graph_features: bad n");
     const int threads = 256;
+    const int ni = static_cast<int>(n);
     const int blocks = static_cast<int>(std::min<int64_t>((n * 32 + threads - 1) / threads, 32 * sm_count()));
+    const int vec_blocks = static_cast<int>(std::min<int64_t>((n + threads - 1) / threads, 8 * sm_count()));
+    const int chunk_blocks = static_cast<int>(std::min<int64_t>((n + 15) / 16 + 1, 16 * sm_count()));
+    // A count is at most d (d - 1) < n^2: with up to 65536 vertices it fits the 32 bits of
+    // a clustering entry, which holds it until the ratio is formed.
+    if (triangle_counts != nullptr) {
+        long long* tri = reinterpret_cast<long long*>(triangle_counts);
+        FUGAL_TRY(cuda_check(cudaMemsetAsync(tri, 0, static_cast<size_t>(n) * 8, stream), "fugal_graph_features"));
+        {
+            LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
+            triangle_kernel<unsigned long long><<<chunk_blocks, threads, 0, stream>>>(
+                col_indices, row_pointers, ni, reinterpret_cast<unsigned long long*>(tri));
+            FUGAL_TRY(launch_check("fugal_graph_features: triangles"));
+        }
+        LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
+        clustering_kernel<long long><<<vec_blocks, threads, 0, stream>>>(row_pointers, ni, tri, clustering, degrees,
+                                                                         degree_counts);
+        return launch_check("fugal_graph_features");
+    }
+    if (n <= 65536) {
+        unsigned* tri = reinterpret_cast<unsigned*>(clustering);
+        FUGAL_TRY(cuda_check(cudaMemsetAsync(tri, 0, static_cast<size_t>(n) * 4, stream), "fugal_graph_features"));
+        {
+            LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
+            triangle_kernel<unsigned><<<chunk_blocks, threads, 0, stream>>>(col_indices, row_pointers, ni, tri);
+            FUGAL_TRY(launch_check("fugal_graph_features: triangles"));
+        }
+        LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
+        clustering_kernel<unsigned><<<vec_blocks, threads, 0, stream>>>(row_pointers, ni, tri, clustering, degrees,
+                                                                        degree_counts);
+        return launch_check("fugal_graph_features");
+    }
     LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-    graph_features_kernel<<<blocks, threads, 0, stream>>>(col_indices, row_pointers, static_cast<int>(n), clustering,
-                                                          degrees, degree_counts,
-                                                          reinterpret_cast<long long*>(triangle_counts));
+    graph_features_kernel<<<blocks, threads, 0, stream>>>(col_indices, row_pointers, ni, clustering, degrees,
+                                                          degree_counts);
     return launch_check("fugal_graph_features");
 }
 
@@ -205,9 +372,9 @@ extern "C" fugal_status fugal_average_neighbor_features(const int32_t* col_indic
     if (row_pointers == nullptr || features == nullptr || averages == nullptr)
         return fail(FUGAL_BAD_ARGUMENT, "fugal_average_neighbor_features: null argument");
     if (n <= 0 || n > INT_MAX - 1) return fail(FUGAL_BAD_SHAPE, "fugal_average_neighbor_features: bad n");
-    const int blocks = static_cast<int>(std::min<int64_t>((n + 127) / 128, 16 * sm_count()));
+    const int blocks = static_cast<int>(std::min<int64_t>((n + 7) / 8, 16 * sm_count()));
     LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-    average_neighbor_kernel<<<blocks, 128, 0, stream>>>(col_indices, row_pointers, static_cast<int>(n), features,
+    average_neighbor_kernel<<<blocks, 256, 0, stream>>>(col_indices, row_pointers, static_cast<int>(n), features,
                                                         averages);
     return launch_check("fugal_average_neighbor_features");
 }
@@ -245,7 +412,8 @@ extern "C" fugal_status fugal_create_adjacency(const int32_t* edges, int64_t edg
     }
     {
         LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-        scan_rows_kernel<<<1, 1024, 0, stream>>>(counts, n, row_pointers, cursor);
+        const int blocks1024 = std::min((n + 1023) / 1024, kScanBlocks);
+        scan_rows_kernel<<<blocks1024, 1024, 0, stream>>>(counts, n, row_pointers, cursor);
         FUGAL_TRY(launch_check("fugal_create_adjacency: scan"));
     }
     if (edge_count > 0) {
@@ -253,6 +421,12 @@ extern "C" fugal_status fugal_create_adjacency(const int32_t* edges, int64_t edg
             LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
             scatter_cols_kernel<<<blocks, 256, 0, stream>>>(edges, edge_count, n, cursor, col_indices);
             FUGAL_TRY(launch_check("fugal_create_adjacency: scatter"));
+        }
+        {
+            LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
+            const int wblocks = static_cast<int>(std::min<int64_t>((node_count + 7) / 8, 16 * sm_count()));
+            sort_short_rows_kernel<<<wblocks, 256, 0, stream>>>(row_pointers, n, col_indices);
+            FUGAL_TRY(launch_check("fugal_create_adjacency: short rows"));
         }
         LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
         const int sblocks = static_cast<int>(std::min<int64_t>(n, 8 * sm_count()));

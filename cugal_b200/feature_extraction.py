@@ -28,7 +28,8 @@ def graph_features(adjacency: Adjacency, with_counts: bool = False):
     clustering = torch.empty(n, dtype=torch.float32, device=dev)
     degrees = torch.empty(n, dtype=torch.float32, device=dev)
     dc = torch.empty(n, dtype=torch.int32, device=dev) if with_counts else None
-    tc = torch.empty(n, dtype=torch.int64, device=dev) if with_counts else None
+    # above 65536 vertices the kernel needs room for 64-bit counts
+    tc = torch.empty(n, dtype=torch.int64, device=dev) if with_counts or n > 65536 else None
     N.call("fugal_graph_features", adjacency.col_indices.data_ptr(), adjacency.row_pointers.data_ptr(), n,
            clustering.data_ptr(), degrees.data_ptr(), N.ptr(dc), N.ptr(tc), N.stream_handle(dev))
     return (degrees, clustering, dc, tc) if with_counts else (degrees, clustering)

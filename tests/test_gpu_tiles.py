@@ -26,6 +26,28 @@ def _csr_graph(lengths, n, seed):
     return torch.from_numpy(rng.permutation(e)).cuda()
 
 
+@pytest.mark.parametrize("n,lengths", [(5, [1]), (33, [31, 32]), (100, [30, 31, 32, 33, 34, 63, 64, 65]),
+                                       (3000, [24, 32, 33, 1500, 2999]), (16385, [40, 9000])])
+def test_graph_rows_at_register_and_memory_lengths(n, lengths):
+    """CSR order, triangle counts (rows of up to 32 entries in registers, longer ones in memory, edges of
+    one row over several warps), with and without 64-bit counts, and neighbour averages: bit for bit."""
+    from cugal_b200.adjacency import Adjacency
+    from cugal_b200.feature_extraction import average_neighbor_features, graph_features
+    lengths = [d for d in lengths if d <= 8000]  # the row sort's limit
+    A = Adjacency.from_edges(_csr_graph(lengths, n, n), n)
+    rp, col = A.row_pointers.cpu().numpy(), A.col_indices.cpu().numpy()
+    for r in range(n):
+        assert np.all(np.diff(col[rp[r]:rp[r + 1]]) > 0)
+    odeg, otri = O.triangle_counts(rp, col)
+    deg, clust, dc, tc = graph_features(A, with_counts=True)
+    assert np.array_equal(dc.cpu().numpy(), odeg) and np.array_equal(tc.cpu().numpy(), otri)
+    deg2, clust2 = graph_features(A)
+    assert torch.equal(deg, deg2) and torch.equal(clust, clust2)
+    assert np.array_equal(clust.cpu().numpy(), O.clustering_from_counts(odeg, otri))
+    avg = average_neighbor_features(A, clust).cpu().numpy()
+    assert np.array_equal(avg, O.average_neighbor(rp, col, clust.cpu().numpy()))
+
+
 @pytest.mark.parametrize("ld_pad,offset", [(0, 0), (3, 0), (0, 1)])
 @pytest.mark.parametrize("cols", [1, 3, 1023, 1024, 1028, 2052, 4100, 8192, 8196, 20001])
 def test_log_step_widths(cols, ld_pad, offset):
