@@ -48,6 +48,34 @@ def test_graph_rows_at_register_and_memory_lengths(n, lengths):
     assert np.array_equal(avg, O.average_neighbor(rp, col, clust.cpu().numpy()))
 
 
+@pytest.mark.parametrize("maximize", [True, False])
+@pytest.mark.parametrize("n", [1, 2, 31, 1023, 1024, 1025, 2049, 4097])
+def test_exact_lap_owned_columns(n, maximize):
+    """Every number of owned columns per thread, with many ties (integers 0 .. 3, zeros of both signs)."""
+    from cugal_b200.exact_lap import exact_assign
+    rng = np.random.default_rng(n)
+    P = np.zeros((n, n), dtype=np.float32)
+    P[rng.random((n, n)) < 0.5] = -0.0
+    rows = np.arange(n)
+    for k in range(3):
+        P[rows, rng.permutation(n)] += rng.integers(0, 4, size=n).astype(np.float32)
+    cols, _, status = exact_assign(torch.tensor(P, device="cuda"), maximize=maximize)
+    assert int(status.item()) == 0
+    np.testing.assert_array_equal(cols.cpu().numpy(), linear_sum_assignment(P, maximize=maximize)[1])
+
+
+def test_exact_lap_above_owned_columns():
+    """8192 is the widest owned matrix, 8193 takes the kernel with its arrays in global memory."""
+    from cugal_b200.exact_lap import exact_assign
+    for n in (8192, 8193):
+        g = _gen(n)
+        perm = torch.randperm(n, generator=g, device="cuda")
+        P = torch.rand((n, n), generator=g, device="cuda") * 1e-4
+        P[torch.arange(n, device="cuda"), perm] += 1.0
+        cols, steps, status = exact_assign(P)
+        assert int(status.item()) == 0 and int(steps.item()) == n and torch.equal(cols, perm)
+
+
 @pytest.mark.parametrize("ld_pad,offset", [(0, 0), (3, 0), (0, 1)])
 @pytest.mark.parametrize("cols", [1, 3, 1023, 1024, 1028, 2052, 4100, 8192, 8196, 20001])
 def test_log_step_widths(cols, ld_pad, offset):
