@@ -35,226 +35,34 @@
 #include <type_traits>
 
 #include "fugal_common.cuh"
-#include "sinkhorn_rows.h"
+#include "sinkhorn_rows.cuh"
 #include "sinkhorn_state.cuh"
 
 namespace fugal {
 
-constexpr int kRowsThreads = 512;
-// The streams' column sums meet in shared memory, unless two streams of more than 32
-// columns per thread need it for their stages (each then writes a partial row).
-constexpr bool rows_dump(int streams, int ept) { return streams > 1 && ept <= 32; }
-constexpr int kRowsWarps = kRowsThreads / 32;
-constexpr int kRowsMaxRows = 256;      // rows per CTA the row-dual staging holds
-constexpr int kRowsStatic = 24 * 1024; // shared memory kept for the static arrays
-
-// Barrier over the GT threads of stream g; true if every thread voted true.
-template <int GT>
-FUGAL_DEVICE bool stream_and(bool ok, int g) {
-    if constexpr (GT == kRowsThreads) {
-        return __syncthreads_and(ok) != 0;
-    } else {
-        uint32_t out;
-        asm volatile(
-            "{\n .reg .pred p, q;\n"
-            " setp.ne.u32 q, %1, 0;\n"
-            " barrier.cta.red.and.aligned.pred p, %2, %3, q;\n"
-            " selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(out)
-            : "r"(static_cast<uint32_t>(ok)), "r"(g + 1), "n"(GT)
-            : "memory");
-        return out != 0;
-    }
-}
-
-// Sum of GW per-warp values in a fixed pairwise order.
-template <int GW>
-FUGAL_DEVICE float sum_warps(const float* r) {
-    if constexpr (GW == 2) {
-        const float2 a = *reinterpret_cast<const float2*>(r);
-        return a.x + a.y;
-    } else {
-        float s[GW / 4];
-#pragma unroll
-        for (int i = 0; i < GW / 4; ++i) {
-            const float4 a = reinterpret_cast<const float4*>(r)[i];
-            s[i] = (a.x + a.y) + (a.z + a.w);
-        }
-        if constexpr (GW == 4) return s[0];
-        else if constexpr (GW == 8) return s[0] + s[1];
-        else return (s[0] + s[1]) + (s[2] + s[3]);
-    }
-}
-
-// 16 elements of a staged row (chunk c of this thread) as 8 float pairs.
-template <typename T, int GT>
-FUGAL_DEVICE void load16(const T* stage, int c, int gt, float2* v) {
-    constexpr int V = Vec<T>::N;
-#pragma unroll
-    for (int i = 0; i < 16 / V; ++i)
-        Pairs<T>::unpack(*reinterpret_cast<const uint4*>(stage + ((c * (16 / V) + i) * GT + gt) * V), v + i * V / 2);
-}
-
-// Column sums and column duals (b log2 e) of a thread's EPT columns: in registers
-// up to 32 columns, else in tensor memory, 16 columns per access.
-template <int EPT, bool REG = (EPT <= 32)>
-struct ColumnState;
-
-template <int EPT>
-struct ColumnState<EPT, true> {
-    static constexpr uint32_t kTmemColumns = 0;
-    float2 sum[EPT / 2], dual[EPT / 2];
-    FUGAL_DEVICE void start(uint32_t, int) {}
-    // 16 duals b of chunk c; their sums start at 0
-    FUGAL_DEVICE void set(int c, const float* b) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            dual[8 * c + q] = make_float2(b[2 * q], b[2 * q + 1]);
-            sum[8 * c + q] = make_float2(0.f, 0.f);
-        }
-    }
-    FUGAL_DEVICE void ready() {}
-    FUGAL_DEVICE void duals(int c, float2* b) const {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) b[q] = dual[8 * c + q];
-    }
-    // adds the pending row's chunk y (weight w) to the sums of chunk c
-    FUGAL_DEVICE void add(int c, const float2* y, float w) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) sum[8 * c + q] = __ffma2_rn(y[q], make_float2(w, w), sum[8 * c + q]);
-    }
-    FUGAL_DEVICE void total(int c, const float2* y, float w, float* out) {
-        add(c, y, w);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            out[2 * q] = sum[8 * c + q].x;
-            out[2 * q + 1] = sum[8 * c + q].y;
-        }
-    }
-};
-
-template <int EPT>
-struct ColumnState<EPT, false> {
-    static constexpr uint32_t kTmemColumns = 512;  // 4 warps per lane quarter x (sums + duals) x EPT <= 64
-    uint32_t tsum, tdual;
-    FUGAL_DEVICE void start(uint32_t base, int warp) {
-        tsum = base + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + static_cast<uint32_t>((warp >> 2) * EPT);
-        tdual = tsum + static_cast<uint32_t>((kRowsThreads / 128) * EPT);
-    }
-    FUGAL_DEVICE void set(int c, const float* b) {
-        float z[16];
-#pragma unroll
-        for (int k = 0; k < 16; ++k) z[k] = 0.f;
-        tmem_st16(tdual + 16 * c, b);
-        tmem_st16(tsum + 16 * c, z);
-    }
-    FUGAL_DEVICE void ready() { tmem_wait_st(); }
-    FUGAL_DEVICE void duals(int c, float2* b) const {
-        float v[16];
-        tmem_ld16(tdual + 16 * c, v);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) b[q] = make_float2(v[2 * q], v[2 * q + 1]);
-    }
-    FUGAL_DEVICE void total(int c, const float2* y, float w, float* out) {
-        tmem_ld16(tsum + 16 * c, out);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const float2 a2 = __ffma2_rn(y[q], make_float2(w, w), make_float2(out[2 * q], out[2 * q + 1]));
-            out[2 * q] = a2.x;
-            out[2 * q + 1] = a2.y;
-        }
-    }
-    FUGAL_DEVICE void add(int c, const float2* y, float w) {
-        float acc[16];
-        total(c, y, w, acc);
-        tmem_st16(tsum + 16 * c, acc);
-    }
-};
-
-// This CTA's share of the columns: FP64 sums over the partial rows, log(colsum),
-// the CTA's error and largest correction.  Lanes of a warp: cgp column quads (a
-// power of two) x the rest over partial rows.  (Not inlined: its registers would
-// be live across the row loop.)
+// This CTA's share of the columns: log(colsum), the next duals, the CTA's error and
+// largest correction.  (Not inlined: its registers would be live across the row loop.)
 __device__ __noinline__ void reduce_columns(const RowsArgs& p, int t, int parts) {
     __shared__ double colred[kRowsWarps][128];
     __shared__ double errred[kRowsWarps];
     __shared__ float corred[kRowsWarps];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n = p.n;
-    const int quads = (n + 3) / 4;
-    const int per = (quads + gridDim.x - 1) / gridDim.x;
-    int cgp = 1;
-    while (cgp < per) cgp <<= 1;
-    const int cg = tid & (cgp - 1);
-    const int q0 = blockIdx.x * per;
-    const bool mine = cg < per && q0 + cg < quads;
-    const int j0 = (q0 + cg) * 4;
-    const int step = kRowsThreads / cgp;
-    double cs[4] = {0.0, 0.0, 0.0, 0.0};
-    // all of a thread's loads in flight (they come from L2): at most 4 up to 8192
-    // columns on 148 SMs, 10 per round above
-    const float* src = p.partials + j0;
-    auto add_rows = [&](auto unroll) {
-        constexpr int U = decltype(unroll)::value;
-        for (int k0 = tid / cgp; k0 < parts; k0 += U * step) {
-            float4 v[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int k = k0 + u * step;
-                v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (mine && k < parts)
-                    v[u] = __ldcg(reinterpret_cast<const float4*>(src + static_cast<size_t>(k) * p.n_pad));
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (k0 + u * step < parts) {
-                    cs[0] += v[u].x;
-                    cs[1] += v[u].y;
-                    cs[2] += v[u].z;
-                    cs[3] += v[u].w;
-                }
-            }
-        }
-    };
-    if (parts <= 4 * step) add_rows(std::integral_constant<int, 4>{});
-    else add_rows(std::integral_constant<int, 10>{});
-    for (int o = cgp; o < 32; o <<= 1) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) cs[q] += __shfl_xor_sync(0xffffffffu, cs[q], o);
-    }
-    // cgp <= 32: lane l < cgp of every warp holds quad l; cgp = 64: warps alternate quads 0..31, 32..63
-    if (lane < cgp) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) colred[warp][lane * 4 + q] = cs[q];
-    }
+    const int per = columns_per_cta(p.n);
+    const int j = blockIdx.x * per + tid;
+    const bool mine = tid < per && j < p.n;
     float b_now = 0.f;
-    if (tid < per * 4 && q0 * 4 + tid < n) b_now = __ldcg(p.b_buf + (t & 1) * p.n_pad + q0 * 4 + tid);
-    __syncthreads();
+    if (mine) b_now = __ldcg(p.b_buf + (t & 1) * p.n_pad + j);
+    const double tot = own_column_sum(p.partials, p.n_pad, parts, p.n, colred);
     double err = 0.0;
     float corr = 0.f;
-    if (tid < per * 4) {
-        const int j = q0 * 4 + tid;
-        if (j < n) {
-            // pairwise over the warps (the upper half is empty at cgp = 64)
-            double h[kRowsWarps];
-#pragma unroll
-            for (int w = 0; w < kRowsWarps; ++w)
-                h[w] = cgp <= 32 ? colred[w][tid]
-                                 : (w < kRowsWarps / 2 ? colred[2 * w + (tid >> 7)][tid & 127] : 0.0);
-#pragma unroll
-            for (int o = kRowsWarps / 2; o > 0; o >>= 1) {
-#pragma unroll
-                for (int w = 0; w < o; ++w) h[w] += h[w + o];
-            }
-            const double tot = h[0];
-            err = fabs(tot - 1.0);
-            const float lg = static_cast<float>(log(fmax(tot, 1e-37)));
-            p.logcs[j] = lg;
-            p.b_next[j] = b_now - lg;  // the next sweep's dual without momentum
-            corr = fabsf(lg);
-        }
+    if (mine) {
+        err = fabs(tot - 1.0);
+        const float lg = static_cast<float>(log(fmax(tot, 1e-37)));
+        p.logcs[j] = lg;
+        p.b_next[j] = b_now - lg;  // the next sweep's dual without momentum
+        corr = fabsf(lg);
     }
-    const int used = (per * 4 + 31) / 32;  // warps that hold columns
+    const int used = (per + 31) / 32;  // warps that hold columns
     if (warp < used) {
         err = warp_sum(err);
         corr = warp_max(corr);
@@ -285,30 +93,11 @@ __device__ __noinline__ void reduce_columns(const RowsArgs& p, int t, int parts)
 
 // The decision at the end of a sweep, the same in every CTA (warp 0).
 __device__ __noinline__ void take_decision(const RowsArgs& p, SolveState* ss) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp == 0) {
-        double e = 0.0;
-        float c = 0.f;
-        constexpr int U = 8;  // 256 CTAs per round, all loads in flight
-        const int ctas = static_cast<int>(gridDim.x);
-        for (int k0 = lane; k0 < ctas; k0 += 32 * U) {
-            double ev[U];
-            float cv[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int k = k0 + 32 * u;
-                ev[u] = k < ctas ? __ldcg(p.errs + k) : 0.0;
-                cv[u] = k < ctas ? __ldcg(p.corrs + k) : 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                e += ev[u];
-                c = fmaxf(c, cv[u]);
-            }
-        }
-        e = warp_sum(e);
-        c = warp_max(c);
-        if (lane == 0) {
+    if (threadIdx.x < 32) {
+        double e;
+        float c;
+        grid_error(p.errs, p.corrs, e, c);
+        if (threadIdx.x == 0) {
             decide(ss, e);
             // the next sweep may use the previous row normaliser as its reference
             // only if no column moves by more than kFastPathLimit nats

@@ -7,13 +7,17 @@
 // and at t % eval_freq == 0 (t = 0 included) the column-marginal error
 //     sum_j | sum_i u_i K_ij v_j - 1 |,
 // stopping below the threshold and updating the Lehmann factor w otherwise.
-// Here round t launches: column partial sums of u K (the error of iteration
-// t-1 uses exactly these sums with the current v, so it costs no extra pass),
-// their FP64 merge with the error and the stop / momentum decision on the
-// device, the v update, and the row products K v with the u update.  Rounds
-// after the decision to stop return at once; the host polls the stop flag with
-// a lag of two rounds.  u and v are read and written in place (warm start
-// across solves, cugal/sinkhorn.py:51-65).
+// The column sums u K of an iteration give both its error (with the current v) and
+// the next v update.  u and v are read and written in place (warm start across
+// solves, cugal/sinkhorn.py:51-65).  Two forms:
+//   std_rows_kernel (up to 16384 columns): the whole solve in one persistent launch.
+//   A CTA owns whole rows (row streams, ring of stages and column state of
+//   sinkhorn_rows.cuh); a row is read once per iteration: its product with v gives
+//   u_i, and u_i times the row, still in registers, goes into the column sums.
+//   wider: round t launches column partial sums of u K, their FP64 merge with the
+//   error and the decision on the device, the v update, and the row products K v with
+//   the u update.  Rounds after the decision to stop return at once; the host polls
+//   the stop flag with a lag of two rounds.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -21,11 +25,14 @@
 
 #include "fugal_common.cuh"
 #include "fugal_host.h"
+#include "sinkhorn_rows.cuh"
 
 namespace fugal {
 
 constexpr float kStdEps = 1e-16f;  // M_EPS, cugal/sinkhorn.py:12
 constexpr int kStdThreads = 256;
+constexpr int kStdRowsLimit = 16384;  // columns of the persistent form
+constexpr int kStdMaxParts = 4;       // partial rows per CTA it writes at most
 
 struct StdState {
     int done;
@@ -45,8 +52,11 @@ struct StdState {
 
 struct StdWs {
     StdState* st;
-    float* colsum;    // [n]
-    float* partials;  // [chunks][n]
+    float* colsum;    // [2][n_pad]: column sums; v of the pass before (momentum)
+    float* v_next;    // [n_pad]
+    float* partials;  // [chunks][n], or [CTAs or streams][n_pad]
+    double* errs;     // [SMs]
+    unsigned* sync;   // [2]: grid barrier, status
     size_t bytes;
 };
 
@@ -65,8 +75,13 @@ StdWs std_layout(int64_t n, char* base) {
         return p;
     };
     w.st = reinterpret_cast<StdState*>(take(sizeof(StdState)));
-    w.colsum = reinterpret_cast<float*>(take(n * 4));
-    w.partials = reinterpret_cast<float*>(take(static_cast<size_t>(std_chunks(n)) * n * 4));
+    const size_t n_pad = (static_cast<size_t>(n) + 63) / 64 * 64;
+    w.colsum = reinterpret_cast<float*>(take(2 * n_pad * 4));
+    w.v_next = reinterpret_cast<float*>(take(n_pad * 4));
+    const size_t rows = std::max<size_t>(std_chunks(n), n <= kStdRowsLimit ? kStdMaxParts * sm_count() : 0);
+    w.partials = reinterpret_cast<float*>(take(rows * n_pad * 4));
+    w.errs = reinterpret_cast<double*>(take(static_cast<size_t>(sm_count()) * 8));
+    w.sync = reinterpret_cast<unsigned*>(take(2 * sizeof(unsigned)));
     w.bytes = off;
     return w;
 }
@@ -175,11 +190,11 @@ __global__ void __launch_bounds__(kStdThreads) std_rowdot_kernel(const float* __
     }
 }
 
-__global__ void std_record_kernel(const StdState* st, fugal_solve_record* rec) {
+__global__ void std_record_kernel(const StdState* st, const unsigned* status, fugal_solve_record* rec) {
     if (threadIdx.x == 0) {
         rec->iteration_count = st->final_it + 1;
         rec->n_errors = min(st->n_err, FUGAL_MAX_RECORDED_ERRORS);
-        rec->status = 0;
+        rec->status = static_cast<int>(*status);
         rec->polish_count = 0;
         rec->last_error = st->last_err;
         rec->polish_error = 0.0;
@@ -213,6 +228,407 @@ __global__ void __launch_bounds__(kStdThreads) std_update_kernel(float* P, long 
     }
     g = block_sum(g, red);
     if (threadIdx.x == 0) atomicAdd(gap, g);
+}
+
+// ------------------------------------------------------------- persistent form
+
+// Per iteration: one read of K (144 MB at n = 6000, 22 us at the copy peak) where the
+// four launches of the wider form read it twice (31 + 49 us) and paid their gaps: 92 us
+// against 45 us an iteration at n = 6000.
+struct StdRowsArgs {
+    const float* K;
+    long long ldk;
+    int n;
+    int n_copy;          // columns copied per row: a multiple of 4 within ldk
+    int rows_per_cta;
+    int stages;
+    int resident;
+    unsigned suspend_ns;
+    float* u;
+    float* v;
+    float* v_next;       // 1 / (column sum + eps): the next v without momentum
+    float* colsum;
+    float* partials;
+    double* errs;
+    long long n_pad;
+    StdState* st;
+    unsigned* arrivals;
+    int* status;
+};
+
+// x^(1-w) y^w, the momentum update (w != 1)
+FUGAL_DEVICE float std_blend(float x, float y, double w) {
+    return powf(x, static_cast<float>(1.0 - w)) * powf(y, static_cast<float>(w));
+}
+
+__device__ __noinline__ void std_reduce_columns(const StdRowsArgs& p, int parts, bool eval) {
+    __shared__ double colred[kRowsWarps][128];
+    __shared__ double red[32];
+    const int per = columns_per_cta(p.n);
+    const int j = blockIdx.x * per + threadIdx.x;
+    const bool mine = static_cast<int>(threadIdx.x) < per && j < p.n;
+    const float vj = mine && eval ? __ldcg(p.v + j) : 0.f;
+    const double tot = own_column_sum(p.partials, p.n_pad, parts, p.n, colred);
+    double err = 0.0;
+    if (mine) {
+        const float cf = static_cast<float>(tot);
+        p.colsum[j] = cf;
+        p.v_next[j] = 1.0f / (cf + kStdEps);
+        if (eval) err = fabs(static_cast<double>(vj) * static_cast<double>(cf) - 1.0);
+    }
+    if (eval) {
+        err = block_sum(err, red);
+        if (threadIdx.x == 0) p.errs[blockIdx.x] = err;
+    }
+}
+
+// The decision after the column sums of round t (thread 0 of every CTA, the same in all).
+__device__ __noinline__ void std_decide(const StdRowsArgs& p, StdState* st, int t, bool eval) {
+    if (threadIdx.x >= 32) return;
+    double e = 0.0;
+    float c;
+    if (eval) grid_error(p.errs, nullptr, e, c);
+    if (threadIdx.x != 0) return;
+    bool stop = false;
+    if (eval) {
+        st->last_err = e;
+        if (st->n_err < FUGAL_MAX_RECORDED_ERRORS) st->errors[st->n_err] = e;
+        st->n_err += 1;
+        if (e < st->threshold)
+            stop = true;
+        else
+            st->omega = lehmann_omega(st->errors, st->n_err, st->eval_freq, st->momentum_start);
+    }
+    if (stop || t >= st->max_it) {
+        st->done = 1;
+        st->final_it = t - 1;
+    }
+}
+
+template <int EPT, int GR>
+__global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_constant__ StdRowsArgs p) {
+    constexpr int GT = kRowsThreads / GR;
+    constexpr int GW = GT / 32;
+    constexpr int COVER = GT * EPT;
+    constexpr int NCH = EPT / 16;
+    constexpr int H = EPT / 2;
+    constexpr bool DUMP = rows_dump(GR, EPT);
+    constexpr uint32_t TCOLS = ColumnState<EPT>::kTmemColumns;
+    extern __shared__ __align__(128) unsigned char ring[];
+    float* dump = reinterpret_cast<float*>(ring + static_cast<size_t>(p.stages) * COVER * sizeof(float));  // DUMP
+    __shared__ uint64_t full[kRowsMaxStages];
+    __shared__ int newest[kRowsMaxStages];  // phase of the newest copy into a stage (-1: none)
+    __shared__ __align__(16) float red_s[GR][2][GW];
+    __shared__ float u_s[kRowsMaxRows];
+    __shared__ StdState ss;
+    __shared__ uint32_t tmem_slot;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = tid / GT, gt = tid % GT, gw = warp % GW;
+    const int n = p.n;
+    const int row_begin = blockIdx.x * p.rows_per_cta;
+    const int nrows = max(0, min(n, row_begin + p.rows_per_cta) - row_begin);
+    const int NST = p.stages;
+    for (int k = tid; k < static_cast<int>(sizeof(StdState) / 4); k += kRowsThreads)
+        reinterpret_cast<int*>(&ss)[k] = reinterpret_cast<const int*>(p.st)[k];
+    for (int i = tid; i < nrows; i += kRowsThreads) u_s[i] = p.u[row_begin + i];
+    for (int s = 0; s < NST; ++s) {  // columns past n_copy are never copied
+        float* row = reinterpret_cast<float*>(ring) + static_cast<size_t>(s) * COVER;
+        for (int j = p.n_copy + tid; j < COVER; j += kRowsThreads) row[j] = 0.f;
+    }
+    if (tid == 0) {
+        for (int s = 0; s < NST; ++s) {
+            mbar_init(&full[s], 1);
+            newest[s] = -1;
+        }
+        fence_mbarrier_init();
+    }
+    if constexpr (TCOLS > 0) {
+        if (warp == 0) {
+            tmem_alloc(&tmem_slot, TCOLS);
+            tmem_relinquish();
+        }
+        tmem_fence_before_sync();
+    }
+    __syncthreads();
+    ColumnState<EPT> cols;
+    if constexpr (TCOLS > 0) {
+        tmem_fence_after_sync();
+        cols.start(tmem_slot, warp);
+    }
+
+    // ring of whole rows: unit u (row u mod nrows) sits in stage u mod NST; see rows_kernel
+    const uint32_t row_bytes = static_cast<uint32_t>(p.n_copy) * sizeof(float);
+    auto issue = [&](int row, int s, uint32_t phase) {
+        newest[s] = static_cast<int>(phase);
+        mbar_arrive_expect_tx(&full[s], row_bytes);
+        bulk_load(ring + static_cast<size_t>(s) * COVER * sizeof(float),
+                  p.K + static_cast<unsigned long long>(static_cast<unsigned>(row_begin + row)) *
+                            static_cast<unsigned long long>(p.ldk),
+                  row_bytes, &full[s]);
+    };
+    if (tid == 0 && nrows > 0) {
+        fence_proxy_async_smem();
+        const int first = p.resident ? min(nrows, NST) : NST;
+        for (int k = 0; k < first; ++k) issue(k % nrows, k, 0u);
+    }
+    int sbase = 0;
+    uint32_t phbase = 0u;
+    const int ahead = NST % max(1, nrows);
+    auto column_of = [&](int e) { return ((e / 4) * GT + gt) * 4 + e % 4; };
+    const bool ragged = (n & 3) != 0;
+    unsigned arrivals = 0;
+    bool alive = true;
+    // round t: the pass over K of iteration t - 1 (t = 0: column sums with the given u),
+    // then the error of that iteration, the decision, and v of iteration t
+    for (int t = 0;; ++t) {
+        const double omega = ss.omega;
+        // ---- v of this pass: written by CTA 0, kept with the columns
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) {
+            float vv[16];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int j = column_of(16 * c + 4 * k);
+                float4 v4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (t > 0 && j < n) {  // v_next is n_pad long, a multiple of 64 columns
+                    v4 = __ldcg(reinterpret_cast<const float4*>(p.v_next + j));
+                    float* e = reinterpret_cast<float*>(&v4);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (j + q >= n) {
+                            e[q] = 0.f;
+                        } else {
+                            // with momentum every thread that needs v_j blends it from v's other copy
+                            if (omega != 1.0) e[q] = std_blend(__ldcg(p.colsum + p.n_pad + j + q), e[q], omega);
+                            if (blockIdx.x == 0 && g == 0) p.v[j + q] = e[q];
+                        }
+                    }
+                }
+                vv[4 * k] = v4.x;
+                vv[4 * k + 1] = v4.y;
+                vv[4 * k + 2] = v4.z;
+                vv[4 * k + 3] = v4.w;
+            }
+            cols.set(c, vv);
+        }
+        cols.ready();
+
+        float2 y[H];
+        float wp = 0.f;
+#pragma unroll
+        for (int h = 0; h < H; ++h) y[h] = make_float2(0.f, 0.f);
+        int s_cur = sbase + g;
+        uint32_t ph = phbase;
+        while (s_cur >= NST) {
+            s_cur -= NST;
+            ph ^= 1u;
+        }
+        int par = 0;
+        for (int r = g; r < nrows; r += GR, par ^= 1) {
+            const int s = s_cur;
+            const float* stage = reinterpret_cast<const float*>(ring) + static_cast<size_t>(s) * COVER;
+            const bool ok = (p.resident && t > 0) ||
+                            mbar_wait<true>(&full[s], p.resident ? 0u : ph, p.status, p.suspend_ns);
+            float2 s2 = make_float2(0.f, 0.f), t2 = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < NCH; ++c) {
+                cols.add(c, y + 8 * c, wp);
+                float2 v2[8];
+                cols.duals(c, v2);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float4 k4 = *reinterpret_cast<const float4*>(stage + ((c * 4 + i) * GT + gt) * 4);
+                    if (ragged) {  // the copied row's last quad may hold anything past n
+                        const int j = column_of(16 * c + 4 * i);
+                        if (j + 1 >= n) k4.y = 0.f;
+                        if (j + 2 >= n) k4.z = 0.f;
+                        if (j + 3 >= n) k4.w = 0.f;
+                    }
+                    y[8 * c + 2 * i] = make_float2(k4.x, k4.y);
+                    y[8 * c + 2 * i + 1] = make_float2(k4.z, k4.w);
+                    s2 = __ffma2_rn(y[8 * c + 2 * i], v2[2 * i], s2);
+                    t2 = __ffma2_rn(y[8 * c + 2 * i + 1], v2[2 * i + 1], t2);
+                }
+            }
+            const float2 u2 = __fadd2_rn(s2, t2);
+            const float part = warp_sum(u2.x + u2.y);
+            if (lane == 0) red_s[g][par][gw] = part;
+            if (!stream_and<GT>(ok, g)) {
+                alive = false;
+                break;
+            }
+            // the stage has been read by every thread of the stream
+            if (gt == 0 && !p.resident) {
+                int row = r + ahead;
+                if (row >= nrows) row -= nrows;
+                issue(row, s, ph ^ 1u);
+            }
+            if (t == 0) {
+                wp = u_s[r];
+            } else {
+                const float x = 1.0f / (sum_warps<GW>(red_s[g][par]) + kStdEps);
+                wp = x;
+                if (omega != 1.0) {
+                    wp = std_blend(u_s[r], x, omega);
+                    stream_and<GT>(true, g);  // every thread has read u_s[r]
+                }
+                if (gt == GT - 32) {
+                    u_s[r] = wp;
+                    p.u[row_begin + r] = wp;
+                }
+            }
+            s_cur += GR;
+            while (s_cur >= NST) {
+                s_cur -= NST;
+                ph ^= 1u;
+            }
+        }
+        // ---- column sums of the CTA
+        {
+            float* prow = p.partials + static_cast<size_t>(blockIdx.x * (DUMP ? 1 : GR) + (DUMP ? 0 : g)) * p.n_pad;
+            float* to = DUMP ? dump + static_cast<size_t>(g) * COVER : prow;
+#pragma unroll
+            for (int c = 0; c < NCH; ++c) {
+                float acc[16];
+                cols.total(c, y + 8 * c, wp, acc);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int j = column_of(16 * c + 4 * k);
+                    if (j < n)
+                        *reinterpret_cast<float4*>(to + j) =
+                            make_float4(acc[4 * k], acc[4 * k + 1], acc[4 * k + 2], acc[4 * k + 3]);
+                }
+            }
+            if constexpr (DUMP) {
+                __syncthreads();
+                for (int j = tid * 4; j < n; j += kRowsThreads * 4) {
+                    float4 v[GR];
+#pragma unroll
+                    for (int k = 0; k < GR; ++k) v[k] = *reinterpret_cast<const float4*>(dump + k * COVER + j);
+#pragma unroll
+                    for (int o = 1; o < GR; o <<= 1) {
+#pragma unroll
+                        for (int k = 0; k < GR; k += 2 * o) {
+                            v[k].x += v[k + o].x;
+                            v[k].y += v[k + o].y;
+                            v[k].z += v[k + o].z;
+                            v[k].w += v[k + o].w;
+                        }
+                    }
+                    *reinterpret_cast<float4*>(prow + j) = v[0];
+                }
+            }
+        }
+        arrivals += gridDim.x;
+        if (!grid_barrier(p.arrivals, p.status, alive, arrivals, 0)) {
+            alive = false;
+            break;
+        }
+        const bool eval = t > 0 && ((t - 1) % ss.eval_freq == 0);
+        std_reduce_columns(p, gridDim.x * (DUMP ? 1 : GR), eval);
+        if (ss.momentum_start >= 0) {
+            // v of this pass for the blend of the next one (CTA 0 overwrites p.v meanwhile)
+            __syncthreads();
+            const int per = columns_per_cta(n);
+            const int j = blockIdx.x * per + tid;
+            if (tid < per && j < n) p.colsum[p.n_pad + j] = __ldcg(p.v + j);
+        }
+        arrivals += gridDim.x;
+        if (!grid_barrier(p.arrivals, p.status, true, arrivals, 0)) {
+            alive = false;
+            break;
+        }
+        std_decide(p, &ss, t, eval);
+        if (!p.resident) {
+            sbase += nrows;
+            while (sbase >= NST) {
+                sbase -= NST;
+                phbase ^= 1u;
+            }
+        }
+        __syncthreads();
+        if (ss.done) break;
+    }
+    __syncthreads();
+    if (tid == 0) {  // copies still in flight (bounded waits)
+        for (int s = 0; s < NST; ++s)
+            if (newest[s] >= 0) mbar_wait<true>(&full[s], static_cast<uint32_t>(newest[s]), p.status, p.suspend_ns);
+    }
+    if (blockIdx.x == 0) {
+        if (tid == 0) {
+            p.st->done = 1;
+            p.st->final_it = ss.final_it;
+            p.st->n_err = ss.n_err;
+            p.st->omega = ss.omega;
+            p.st->last_err = ss.last_err;
+        }
+        for (int k = tid; k < min(ss.n_err, FUGAL_MAX_RECORDED_ERRORS); k += kRowsThreads) p.st->errors[k] = ss.errors[k];
+    }
+    if constexpr (TCOLS > 0) {
+        tmem_fence_before_sync();
+        __syncthreads();
+        tmem_fence_after_sync();
+        if (warp == 0) tmem_dealloc(tmem_slot, TCOLS);
+    }
+}
+
+struct StdRowsPlan {
+    bool use = false;
+    int ept = 0, streams = 0, ctas = 0, rows_per_cta = 0, stages = 0, resident = 0, parts = 0;
+    size_t smem = 0;
+};
+constexpr int kStdShapes[][2] = {{8, 16}, {8, 32}, {4, 32}, {4, 48}, {2, 32}, {2, 48}, {2, 64}};
+
+using StdRowsFn = void (*)(StdRowsArgs);
+StdRowsFn std_rows_fn(const StdRowsPlan& pl) {
+    switch (pl.streams * 100 + pl.ept) {
+        case 816: return std_rows_kernel<16, 8>;
+        case 832: return std_rows_kernel<32, 8>;
+        case 432: return std_rows_kernel<32, 4>;
+        case 448: return std_rows_kernel<48, 4>;
+        case 232: return std_rows_kernel<32, 2>;
+        case 248: return std_rows_kernel<48, 2>;
+        default: return std_rows_kernel<64, 2>;
+    }
+}
+
+// Rows are copied in 16-byte pieces: K's rows aligned, n rounded up to 4 within ldk.
+StdRowsPlan std_rows_plan(int64_t n, int64_t ldk, const float* K) {
+    StdRowsPlan pl;
+    if (n > kStdRowsLimit || (ldk % 4) != 0 || ldk < (n + 3) / 4 * 4 || !aligned16(K)) return pl;
+    for (const auto& sh : kStdShapes)
+        if (static_cast<int64_t>(kRowsThreads / sh[0]) * sh[1] >= n) {
+            pl.streams = sh[0];
+            pl.ept = sh[1];
+            break;
+        }
+    const int want = static_cast<int>(std::min<int64_t>(sm_count(), n));
+    pl.rows_per_cta = static_cast<int>((n + want - 1) / want);
+    if (pl.rows_per_cta > kRowsMaxRows) return pl;
+    pl.ctas = static_cast<int>((n + pl.rows_per_cta - 1) / pl.rows_per_cta);
+    const size_t stage = static_cast<size_t>(kRowsThreads / pl.streams) * pl.ept * 4;
+    const size_t dump = rows_dump(pl.streams, pl.ept) ? static_cast<size_t>(kRowsThreads) * pl.ept * 4 : 0;
+    const size_t room = 227 * 1024 - kRowsStatic - dump;
+    pl.stages = static_cast<int>(
+        std::min<size_t>({room / stage, static_cast<size_t>(kRowsMaxStages), static_cast<size_t>(pl.rows_per_cta)}));
+    pl.resident = pl.stages >= pl.rows_per_cta;
+    if (!pl.resident) pl.stages -= pl.stages % pl.streams;  // a stage stays with its stream: see make_rows_plan
+    if (pl.stages < 1) return pl;
+    pl.parts = pl.ctas * (dump > 0 ? 1 : pl.streams);
+    if (pl.parts > kStdMaxParts * sm_count()) return pl;
+    pl.smem = stage * pl.stages + dump;
+    int dev = 0, coop = 0, blocks = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return pl;
+    StdRowsFn fn = std_rows_fn(pl);
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, kRowsThreads, pl.smem) != cudaSuccess || blocks < 1) {
+        (void)cudaGetLastError();
+        return pl;
+    }
+    pl.use = true;
+    return pl;
 }
 
 }  // namespace fugal
@@ -259,6 +675,49 @@ extern "C" fugal_status fugal_sinkhorn_standard_solve(const float* K, int64_t ld
         std_init_kernel<<<1, 1, 0, stream>>>(w.st, max_iterations, eval_freq, momentum_start < 0 ? -1 : momentum_start,
                                              threshold);
         FUGAL_TRY(launch_check("sinkhorn standard: init"));
+    }
+    FUGAL_TRY(cuda_check(cudaMemsetAsync(w.sync, 0, 2 * sizeof(unsigned), stream), "sinkhorn standard: clear"));
+    const StdRowsPlan plan = std_rows_plan(n, ldk, K);
+    if (plan.use) {
+        StdRowsArgs ra{};
+        ra.K = K;
+        ra.ldk = ldk;
+        ra.n = nn;
+        ra.n_copy = (nn + 3) / 4 * 4;
+        ra.rows_per_cta = plan.rows_per_cta;
+        ra.stages = plan.stages;
+        ra.resident = plan.resident;
+        ra.suspend_ns = kSuspendHintNs;
+        ra.u = u;
+        ra.v = v;
+        ra.v_next = w.v_next;
+        ra.colsum = w.colsum;
+        ra.partials = w.partials;
+        ra.errs = w.errs;
+        ra.n_pad = (n + 63) / 64 * 64;
+        ra.st = w.st;
+        ra.arrivals = w.sync;
+        ra.status = reinterpret_cast<int*>(w.sync + 1);
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        cfg.gridDim = dim3(plan.ctas, 1, 1);
+        cfg.blockDim = dim3(kRowsThreads, 1, 1);
+        cfg.dynamicSmemBytes = plan.smem;
+        cfg.stream = stream;
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        {
+            LaunchScope scope(FUGAL_KERNEL_SWEEP_F32, stream);
+            FUGAL_TRY(cuda_check(cudaLaunchKernelEx(&cfg, std_rows_fn(plan), ra), "sinkhorn standard: rows"));
+        }
+        if (record != nullptr) {
+            LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
+            std_record_kernel<<<1, 256, 0, stream>>>(w.st, w.sync + 1, static_cast<fugal_solve_record*>(record));
+            FUGAL_TRY(launch_check("sinkhorn standard: record"));
+        }
+        return FUGAL_OK;
     }
     if (g_std_pinned == nullptr) {
         void* p = nullptr;
@@ -320,7 +779,7 @@ extern "C" fugal_status fugal_sinkhorn_standard_solve(const float* K, int64_t ld
     }
     if (status == FUGAL_OK && record != nullptr) {
         LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-        std_record_kernel<<<1, 256, 0, stream>>>(w.st, static_cast<fugal_solve_record*>(record));
+        std_record_kernel<<<1, 256, 0, stream>>>(w.st, w.sync + 1, static_cast<fugal_solve_record*>(record));
         status = launch_check("sinkhorn standard: record");
     }
     cudaEventDestroy(ev[0]);

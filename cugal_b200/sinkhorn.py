@@ -173,8 +173,12 @@ class SinkhornState:
         start = TimeStamp(config.device)
         N.require_cuda(C, "C")
         C32 = C.to(torch.float32).contiguous()
-        K = exp_scale(C32, -1.0 / config.sinkhorn_regularization, torch.empty_like(C32))
-        self._std.solve(K, self.u_std, self.v_std, self._rec.data_ptr())
+        n = C32.shape[0]
+        # the solve streams 16-byte rows; K itself is returned contiguous
+        rows = torch.empty((n, padded_ld(n)), dtype=torch.float32, device=C32.device)
+        exp_scale(C32, -1.0 / config.sinkhorn_regularization, rows)
+        self._std.solve(rows, self.u_std, self.v_std, self._rec.data_ptr())
+        K = rows[:, :n].contiguous()
         if profile is not None:
             rec = read_record(self._rec.cpu())
             profile.errors, profile.iteration_count = rec.errors, rec.iteration_count

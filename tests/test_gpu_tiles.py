@@ -164,3 +164,52 @@ def test_adjoint_solve_matches_fp64(n):
     x = torch.linalg.solve(M + z @ z.T, a - z[:, 0] * (z[:, 0] @ a))
     ref = -2.0 * Pd * (Gd - x[:n, None] - x[None, n:])
     assert (dC.double() - ref).abs().max() < 1e-6 * max(float(ref.abs().max()), float(Pd.abs().max() * Gd.abs().max()))
+
+
+@pytest.mark.parametrize("n", [1, 6, 150, 1025, 2050, 4097, 6143, 8190, 8193, 12289, 16387])
+def test_standard_solve_widths(n):
+    """The persistent scaling-form solve at the edges of its shapes (rows of odd widths included) and the
+    launches above it, against FP64: u and v after 15 iterations to 2e-5, the FP32 sums' sqrt(n) 2^-24 of
+    30 updates that do not amplify them."""
+    from cugal_b200.config import Config, SinkhornMethod
+    from cugal_b200.profile import SinkhornProfile
+    from cugal_b200.sinkhorn import SinkhornState
+    C = torch.rand((n, n), generator=_gen(n), device="cuda") * 3
+    cfg = Config(device="cuda", dtype=torch.float32, sinkhorn_method=SinkhornMethod.STANDARD,
+                 sinkhorn_regularization=0.5, sinkhorn_iterations=15, sinkhorn_threshold=-1.0, sinkhorn_eval_freq=5)
+    prof = SinkhornProfile()
+    K, u, v = SinkhornState(n, cfg).solve(C, cfg, prof)
+    assert prof.iteration_count == 15 and K.is_contiguous()
+    Kd = K.double()
+    errors = []
+    ue = torch.full((n,), 1.0 / n, dtype=torch.float64, device="cuda")
+    for t in range(15):
+        ve = 1 / (ue @ Kd + 1e-16)
+        ue = 1 / (Kd @ ve + 1e-16)
+        if t % 5 == 0:
+            errors.append(float(((ue @ Kd) * ve - 1).abs().sum()))
+    assert torch.allclose(u.double(), ue, rtol=2e-5, atol=0) and torch.allclose(v.double(), ve, rtol=2e-5, atol=0)
+    np.testing.assert_allclose(prof.errors, errors, rtol=1e-2, atol=1e-6 * n)
+
+
+@pytest.mark.parametrize("n", [150, 2050, 6143, 12289])
+def test_standard_momentum_matches_the_launches(n):
+    """Momentum (and rows whose last quad holds NaN past n) in the persistent form against the form with
+    launches, which unaligned rows take: the same FP32 updates, to 2e-5."""
+    from cugal_b200 import _native as N
+    from cugal_b200.sinkhorn import exp_scale, read_record
+    C = torch.rand((n, n), generator=_gen(n), device="cuda") * 3
+    ws = torch.empty(N.workspace_size("fugal_sinkhorn_standard_workspace_size", n), dtype=torch.uint8, device="cuda")
+    got = []
+    for ld in ((n + 7) // 8 * 8, n + 1 if (n + 1) % 4 else n + 2):
+        K = torch.full((n, ld), float("nan"), device="cuda")
+        exp_scale(C, -2.0, K)
+        u = torch.full((n,), 1.0 / n, device="cuda")
+        v = u.clone()
+        rec = torch.empty(N.RECORD_BYTES, dtype=torch.uint8, device="cuda")
+        N.call("fugal_sinkhorn_standard_solve", K.data_ptr(), ld, n, u.data_ptr(), v.data_ptr(), 15, -1.0, 5, 5,
+               rec.data_ptr(), ws.data_ptr(), ws.numel(), N.stream_handle())
+        got.append((u, v, read_record(rec.cpu())))
+    (u1, v1, r1), (u2, v2, r2) = got
+    assert r1.iteration_count == r2.iteration_count == 15
+    assert torch.allclose(u1, u2, rtol=2e-5, atol=0) and torch.allclose(v1, v2, rtol=2e-5, atol=0)
