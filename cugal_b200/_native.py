@@ -75,6 +75,7 @@ SIGNATURES = {
     "fugal_sampled_lap": (_INT, [_P, _I64, _I64, _P, _P, _INT, _P, _P]),
     "fugal_exact_lap_workspace_size": (_INT, [_I64, POINTER(c_size_t)]),
     "fugal_exact_lap": (_INT, [_P, _I64, _I64, _INT, _I64, _P, _P, _P, _P, _SZ, _P]),
+    "fugal_absorb_cost": (_INT, [_P, _I64, _I64, _D, _P, _P, _P, _I64, _P, _I64, _P]),
     "fugal_count_le": (_INT, [_P, _I64, _I64, _F, _P, _P]),
     "fugal_alignment_overlap_workspace_size": (_INT, [_I64, POINTER(c_size_t)]),
     "fugal_alignment_overlap": (_INT, [_P, _P, _P, _P, _I64, _P, _P, _P, _P, _P, _SZ, _P]),

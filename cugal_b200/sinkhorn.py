@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import ctypes
 
+import numpy as np
 import torch
 
 from . import _native as N
@@ -204,9 +205,20 @@ class SinkhornState:
         start = TimeStamp(config.device)
         n = self.n
         N.require_cuda(C, "C")
-        K = (-C / config.sinkhorn_regularization).to(torch.float32)
-        cost32 = torch.zeros((n, padded_ld(n)), dtype=torch.float32, device=C.device)  # finite padding
-        cost32[:, :n] = (K.double() + self.U[:, None] + self.V[None, :]).float()
+        reg = config.sinkhorn_regularization
+        rows = C.dim() == 2 and C.stride(1) == 1 and C.stride(0) >= C.shape[1]
+        if C.dtype == torch.float32 and rows and not (C.requires_grad and torch.is_grad_enabled()):
+            K = torch.empty((n, n), dtype=torch.float32, device=C.device)
+            # -C / reg as torch divides a float32 tensor by a number: times the FP32 reciprocal
+            src, scale, K_out = C, -float(np.float32(1.0) / np.float32(reg)), K
+        else:
+            K = (-C / reg).to(torch.float32)
+            src, scale, K_out = K.detach().contiguous(), 1.0, None
+        if src.shape[0] != n or src.shape[1] != n:
+            raise ValueError(f"solve: C must be {n} x {n}")
+        cost32 = torch.empty((n, padded_ld(n)), dtype=torch.float32, device=C.device)
+        N.call("fugal_absorb_cost", src.data_ptr(), N.matrix_ld(src, "C"), n, scale, self.U.data_ptr(),
+               self.V.data_ptr(), N.ptr(K_out), n, cost32.data_ptr(), cost32.stride(0), N.stream_handle(C.device))
         self._solver.solve(cost32, self._du, self._dv, self._rec.data_ptr())
         self._cost32 = cost32
         self.U += self._du.double()

@@ -310,6 +310,12 @@ fugal_status fugal_fw_gradient_fixed_scratch(int64_t n, const int32_t* a_row_poi
                                              double out_scale, const double* U, const double* V, float* out,
                                              int64_t ldo, fugal_stream_t stream);
 
+/* The solve's input from a cost: K = scale * C (FP32; scale = -1/reg, cugal/sinkhorn.py:98)
+ * and cost32 = (float)(K + U_i + V_j) with FP64 duals, zero in the padding columns [n, ld32).
+ * K may be NULL. */
+fugal_status fugal_absorb_cost(const float* C, int64_t ldc, int64_t n, double scale, const double* U, const double* V,
+                               float* K, int64_t ldk, float* cost32, int64_t ld32, fugal_stream_t stream);
+
 /* Log-domain Sinkhorn solve (cugal/sinkhorn.py:90-120) on the absorbed cost
  * cost32 = K + U_i + V_j, warm-started at u = v = 0 relative to that frame.
  * Same iteration as the reference: per iteration a column then a row update
