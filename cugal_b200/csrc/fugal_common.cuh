@@ -62,6 +62,10 @@ FUGAL_DEVICE float warp_max(float v) {
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
+// Maximum of values >= 0 (NaNs count as 0): one instruction on their bits.
+FUGAL_DEVICE float warp_max_positive(float v) {
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, v >= 0.f ? __float_as_uint(v) : 0u));
+}
 FUGAL_DEVICE float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -14,13 +14,13 @@
 // while the CTAs exchange column sums.  When all rows of a CTA fit the ring they are
 // copied once and stay.
 //
-// What bounds it: small n, the two grid exchanges (about 6 us a sweep, of which 1.3 us
-// are each barrier and 2.5 us the FP64 column sums); from n = 3000 on the per-row
+// What bounds it: small n, the two grid exchanges (about 6 us a sweep, of which 1.4 us
+// are each barrier and 2.2 us the FP64 column sums); from n = 3000 on the per-row
 // chain of a stream (wait, exponentials, shuffles, barrier, reciprocal: about 1.5 us
 // with 32 columns a thread) against MUFU and HBM.  Time per iteration, FP32, this
-// kernel against a cluster sweep and a finalize kernel per iteration: n = 1000 8.2
-// against 23.5 us, 4096 20.0 against 45.7, 8192 51.3 against 77.5 (41 us at the copy
-// peak); BF16: 4096 19.3 against 37.6, 8192 43.7 against 62.1, 16384 120 against 158,
+// kernel against a cluster sweep and a finalize kernel per iteration: n = 1000 7.8
+// against 23.5 us, 4096 19.7 against 45.7, 8192 50.4 against 77.5 (41 us at the copy
+// peak); BF16: 4096 18.6 against 37.6, 8192 41.1 against 62.1, 16384 119 against 158,
 // 20011 217 against 275.  One exponential pair in 8 on the FMA pipe, worth 1.5% in the
 // 64-column kernel, costs 2 to 7% here (instruction issue) and is not used.
 //
@@ -42,8 +42,7 @@ namespace fugal {
 
 // This CTA's share of the columns: log(colsum), the next duals, the CTA's error and
 // largest correction.  (Not inlined: its registers would be live across the row loop.)
-__device__ __noinline__ void reduce_columns(const RowsArgs& p, int t, int parts) {
-    __shared__ double colred[kRowsWarps][128];
+__device__ __noinline__ void reduce_columns(const RowsArgs& p, int t, double (*colred)[128]) {
     __shared__ double errred[kRowsWarps];
     __shared__ float corred[kRowsWarps];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -52,7 +51,7 @@ __device__ __noinline__ void reduce_columns(const RowsArgs& p, int t, int parts)
     const bool mine = tid < per && j < p.n;
     float b_now = 0.f;
     if (mine) b_now = __ldcg(p.b_buf + (t & 1) * p.n_pad + j);
-    const double tot = own_column_sum(p.partials, p.n_pad, parts, p.n, colred);
+    const double tot = own_column_sum(p.partials, p.n_pad, static_cast<int>(gridDim.x), p.n, colred);
     double err = 0.0;
     float corr = 0.f;
     if (mine) {
@@ -64,8 +63,9 @@ __device__ __noinline__ void reduce_columns(const RowsArgs& p, int t, int parts)
     }
     const int used = (per + 31) / 32;  // warps that hold columns
     if (warp < used) {
-        err = warp_sum(err);
-        corr = warp_max(corr);
+        // (columns sit in lanes below `per`; adding the zeros of the others changes nothing)
+        for (int o = per > 16 ? 16 : per > 8 ? 8 : per > 4 ? 4 : 2; o > 0; o >>= 1) err += __shfl_xor_sync(0xffffffffu, err, o);
+        corr = warp_max_positive(corr);
         if (used == 1) {
             if (lane == 0) {
                 p.errs[blockIdx.x] = err;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
     constexpr int NCH = EPT / 16;
     constexpr int H = EPT / 2;
     constexpr bool F32 = sizeof(T) == 4;
-    constexpr bool DUMP = rows_dump(GR, EPT);
+    constexpr bool DUMP = rows_dump_bytes(GR, EPT) > 0;
     constexpr uint32_t TCOLS = ColumnState<EPT>::kTmemColumns;
     static_assert(EPT <= 64, "column sums and duals of every thread fit the tensor memory");
     static_assert(COVER * sizeof(T) <= 64 * 1024, "a stage holds one row");
@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
     __shared__ uint64_t full[kRowsMaxStages];
     __shared__ __align__(16) float red_s[GR][2][GW];
     __shared__ __align__(16) float red_m[GR][2][GW];
+    __shared__ __align__(16) double colred[kRowsWarps][128];  // also where fewer than 8 streams meet
     __shared__ float a_s[kRowsMaxRows];
     __shared__ SolveState ss;
     __shared__ int newest[kRowsMaxStages];  // phase of the newest copy into a stage (-1: none)
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
     // The duals of this thread's columns; up to 32 columns they are fetched while warp
     // 0 still takes the decision of the sweep before.
     constexpr bool PREFETCH = EPT <= 32;
-    float4 b_raw[PREFETCH ? EPT / 4 : 4];
+    float4 b_raw[EPT / 4];
     auto column_of = [&](int e) { return ((e / V) * GT + gt) * V + e % V; };
     // duals of sweep t before scaling: b_prev - omega logcs, or b_next, which the sweep
     // before wrote for omega = 1
@@ -229,18 +230,21 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
         {
             const bool next = plain && sw > 0;
             float* b_out = p.b_buf + (t & 1) * p.n_pad;
+            if (!PREFETCH) {
+#pragma unroll
+                for (int k = 0; k < EPT / 4; ++k) b_raw[k] = load_duals(4 * k, t, next, omega);
+            }
 #pragma unroll
             for (int c = 0; c < NCH; ++c) {
                 float bb[16];
+                if (PREFETCH && !next) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if (!PREFETCH) b_raw[k] = load_duals(16 * c + 4 * k, t, next, omega);
-                    else if (!next) b_raw[4 * c + k] = load_duals(16 * c + 4 * k, t, false, omega);
+                    for (int k = 0; k < 4; ++k) b_raw[4 * c + k] = load_duals(16 * c + 4 * k, t, false, omega);
                 }
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const int j = column_of(16 * c + 4 * k);
-                    const float4 b = b_raw[(PREFETCH ? 4 * c : 0) + k];
+                    const float4 b = b_raw[4 * c + k];
                     if (blockIdx.x == 0 && g == 0 && j < n) *reinterpret_cast<float4*>(b_out + j) = b;
                     const float b4[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
@@ -387,18 +391,22 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
         // ---- this CTA's column sums: the streams' sums (the pending rows included) meet in
         //      shared memory, so that the grid exchanges one row per CTA
         {
-            float* prow = p.partials + static_cast<size_t>(blockIdx.x * (DUMP ? 1 : GR) + (DUMP ? 0 : g)) * p.n_pad;
+            float* prow = p.partials + static_cast<size_t>(blockIdx.x) * p.n_pad;
             float* mine = DUMP ? dump + static_cast<size_t>(g) * COVER : prow;
 #pragma unroll
             for (int c = 0; c < NCH; ++c) {
                 float acc[16];
                 cols.total(c, y + 8 * c, wp, acc);
+                if constexpr (GR > 1 && !DUMP) {
+                    meet_streams<GR, GT, V>(reinterpret_cast<float*>(colred), acc, c, g, gt, n, prow);
+                } else {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int j = column_of(16 * c + 4 * k);
-                    if (j < n)  // partial rows are n_pad wide, a multiple of 64 columns
-                        *reinterpret_cast<float4*>(mine + j) =
-                            make_float4(acc[4 * k], acc[4 * k + 1], acc[4 * k + 2], acc[4 * k + 3]);
+                    for (int k = 0; k < 4; ++k) {
+                        const int j = column_of(16 * c + 4 * k);
+                        if (j < n)  // partial rows are n_pad wide, a multiple of 64 columns
+                            *reinterpret_cast<float4*>(mine + j) =
+                                make_float4(acc[4 * k], acc[4 * k + 1], acc[4 * k + 2], acc[4 * k + 3]);
+                    }
                 }
             }
             if constexpr (DUMP) {
@@ -426,7 +434,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
             alive = false;
             break;
         }
-        reduce_columns(p, t, gridDim.x * (DUMP ? 1 : GR));
+        reduce_columns(p, t, colred);
         arrivals += gridDim.x;
         if (!grid_barrier(&p.st->arrivals, &p.st->status, true, arrivals, p.wait_limit_ns)) {
             alive = false;
@@ -434,7 +442,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
         }
         if (PREFETCH && plain) {
 #pragma unroll
-            for (int k = 0; k < (PREFETCH ? EPT / 4 : 0); ++k) b_raw[k] = load_duals(4 * k, t + 1, true, 1.f);
+            for (int k = 0; k < EPT / 4; ++k) b_raw[k] = load_duals(4 * k, t + 1, true, 1.f);
         }
         take_decision(p, &ss);
         ubase += nrows;
@@ -526,8 +534,8 @@ RowsFn rows_fn(const RowsPlan& pl) {
 
 // (streams, columns per thread) in the order of the columns they cover,
 // 512 / streams * ept: the narrowest that covers n.  Measured per iteration: BF16 at
-// n = 8192 43.7 us as {4, 64}, 51.2 as {2, 32}; n = 6000 29.6 as {4, 48}, 39.1 as
-// {2, 32}; n = 4096 19.3 as {4, 32}, 25.5 as {8, 64}.  FP32 rows of 6145 to 8192
+// n = 8192 41.1 us as {4, 64}, 51.2 as {2, 32}; n = 6000 28.2 as {4, 48}, 39.1 as
+// {2, 32}; n = 4096 18.6 as {4, 32}, 25.5 as {8, 64}.  FP32 rows of 6145 to 8192
 // columns take two streams, so that two stages of 32 KB are left for each.  Wider
 // rows: FP32 sweeps are at 85% of the copy peak in the cluster kernel; 16-bit ones of
 // more than 24576 columns have too few stages left here (469 against 454 us at 32768).
@@ -565,8 +573,8 @@ fugal_status make_rows_plan(int64_t n, int dt, RowsPlan& pl, bool device) {
     if (pl.rows_per_cta > kRowsMaxRows) return FUGAL_OK;
     pl.ctas = static_cast<int>((n + pl.rows_per_cta - 1) / pl.rows_per_cta);
     const size_t stage = static_cast<size_t>(kRowsThreads / pl.streams) * pl.ept * es;
-    const size_t dump = rows_dump(pl.streams, pl.ept) ? static_cast<size_t>(kRowsThreads) * pl.ept * 4 : 0;
-    pl.parts = pl.ctas * (dump > 0 ? 1 : pl.streams);
+    const size_t dump = rows_dump_bytes(pl.streams, pl.ept);
+    pl.parts = pl.ctas;
     const size_t room = 227 * 1024 - kRowsStatic - dump;
     pl.stages = static_cast<int>(std::min<size_t>({room / stage, static_cast<size_t>(kRowsMaxStages),
                                                    static_cast<size_t>(pl.rows_per_cta)}));

@@ -12,12 +12,14 @@
 namespace fugal {
 
 constexpr int kRowsThreads = 512;
-// The streams' column sums meet in shared memory, unless two streams of more than 32
-// columns per thread need it for their stages (each then writes a partial row).
-constexpr bool rows_dump(int streams, int ept) { return streams > 1 && ept <= 32; }
 constexpr int kRowsWarps = kRowsThreads / 32;
 constexpr int kRowsMaxRows = 256;      // rows per CTA the row-dual staging holds
 constexpr int kRowsStatic = 24 * 1024; // shared memory kept for the static arrays
+// Eight streams (rows of up to 4096 columns) leave room for all their column sums next to the
+// stages; fewer meet 8 columns per thread at a time in `colred` (meet_streams).
+constexpr size_t rows_dump_bytes(int streams, int ept) {
+    return streams == 8 ? static_cast<size_t>(kRowsThreads) * ept * 4 : 0;
+}
 
 // Barrier over the GT threads of stream g; true if every thread voted true.
 template <int GT>
@@ -142,6 +144,52 @@ struct ColumnState<EPT, false> {
     }
 };
 
+// The column sums of GR = 2 or 4 streams: every thread holds 16 sums (chunk c) of its
+// stream; their totals go to prow, neighbouring streams first.  8 columns of every thread
+// meet at a time, 8 GT consecutive ones, in 16 KB of shared memory.  A partial row per
+// stream instead made the exchange half of a sweep at n = 8192 BF16 (4 streams): the CTAs'
+// FP64 sums 16400 cycles and the writes 8000, against 8200 and 5000.
+template <int GR, int GT, int V>
+FUGAL_DEVICE void meet_streams(float* meet, const float* acc, int c, int g, int gt, int n, float* prow) {
+    static_assert(GR == 2 || GR == 4, "a thread adds 8 / GR columns, at least 2");
+    constexpr int W = 8 / GR;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        __syncthreads();  // the columns before have been read
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int at = (4 * k / V) * GT * V + gt * V + 4 * k % V;
+            const float* a4 = acc + 8 * h + 4 * k;
+            *reinterpret_cast<float4*>(meet + g * GT * 8 + at) = make_float4(a4[0], a4[1], a4[2], a4[3]);
+        }
+        __syncthreads();
+        const int at = static_cast<int>(threadIdx.x) * W;
+        const int j = (16 * c + 8 * h) * GT + at;
+        float v[GR][W];
+#pragma unroll
+        for (int k = 0; k < GR; ++k) {
+#pragma unroll
+            for (int q = 0; q < W; q += 2) {
+                const float2 f = *reinterpret_cast<const float2*>(meet + k * GT * 8 + at + q);
+                v[k][q] = f.x;
+                v[k][q + 1] = f.y;
+            }
+        }
+#pragma unroll
+        for (int o = 1; o < GR; o <<= 1) {
+#pragma unroll
+            for (int k = 0; k < GR; k += 2 * o) {
+#pragma unroll
+                for (int q = 0; q < W; ++q) v[k][q] += v[k + o][q];
+            }
+        }
+        if (j < n) {  // partial rows are n_pad wide, a multiple of 64 columns
+#pragma unroll
+            for (int q = 0; q < W; q += 2) *reinterpret_cast<float2*>(prow + j + q) = make_float2(v[0][q], v[0][q + 1]);
+        }
+    }
+}
+
 // FP64 sums of this CTA's share of the columns over `parts` partial rows: on return
 // thread t < 4 * per holds the sum of column 4 * per * blockIdx.x + t (others: 0).
 // Lanes of a warp: cgp column quads (a power of two) x the rest over partial rows;
@@ -236,7 +284,7 @@ FUGAL_DEVICE void grid_error(const double* errs, const float* corrs, double& e, 
         }
     }
     e = warp_sum(e);
-    c = warp_max(c);
+    c = warp_max_positive(c);
 }
 
 }  // namespace fugal

@@ -32,7 +32,6 @@ namespace fugal {
 constexpr float kStdEps = 1e-16f;  // M_EPS, cugal/sinkhorn.py:12
 constexpr int kStdThreads = 256;
 constexpr int kStdRowsLimit = 16384;  // columns of the persistent form
-constexpr int kStdMaxParts = 4;       // partial rows per CTA it writes at most
 
 struct StdState {
     int done;
@@ -78,7 +77,7 @@ StdWs std_layout(int64_t n, char* base) {
     const size_t n_pad = (static_cast<size_t>(n) + 63) / 64 * 64;
     w.colsum = reinterpret_cast<float*>(take(2 * n_pad * 4));
     w.v_next = reinterpret_cast<float*>(take(n_pad * 4));
-    const size_t rows = std::max<size_t>(std_chunks(n), n <= kStdRowsLimit ? kStdMaxParts * sm_count() : 0);
+    const size_t rows = std::max<size_t>(std_chunks(n), n <= kStdRowsLimit ? sm_count() : 0);
     w.partials = reinterpret_cast<float*>(take(rows * n_pad * 4));
     w.errs = reinterpret_cast<double*>(take(static_cast<size_t>(sm_count()) * 8));
     w.sync = reinterpret_cast<unsigned*>(take(2 * sizeof(unsigned)));
@@ -234,7 +233,7 @@ __global__ void __launch_bounds__(kStdThreads) std_update_kernel(float* P, long 
 
 // Per iteration: one read of K (144 MB at n = 6000, 22 us at the copy peak) where the
 // four launches of the wider form read it twice (31 + 49 us) and paid their gaps: 92 us
-// against 45 us an iteration at n = 6000.
+// against 40 us an iteration at n = 6000.
 struct StdRowsArgs {
     const float* K;
     long long ldk;
@@ -261,14 +260,13 @@ FUGAL_DEVICE float std_blend(float x, float y, double w) {
     return powf(x, static_cast<float>(1.0 - w)) * powf(y, static_cast<float>(w));
 }
 
-__device__ __noinline__ void std_reduce_columns(const StdRowsArgs& p, int parts, bool eval) {
-    __shared__ double colred[kRowsWarps][128];
+__device__ __noinline__ void std_reduce_columns(const StdRowsArgs& p, bool eval, double (*colred)[128]) {
     __shared__ double red[32];
     const int per = columns_per_cta(p.n);
     const int j = blockIdx.x * per + threadIdx.x;
     const bool mine = static_cast<int>(threadIdx.x) < per && j < p.n;
     const float vj = mine && eval ? __ldcg(p.v + j) : 0.f;
-    const double tot = own_column_sum(p.partials, p.n_pad, parts, p.n, colred);
+    const double tot = own_column_sum(p.partials, p.n_pad, static_cast<int>(gridDim.x), p.n, colred);
     double err = 0.0;
     if (mine) {
         const float cf = static_cast<float>(tot);
@@ -312,13 +310,14 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
     constexpr int COVER = GT * EPT;
     constexpr int NCH = EPT / 16;
     constexpr int H = EPT / 2;
-    constexpr bool DUMP = rows_dump(GR, EPT);
+    constexpr bool DUMP = rows_dump_bytes(GR, EPT) > 0;
     constexpr uint32_t TCOLS = ColumnState<EPT>::kTmemColumns;
     extern __shared__ __align__(128) unsigned char ring[];
     float* dump = reinterpret_cast<float*>(ring + static_cast<size_t>(p.stages) * COVER * sizeof(float));  // DUMP
     __shared__ uint64_t full[kRowsMaxStages];
     __shared__ int newest[kRowsMaxStages];  // phase of the newest copy into a stage (-1: none)
     __shared__ __align__(16) float red_s[GR][2][GW];
+    __shared__ __align__(16) double colred[kRowsWarps][128];  // also where fewer than 8 streams meet
     __shared__ float u_s[kRowsMaxRows];
     __shared__ StdState ss;
     __shared__ uint32_t tmem_slot;
@@ -384,15 +383,22 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
     for (int t = 0;; ++t) {
         const double omega = ss.omega;
         // ---- v of this pass: written by CTA 0, kept with the columns
+        float4 v_raw[EPT / 4];  // all loads in flight
+#pragma unroll
+        for (int k = 0; k < EPT / 4; ++k) {
+            const int j = column_of(4 * k);
+            v_raw[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            // v_next is n_pad long, a multiple of 64 columns
+            if (t > 0 && j < n) v_raw[k] = __ldcg(reinterpret_cast<const float4*>(p.v_next + j));
+        }
 #pragma unroll
         for (int c = 0; c < NCH; ++c) {
             float vv[16];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int j = column_of(16 * c + 4 * k);
-                float4 v4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (t > 0 && j < n) {  // v_next is n_pad long, a multiple of 64 columns
-                    v4 = __ldcg(reinterpret_cast<const float4*>(p.v_next + j));
+                float4 v4 = v_raw[4 * c + k];
+                if (t > 0 && j < n) {
                     float* e = reinterpret_cast<float*>(&v4);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
@@ -486,18 +492,22 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
         }
         // ---- column sums of the CTA
         {
-            float* prow = p.partials + static_cast<size_t>(blockIdx.x * (DUMP ? 1 : GR) + (DUMP ? 0 : g)) * p.n_pad;
+            float* prow = p.partials + static_cast<size_t>(blockIdx.x) * p.n_pad;
             float* to = DUMP ? dump + static_cast<size_t>(g) * COVER : prow;
 #pragma unroll
             for (int c = 0; c < NCH; ++c) {
                 float acc[16];
                 cols.total(c, y + 8 * c, wp, acc);
+                if constexpr (GR > 1 && !DUMP) {
+                    meet_streams<GR, GT, 4>(reinterpret_cast<float*>(colred), acc, c, g, gt, n, prow);
+                } else {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int j = column_of(16 * c + 4 * k);
-                    if (j < n)
-                        *reinterpret_cast<float4*>(to + j) =
-                            make_float4(acc[4 * k], acc[4 * k + 1], acc[4 * k + 2], acc[4 * k + 3]);
+                    for (int k = 0; k < 4; ++k) {
+                        const int j = column_of(16 * c + 4 * k);
+                        if (j < n)
+                            *reinterpret_cast<float4*>(to + j) =
+                                make_float4(acc[4 * k], acc[4 * k + 1], acc[4 * k + 2], acc[4 * k + 3]);
+                    }
                 }
             }
             if constexpr (DUMP) {
@@ -526,7 +536,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
             break;
         }
         const bool eval = t > 0 && ((t - 1) % ss.eval_freq == 0);
-        std_reduce_columns(p, gridDim.x * (DUMP ? 1 : GR), eval);
+        std_reduce_columns(p, eval, colred);
         if (ss.momentum_start >= 0) {
             // v of this pass for the blend of the next one (CTA 0 overwrites p.v meanwhile)
             __syncthreads();
@@ -575,7 +585,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
 
 struct StdRowsPlan {
     bool use = false;
-    int ept = 0, streams = 0, ctas = 0, rows_per_cta = 0, stages = 0, resident = 0, parts = 0;
+    int ept = 0, streams = 0, ctas = 0, rows_per_cta = 0, stages = 0, resident = 0;
     size_t smem = 0;
 };
 constexpr int kStdShapes[][2] = {{8, 16}, {8, 32}, {4, 32}, {4, 48}, {2, 32}, {2, 48}, {2, 64}};
@@ -608,15 +618,13 @@ StdRowsPlan std_rows_plan(int64_t n, int64_t ldk, const float* K) {
     if (pl.rows_per_cta > kRowsMaxRows) return pl;
     pl.ctas = static_cast<int>((n + pl.rows_per_cta - 1) / pl.rows_per_cta);
     const size_t stage = static_cast<size_t>(kRowsThreads / pl.streams) * pl.ept * 4;
-    const size_t dump = rows_dump(pl.streams, pl.ept) ? static_cast<size_t>(kRowsThreads) * pl.ept * 4 : 0;
+    const size_t dump = rows_dump_bytes(pl.streams, pl.ept);
     const size_t room = 227 * 1024 - kRowsStatic - dump;
     pl.stages = static_cast<int>(
         std::min<size_t>({room / stage, static_cast<size_t>(kRowsMaxStages), static_cast<size_t>(pl.rows_per_cta)}));
     pl.resident = pl.stages >= pl.rows_per_cta;
     if (!pl.resident) pl.stages -= pl.stages % pl.streams;  // a stage stays with its stream: see make_rows_plan
     if (pl.stages < 1) return pl;
-    pl.parts = pl.ctas * (dump > 0 ? 1 : pl.streams);
-    if (pl.parts > kStdMaxParts * sm_count()) return pl;
     pl.smem = stage * pl.stages + dump;
     int dev = 0, coop = 0, blocks = 0;
     cudaGetDevice(&dev);
