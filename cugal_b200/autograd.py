@@ -205,21 +205,26 @@ class SinkhornPlanUnrolled(torch.autograd.Function):
         seg_end = T
         while seg_end > 0:
             seg_start = ((seg_end - 1) // every) * every
-            u, v = (x.clone() for x in ctx.checkpoints[seg_start])
-            states = [(u.clone(), v.clone())]          # (u_t, v_t) for t = seg_start .. seg_end
-            for _ in range(seg_start, seg_end):
-                N.call("fugal_sinkhorn_log_step", Kt.data_ptr(), n, n, n, u.data_ptr(), v.data_ptr(), 1.0, stream)
-                N.call("fugal_sinkhorn_log_step", K.data_ptr(), n, n, n, v.data_ptr(), u.data_ptr(), 1.0, stream)
-                states.append((u.clone(), v.clone()))
+            # (u_t, v_t) for t = seg_start .. seg_end, each step writing the next pair
+            steps, ld = seg_end - seg_start, (n + 63) // 64 * 64  # every vector on a 256-byte boundary
+            duals = torch.zeros((steps + 1, 2, ld), dtype=torch.float32, device=dev)[:, :, :n]
+            states = [tuple(pair) for pair in duals]
+            for mine, saved in zip(states[0], ctx.checkpoints[seg_start]):
+                mine.copy_(saved)
+            grads = iter(torch.zeros((2 * steps, ld), dtype=torch.float64, device=dev)[:, :n])
+            for (u, _), (u_next, v_next) in zip(states, states[1:]):
+                N.call("fugal_sinkhorn_log_step", Kt.data_ptr(), n, n, n, u.data_ptr(), v_next.data_ptr(), 1.0, stream)
+                N.call("fugal_sinkhorn_log_step", K.data_ptr(), n, n, n, v_next.data_ptr(), u_next.data_ptr(), 1.0,
+                       stream)
             for t in range(seg_end - 1, seg_start - 1, -1):
                 u_t = states[t - seg_start][0]
                 u_next, v_next = states[t + 1 - seg_start]
                 # row half: u_{t+1} = -LSE_j(K + v_{t+1})
                 step_back(u_next, v_next, gu, 1, gv)
                 # column half: v_{t+1} = -LSE_i(K + u_t)
-                gu = torch.zeros(n, dtype=torch.float64, device=dev)
+                gu = next(grads)
                 step_back(v_next, u_t, gv, 0, gu)
-                gv = torch.zeros(n, dtype=torch.float64, device=dev)
+                gv = next(grads)
             seg_end = seg_start
         return -gK / ctx.reg, None, None
 

@@ -1086,10 +1086,10 @@ __global__ void __launch_bounds__(kFinThreads) finalize_kernel(const float* part
 }
 
 // First column update of a solve, max-stabilised: per (row chunk, column) an
-// online (max, sum) of exp(cost_ij + a_i).
-__global__ void __launch_bounds__(256) column_pass_kernel(const float* L, long long ld, int n, const float* a,
-                                                          int rows_per_chunk, float2* part, long long n_pad) {
-    // Per column and row chunk: online (max, sum) of 2^((L_ij + a_i) log2 e), base-2 units,
+// online (max, sum) of exp(cost_ij).
+__global__ void __launch_bounds__(256) column_pass_kernel(const float* L, long long ld, int n, int rows_per_chunk,
+                                                          float2* part, long long n_pad) {
+    // Per column and row chunk: online (max, sum) of 2^(L_ij log2 e), base-2 units,
     // eight rows per step (their loads are all in flight before the exponentials).
     const int j0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     const int chunk = blockIdx.y;
@@ -1110,15 +1110,14 @@ __global__ void __launch_bounds__(256) column_pass_kernel(const float* L, long l
         for (int r = 0; r < RR; ++r) {
             const int row = i + r;
             if (row < i1) {
-                const float ai = a[row];
                 const float* src = L + static_cast<size_t>(row) * ld + j0;
                 if (full4) {
                     const float4 v = *reinterpret_cast<const float4*>(src);
-                    x[r][0] = (v.x + ai) * kLog2e; x[r][1] = (v.y + ai) * kLog2e;
-                    x[r][2] = (v.z + ai) * kLog2e; x[r][3] = (v.w + ai) * kLog2e;
+                    x[r][0] = v.x * kLog2e; x[r][1] = v.y * kLog2e;
+                    x[r][2] = v.z * kLog2e; x[r][3] = v.w * kLog2e;
                 } else {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) x[r][q] = (j0 + q < n) ? (src[q] + ai) * kLog2e : -INFINITY;
+                    for (int q = 0; q < 4; ++q) x[r][q] = (j0 + q < n) ? src[q] * kLog2e : -INFINITY;
                 }
             } else {
 #pragma unroll
@@ -1157,8 +1156,8 @@ struct InitArgs {
 // combines the 8 pairs.  Grid: ceil(n / 32) blocks of 256 threads.
 constexpr int kMergeLanes = 8;
 __global__ void __launch_bounds__(256) column_merge_kernel(const float2* part, int nchunks, long long part_ld,
-                                                           long long n_pad, int n, float* b_buf, float* logcs,
-                                                           SolveState* st, InitArgs ia) {
+                                                           long long n_pad, int n, float* a, float* b_buf,
+                                                           float* logcs, SolveState* st, InitArgs ia) {
     __shared__ float2 red[kMergeLanes][32];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         st->it = 0;
@@ -1186,6 +1185,8 @@ __global__ void __launch_bounds__(256) column_merge_kernel(const float2* part, i
     }
     const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
     const int j = blockIdx.x * 32 + lane;
+    if (grp == 1)  // the row duals start at 0
+        for (long long k = j; k < n_pad; k += gridDim.x * 32) a[k] = 0.f;
     float M = -INFINITY, S = 0.f;
     if (j < n) {
         for (int c = grp; c < nchunks; c += kMergeLanes) M = fmaxf(M, part[static_cast<size_t>(c) * part_ld + j].x);
@@ -1778,7 +1779,6 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
 
     // ---- iteration 0, column update: v_0 = -LSE_i(cost32_ij + a_i), a = 0, from
     //      the caller's column partials (written with the cost) or a pass over cost32
-    FUGAL_TRY(cuda_check(cudaMemsetAsync(w.a, 0, w.n_pad * 4, stream), "sinkhorn: clear row duals"));
     const float2* part = reinterpret_cast<const float2*>(w.partials);
     int chunks = colpass_chunks(n);
     long long part_ld = w.n_pad;
@@ -1790,7 +1790,7 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
         const int rows_per_chunk = static_cast<int>((n + chunks - 1) / chunks);
         dim3 grid(static_cast<unsigned>((n + kColThreads * 4 - 1) / (kColThreads * 4)), chunks);
         LaunchScope scope(FUGAL_KERNEL_COLUMN_PASS, stream);
-        column_pass_kernel<<<grid, kColThreads, 0, stream>>>(p.cost32, p.ld32, static_cast<int>(n), w.a,
+        column_pass_kernel<<<grid, kColThreads, 0, stream>>>(p.cost32, p.ld32, static_cast<int>(n),
                                                               rows_per_chunk, reinterpret_cast<float2*>(w.partials),
                                                               w.n_pad);
         FUGAL_TRY(launch_check("sinkhorn: column pass"));
@@ -1800,7 +1800,7 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
         InitArgs ia{p.max_iterations, p.eval_freq, p.momentum_start < 0 ? -1 : p.momentum_start, p.threshold};
         LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
         column_merge_kernel<<<static_cast<unsigned>((n + 31) / 32), 256, 0, stream>>>(
-            part, chunks, part_ld, w.n_pad, static_cast<int>(n), w.b_buf, w.logcs, w.st, ia);
+            part, chunks, part_ld, w.n_pad, static_cast<int>(n), w.a, w.b_buf, w.logcs, w.st, ia);
         FUGAL_TRY(launch_check("sinkhorn: column merge"));
     }
 
@@ -1868,12 +1868,10 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
     }
     int* g_pinned_done = g_pinned_ring + g_pinned_next;
     g_pinned_next = (g_pinned_next + 2) % kPinnedSlots;
-    cudaEvent_t ev[2] = {nullptr, nullptr};
-    FUGAL_TRY(cuda_check(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming), "sinkhorn: event"));
-    FUGAL_TRY(cuda_check(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming), "sinkhorn: event"));
+    cudaEvent_t ev[2] = {nullptr, nullptr};  // made at the first poll: most solves have none
     auto destroy = [&]() {
-        cudaEventDestroy(ev[0]);
-        cudaEventDestroy(ev[1]);
+        for (cudaEvent_t e : ev)
+            if (e != nullptr) cudaEventDestroy(e);
     };
     int slot = 0;
     int poll_slot = -1, poll_t = 0;  // the copy of `done` in flight, issued after sweep poll_t
@@ -1981,6 +1979,8 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
             status = cuda_check(cudaMemcpyAsync(&g_pinned_done[slot], &w.st->done, sizeof(int),
                                                 cudaMemcpyDeviceToHost, stream),
                                 "sinkhorn: poll copy");
+            if (status == FUGAL_OK && ev[slot] == nullptr)
+                status = cuda_check(cudaEventCreateWithFlags(&ev[slot], cudaEventDisableTiming), "sinkhorn: event");
             if (status == FUGAL_OK) status = cuda_check(cudaEventRecord(ev[slot], stream), "sinkhorn: poll event");
             poll_slot = slot;
             poll_t = t + len - 1;

@@ -383,15 +383,14 @@ def find_quasi_permutation_matrix(A: Adjacency, B: Adjacency, features: Features
     solve_times = []
     for lam in range(config.iter_count):
         for it in range(1, config.frank_wolfe_iter_count + 1):
-            start_time = TimeStamp(config.device)
+            gradient_start = TimeStamp(config.device)
             engine.gradient(lam)
-            profile.log_time(start_time, Phase.GRADIENT)
-
-            start_time = TimeStamp(config.device)
+            solve_start = TimeStamp(config.device)
             engine.solve()
-            end_time = TimeStamp(config.device)
-            solve_times.append((start_time, end_time))
-            profile.log_time(start_time, Phase.SINKHORN)
+            solve_end = TimeStamp(config.device)
+            profile.log_time(gradient_start, Phase.GRADIENT, solve_start)
+            profile.log_time(solve_start, Phase.SINKHORN, solve_end)
+            solve_times.append((solve_start, solve_end))
 
             alpha = 2.0 / float(2.0 + it)
             gap = engine.update(alpha, lam)

@@ -49,7 +49,8 @@ class TimeStamp:
     def __init__(self, device: str):
         if "cuda" in device:
             self.time = torch.cuda.Event(enable_timing=True)
-            self.time.record()
+            stream, index, kind = torch._C._cuda_getCurrentStream(torch.cuda.current_device())
+            self.time.record(torch.cuda.Stream(stream_id=stream, device_index=index, device_type=kind))
         else:
             self.time = time()
         self.device = device
@@ -82,8 +83,9 @@ class Profile:
     def frank_wolfe_steps(self) -> list[float]:
         return list(self._steps)
 
-    def log_time(self, start_time: TimeStamp, phase: Phase):
-        now = TimeStamp(start_time.device)
+    def log_time(self, start_time: TimeStamp, phase: Phase, now: TimeStamp | None = None):
+        """Adds the time from ``start_time`` to ``now`` (default: a new time stamp)."""
+        now = TimeStamp(start_time.device) if now is None else now
         if now.is_cuda_event():
             self._pending.append((phase, start_time, now))
         else:
