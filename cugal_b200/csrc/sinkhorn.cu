@@ -184,8 +184,6 @@ __global__ void __launch_bounds__(THREADS, 2) sweep_kernel(const SweepArgs p) {
     unsigned char* stage_base = reinterpret_cast<unsigned char*>(a_s + p.rows_pad);
 
     SolveState* st = p.st;
-    if (*reinterpret_cast<volatile int*>(&st->done)) return;  // uniform: written by an earlier kernel
-
     const int tid = threadIdx.x;
     const int C = static_cast<int>(cluster_nctarank());
     const int rank = static_cast<int>(cluster_ctarank());
@@ -197,40 +195,10 @@ __global__ void __launch_bounds__(THREADS, 2) sweep_kernel(const SweepArgs p) {
     const int row_begin = cid * p.rows_per_cluster;
     const int row_end = min(n, row_begin + p.rows_per_cluster);
     const int nbatch = row_end > row_begin ? (row_end - row_begin + R - 1) / R : 0;
-    const int t = st->it;
-    const float omega = static_cast<float>(st->omega);
-    const bool momentum = omega != 1.0f;
-    // the absorb sweep always takes the exact path: it writes the copy centred on the row maximum
-    const bool exact_only = ABSORB || st->exact_next != 0 || momentum;  // uniform
     const uint32_t row_bytes = static_cast<uint32_t>(ncopy) * sizeof(T);
     const size_t stage_bytes = static_cast<size_t>(R) * p.slice_w * sizeof(T);
-    const float* b_prev = p.b_buf + ((t - 1) & 1) * p.n_pad;
-    float* b_out = p.b_buf_w + (t & 1) * p.n_pad;
     const float2 log2e2 = make_float2(kLog2e, kLog2e);
 
-    // Column duals of this sweep: b = b_off + b_prev - w log(colsum_prev); kept as b * log2 e.
-    for (int j = tid; j < p.slice_w; j += THREADS) {
-        float b = 0.f;
-        if (j < nvalid) {
-            const int jg = col0 + j;
-            b = b_prev[jg] - omega * p.logcs[jg];
-            if (p.b_off != nullptr) b += p.b_off[jg];
-            if (cid == 0) {
-                if (ABSORB) {
-                    p.b_snap[jg] = b;
-                    b_out[jg] = 0.f;
-                } else {
-                    b_out[jg] = b;
-                }
-            }
-        }
-        // columns past n contribute 2^(-inf) = 0 without any masking in the hot loop
-        // 16-bit rows (8 columns per 16-byte chunk): split layout, columns 8g..8g+3 at
-        // [4g, 4g+4) and 8g+4..8g+7 at [slice_w/2 + 4g, ...), so consecutive threads read
-        // consecutive 16 bytes (no bank conflicts); FP32 rows (4 per chunk) are already so
-        const int js = (V == 8) ? (((j & 7) < 4 ? 0 : p.slice_w / 2) + (j >> 3) * 4 + (j & 3)) : j;
-        b_s[js] = j < nvalid ? b * kLog2e : -INFINITY;
-    }
     // Stage columns [ncopy, slice_w) are never written by the bulk copies: zero
     // them once so that they hold finite values (their b_s is -inf).
     if (ncopy < p.slice_w) {
@@ -240,13 +208,6 @@ __global__ void __launch_bounds__(THREADS, 2) sweep_kernel(const SweepArgs p) {
                 T* row = reinterpret_cast<T*>(stage_base + s * stage_bytes) + static_cast<size_t>(r) * p.slice_w;
                 for (int j = tid; j < tail; j += THREADS) row[ncopy + j] = from_float<T>(0.f);
             }
-    }
-    // Row duals of the previous sweep (the fast path's exponent reference and
-    // the momentum term), read once here instead of on every batch's critical path.
-    for (int i = tid; i < row_end - row_begin; i += THREADS) {
-        float a = p.a[row_begin + i];
-        if (p.a_off != nullptr) a += p.a_off[row_begin + i];
-        a_s[i] = a;
     }
     if (tid == 0) {
         for (int s = 0; s < p.stages; ++s) mbar_init(&full[s], 1);
@@ -270,10 +231,65 @@ __global__ void __launch_bounds__(THREADS, 2) sweep_kernel(const SweepArgs p) {
         }
     };
     int issued = 0;
-    if (tid == 0) {
-        issued = min(p.stages, nbatch);
-        for (int bt = 0; bt < issued; ++bt) issue(bt, bt);
+    auto fill = [&]() {
+        if (tid == 0) {
+            issued = min(p.stages, nbatch);
+            for (int bt = 0; bt < issued; ++bt) issue(bt, bt);
+        }
+    };
+    // Up to here nothing of the kernels before was read.  The FP32 cost is older than they
+    // are: its first rows are fetched while the previous sweep's column sums are finished.
+    launch_dependents();
+    constexpr bool OLD_COST = sizeof(T) == 4;
+    if (OLD_COST) {
+        fence_proxy_async_smem();
+        fill();
     }
+    wait_for_previous();
+    if (*reinterpret_cast<volatile int*>(&st->done)) {  // uniform: written by an earlier kernel
+        // the copies in flight land before their shared memory is released
+        for (int bt = 0; bt < issued; ++bt) mbar_wait(&full[bt], 0u, &st->status, p.suspend_ns);
+        return;
+    }
+    const int t = st->it;
+    const float omega = static_cast<float>(st->omega);
+    const bool momentum = omega != 1.0f;
+    // the absorb sweep always takes the exact path: it writes the copy centred on the row maximum
+    const bool exact_only = ABSORB || st->exact_next != 0 || momentum;  // uniform
+    const float* b_prev = p.b_buf + ((t - 1) & 1) * p.n_pad;
+    float* b_out = p.b_buf_w + (t & 1) * p.n_pad;
+    // Column duals of this sweep: b = b_off + b_prev - w log(colsum_prev); kept as b * log2 e.
+    for (int j = tid; j < p.slice_w; j += THREADS) {
+        float b = 0.f;
+        if (j < nvalid) {
+            const int jg = col0 + j;
+            b = b_prev[jg] - omega * p.logcs[jg];
+            if (p.b_off != nullptr) b += p.b_off[jg];
+            if (cid == 0) {
+                if (ABSORB) {
+                    p.b_snap[jg] = b;
+                    b_out[jg] = 0.f;
+                } else {
+                    b_out[jg] = b;
+                }
+            }
+        }
+        // columns past n contribute 2^(-inf) = 0 without any masking in the hot loop
+        // 16-bit rows (8 columns per 16-byte chunk): split layout, columns 8g..8g+3 at
+        // [4g, 4g+4) and 8g+4..8g+7 at [slice_w/2 + 4g, ...), so consecutive threads read
+        // consecutive 16 bytes (no bank conflicts); FP32 rows (4 per chunk) are already so
+        const int js = (V == 8) ? (((j & 7) < 4 ? 0 : p.slice_w / 2) + (j >> 3) * 4 + (j & 3)) : j;
+        b_s[js] = j < nvalid ? b * kLog2e : -INFINITY;
+    }
+    // Row duals of the previous sweep (the fast path's exponent reference and
+    // the momentum term), read once here instead of on every batch's critical path.
+    for (int i = tid; i < row_end - row_begin; i += THREADS) {
+        float a = p.a[row_begin + i];
+        if (p.a_off != nullptr) a += p.a_off[row_begin + i];
+        a_s[i] = a;
+    }
+    __syncthreads();
+    if (!OLD_COST) fill();
     // Stage s of batch bt is no longer read: refill it with batch bt + stages (thread 0).
     auto release = [&](int bt, int s) {
         if (tid == 0 && bt + p.stages < nbatch) {
@@ -1016,20 +1032,22 @@ __global__ void __launch_bounds__(THREADS, 1) row_sweep_kernel(const RowArgs p) 
 
 // Reduce the per-cluster column sums (FP64), write log(colsum), decide.
 // Block: 8 warps x 32 lanes, one column per lane; warps split the partial rows, up
-// to 12 loads in flight per lane (a chain of dependent loads was most of this
-// kernel: 9.1 us at n = 4096 on 293 partial rows with 4 columns per lane and 32
-// blocks).  One FP64 error sum and one maximum |column correction| per block go to
-// the solve state by atomics.
+// to 20 loads in flight per lane.  A chain of latencies (loads, FP64 sums, log, the
+// ticket): 9 us at n = 4096, during which the next sweep is launched, sets up its barriers
+// and fetches its first rows (programmatic launch): a sweep and its finalize take 36 us an
+// iteration there, 43 launched one after the other.
+// One FP64 error sum and one maximum |column correction| per block go to the solve state
+// by atomics.
 constexpr int kFinThreads = 256;
 constexpr int kFinCols = 32;
 
 __global__ void __launch_bounds__(kFinThreads) finalize_kernel(const float* partials, int nparts, long long n_pad,
                                                                int n, float* logcs, SolveState* st) {
     constexpr int kWarps = kFinThreads / 32;
-    constexpr int U = 12;
+    constexpr int U = 20;
     __shared__ double part[kWarps][kFinCols];
-    __shared__ double red[32];
-    __shared__ float red_corr[kWarps];
+    launch_dependents();
+    wait_for_previous();
     if (*reinterpret_cast<volatile int*>(&st->done)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int j = blockIdx.x * kFinCols + lane;
@@ -1040,7 +1058,7 @@ __global__ void __launch_bounds__(kFinThreads) finalize_kernel(const float* part
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int c = c0 + u * kWarps;
-                v[u] = c < nparts ? partials[static_cast<size_t>(c) * n_pad + j] : 0.f;
+                v[u] = partials[static_cast<size_t>(min(c, nparts - 1)) * n_pad + j];
             }
 #pragma unroll
             for (int u = 0; u < U; ++u)
@@ -1049,9 +1067,10 @@ __global__ void __launch_bounds__(kFinThreads) finalize_kernel(const float* part
     }
     part[warp][lane] = cs;
     __syncthreads();
+    if (warp != 0) return;
     double err = 0.0;
     float corr = 0.f;
-    if (warp == 0 && j < n) {
+    if (j < n) {
         double tot = 0.0;
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) tot += part[w][lane];
@@ -1060,13 +1079,10 @@ __global__ void __launch_bounds__(kFinThreads) finalize_kernel(const float* part
         logcs[j] = lg;
         corr = fabsf(lg);
     }
-    corr = warp_max(corr);
-    if (lane == 0) red_corr[warp] = corr;
-    err = block_sum(err, red);  // contains __syncthreads: red_corr is complete
-    if (threadIdx.x == 0) {
-        float bc = 0.f;
-        for (int w = 0; w < kFinThreads / 32; ++w) bc = fmaxf(bc, red_corr[w]);
-        if (bc > 0.f) atomicMax(reinterpret_cast<unsigned int*>(&st->max_corr), __float_as_uint(bc));
+    corr = warp_max_positive(corr);
+    err = warp_sum(err);
+    if (lane == 0) {
+        if (corr > 0.f) atomicMax(reinterpret_cast<unsigned int*>(&st->max_corr), __float_as_uint(corr));
         atomicAdd(&st->err_accum, err);
         __threadfence();
         const unsigned prev = atomicAdd(&st->ticket, 1u);
@@ -1639,7 +1655,7 @@ int partial_rows_bound(int64_t n) {
 fugal_status launch_sweep(const SweepPlan& pl, KernelFn fn, const SweepArgs& args, cudaStream_t stream,
                           int family) {
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     cfg.gridDim = dim3(pl.clusters * pl.cluster, 1, 1);
     cfg.blockDim = dim3(pl.threads, 1, 1);
     cfg.dynamicSmemBytes = pl.smem;
@@ -1648,8 +1664,10 @@ fugal_status launch_sweep(const SweepPlan& pl, KernelFn fn, const SweepArgs& arg
     attr[0].val.clusterDim.x = pl.cluster;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     LaunchScope scope(family, stream);
     return cuda_check(cudaLaunchKernelEx(&cfg, fn, args), "sinkhorn: sweep launch");
 }
@@ -1854,9 +1872,18 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
     const int fin_grid = static_cast<int>((n + kFinCols - 1) / kFinCols);
     auto finalize = [&](int nparts) -> fugal_status {
         LaunchScope scope(FUGAL_KERNEL_FINALIZE, stream);
-        finalize_kernel<<<fin_grid, kFinThreads, 0, stream>>>(w.partials, nparts, w.n_pad, static_cast<int>(n),
-                                                              w.logcs, w.st);
-        return launch_check("sinkhorn: finalize");
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        cfg.gridDim = dim3(fin_grid, 1, 1);
+        cfg.blockDim = dim3(kFinThreads, 1, 1);
+        cfg.stream = stream;
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        return cuda_check(cudaLaunchKernelEx(&cfg, finalize_kernel, static_cast<const float*>(w.partials), nparts,
+                                             static_cast<long long>(w.n_pad), static_cast<int>(n), w.logcs, w.st),
+                          "sinkhorn: finalize");
     };
 
     // ---- main phase: sweeps t = 0 .. max_iterations-1, polled at evaluation points
