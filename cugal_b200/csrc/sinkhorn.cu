@@ -1470,9 +1470,9 @@ fugal_status make_plan(int64_t n, int dt, int kind, SweepPlan& pl, bool query_oc
     return fail(FUGAL_UNSUPPORTED, "sinkhorn: could not fit the row-dual staging for n = %lld", (long long)n);
 }
 
-// Row-owned 16-bit sweep plan (row_sweep_kernel): used for 16-bit sweeps when
-// the padded row fits 32768 columns; FUGAL_ROW_SWEEP=0 selects the cluster
-// kernel instead.
+// Row-owned 16-bit sweep plan (row_sweep_kernel): 16-bit sweeps of rows wider than the
+// persistent kernel takes (24576 columns; 469 against 454 us at 32768) up to 65536 columns;
+// FUGAL_ROW_SWEEP=0 selects the cluster kernel instead.
 struct RowPlan {
     bool use = false;
     bool bt = true;
@@ -1491,25 +1491,23 @@ struct RowPlan {
 using RowKernelFn = void (*)(const RowArgs);
 
 template <typename T, bool BT, int POLY>
-RowKernelFn row_kernel_typed(int ept, int cl) {
+RowKernelFn row_kernel_typed(int cl) {
     if (cl == 2) return row_sweep_kernel<T, 64, 512, BT, POLY, (BT ? 2 : 1)>;
     return row_sweep_kernel<T, 64, 512, BT, POLY, 1>;
 }
 
 template <typename T>
-RowKernelFn row_kernel_dt(int ept, bool bt, int poly, int cl) {
-    if (!bt) return row_kernel_typed<T, false, 0>(ept, 1);
+RowKernelFn row_kernel_dt(bool bt, int poly, int cl) {
+    if (!bt) return row_kernel_typed<T, false, 0>(1);
     switch (poly) {
-        case 4: return row_kernel_typed<T, true, 4>(ept, cl);
-        case 8: return row_kernel_typed<T, true, 8>(ept, cl);
-        default: return row_kernel_typed<T, true, 0>(ept, cl);
+        case 4: return row_kernel_typed<T, true, 4>(cl);
+        case 8: return row_kernel_typed<T, true, 8>(cl);
+        default: return row_kernel_typed<T, true, 0>(cl);
     }
 }
 
-RowKernelFn row_kernel_for(int dt, int ept, int threads, bool bt, int poly, int cl) {
-    (void)threads;
-    return dt == FUGAL_BF16 ? row_kernel_dt<__nv_bfloat16>(ept, bt, poly, cl)
-                            : row_kernel_dt<__half>(ept, bt, poly, cl);
+RowKernelFn row_kernel_for(int dt, bool bt, int poly, int cl) {
+    return dt == FUGAL_BF16 ? row_kernel_dt<__nv_bfloat16>(bt, poly, cl) : row_kernel_dt<__half>(bt, poly, cl);
 }
 
 // Share of the row sweep's fast-path exponentials evaluated on the FMA pipe:
@@ -1570,7 +1568,7 @@ fugal_status make_row_plan(int64_t n, int dt, int64_t n_pad, RowPlan& rp, bool s
     if (rp.stages < 2) return FUGAL_OK;
     rp.smem = fixed + rp.stages * stage_bytes;
     int groups = static_cast<int>(std::min<int64_t>(sm_count() / rp.cl, n));
-    RowKernelFn fn = row_kernel_for(dt, rp.ept, rp.threads, rp.bt, rp.poly, rp.cl);
+    RowKernelFn fn = row_kernel_for(dt, rp.bt, rp.poly, rp.cl);
     if (set_attributes) {
         FUGAL_TRY(cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rp.smem),
                              "sinkhorn: row sweep shared memory"));
@@ -1961,8 +1959,7 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
             ra.fault_row = test_fault_row();
             {
                 LaunchScope scope(FUGAL_KERNEL_SWEEP, stream);
-                RowKernelFn fn = row_kernel_for(p.stream_dtype, rowplan.ept, rowplan.threads, rowplan.bt,
-                                                rowplan.poly, rowplan.cl);
+                RowKernelFn fn = row_kernel_for(p.stream_dtype, rowplan.bt, rowplan.poly, rowplan.cl);
                 if (rowplan.cl == 1) {
                     fn<<<rowplan.ctas, rowplan.threads, rowplan.smem, stream>>>(ra);
                     status = launch_check("sinkhorn: row sweep");
