@@ -973,8 +973,11 @@ __global__ void __launch_bounds__(THREADS, 1) row_sweep_kernel(const RowArgs p) 
         }
         if (tid == 0 && rank == 0) p.a[row] = anew;
         // column sums of the row-normalised plan, accumulated in TMEM (one 16-column
-        // chunk per load; batching two chunks per wait measured slower)
+        // chunk per load; batching two chunks per wait measured slower).  A load follows
+        // the stores of the row before only through this wait; they have the row's reduction
+        // behind them by now.
         const float2 w2 = make_float2(wr, wr);
+        tmem_wait_st();
 #pragma unroll
         for (int k = 0; k < EPT / 16; ++k) {
             float acc[16];

@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
             // a resident row is waited for once per launch
             bool ok = (p.resident && sw > 0) ||
                       mbar_wait<true>(&full[s], p.resident ? 0u : ph, &p.st->status, p.suspend_ns, p.wait_limit_ns);
+            cols.settle();
             auto release = [&]() {
                 // (every thread of the stream has read the stage before the barrier just passed)
                 if (gt == 0 && ubase + r + NST < units) {
@@ -393,6 +394,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
         {
             float* prow = p.partials + static_cast<size_t>(blockIdx.x) * p.n_pad;
             float* mine = DUMP ? dump + static_cast<size_t>(g) * COVER : prow;
+            cols.settle();
 #pragma unroll
             for (int c = 0; c < NCH; ++c) {
                 float acc[16];

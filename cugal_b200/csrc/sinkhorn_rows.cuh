@@ -87,6 +87,7 @@ struct ColumnState<EPT, true> {
         }
     }
     FUGAL_DEVICE void ready() {}
+    FUGAL_DEVICE void settle() {}
     FUGAL_DEVICE void duals(int c, float2* b) const {
 #pragma unroll
         for (int q = 0; q < 8; ++q) b[q] = dual[8 * c + q];
@@ -122,6 +123,10 @@ struct ColumnState<EPT, false> {
         tmem_st16(tsum + 16 * c, z);
     }
     FUGAL_DEVICE void ready() { tmem_wait_st(); }
+    // Tensor memory orders a load after a store of the same thread only through a wait: called
+    // once per row before its sums are added to and once before they are read out, when the
+    // stores of the row before have a reduction and a barrier behind them.
+    FUGAL_DEVICE void settle() { tmem_wait_st(); }
     FUGAL_DEVICE void duals(int c, float2* b) const {
         float v[16];
         tmem_ld16(tdual + 16 * c, v);

@@ -436,6 +436,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
             const float* stage = reinterpret_cast<const float*>(ring) + static_cast<size_t>(s) * COVER;
             const bool ok = (p.resident && t > 0) ||
                             mbar_wait<true>(&full[s], p.resident ? 0u : ph, p.status, p.suspend_ns);
+            cols.settle();
             float2 s2 = make_float2(0.f, 0.f), t2 = make_float2(0.f, 0.f);
 #pragma unroll
             for (int c = 0; c < NCH; ++c) {
@@ -494,6 +495,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
         {
             float* prow = p.partials + static_cast<size_t>(blockIdx.x) * p.n_pad;
             float* to = DUMP ? dump + static_cast<size_t>(g) * COVER : prow;
+            cols.settle();
 #pragma unroll
             for (int c = 0; c < NCH; ++c) {
                 float acc[16];
