@@ -573,7 +573,7 @@ extern "C" fugal_status fugal_sinkhorn_adjoint_solve(const float* P, int64_t ldp
     void (*fn)(CgArgs) = vec ? cg_kernel<true> : cg_kernel<false>;
     const size_t span = kCgThreads * 4;
     const size_t smem = (static_cast<size_t>(n) + span - 1) / span * span * 8;
-    FUGAL_TRY(cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), who));
+    FUGAL_TRY(allow_dynamic_smem(fn, smem, who));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cfg.gridDim = dim3(ctas, 1, 1);

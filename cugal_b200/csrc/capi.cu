@@ -4,7 +4,9 @@
 
 #include <atomic>
 #include <cstdio>
+#include <map>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "fugal_host.h"
@@ -112,6 +114,28 @@ int sm_count() {
         cached[dev] = v > 0 ? v : 148;
     }
     return cached[dev];
+}
+
+fugal_status allow_dynamic_smem(const void* fn, size_t bytes, const char* what) {
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, int> limits;  // (function, device): bytes
+    int dev = 0, limit = 0;
+    FUGAL_TRY(cuda_check(cudaGetDevice(&dev), what));
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        const auto known = limits.find({fn, dev});
+        if (known != limits.end()) {
+            limit = known->second;
+        } else {
+            cudaFuncAttributes a;
+            FUGAL_TRY(cuda_check(cudaFuncGetAttributes(&a, fn), what));
+            FUGAL_TRY(cuda_check(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), what));
+            limit -= static_cast<int>(a.sharedSizeBytes);
+            limits[{fn, dev}] = limit;
+        }
+    }
+    if (limit < 0 || bytes > static_cast<size_t>(limit)) return cuda_check(cudaErrorInvalidValue, what);
+    return cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, limit), what);
 }
 
 }  // namespace fugal

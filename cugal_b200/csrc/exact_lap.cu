@@ -537,8 +537,7 @@ extern "C" fugal_status fugal_exact_lap(const float* P, int64_t ldp, int64_t n, 
         if (n <= kOwnedMaxN) {
             OwnedFn fn = owned_kernel(n);
             const size_t smem = owned_smem(n);
-            FUGAL_TRY(cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                                 "fugal_exact_lap: shared memory"));
+            FUGAL_TRY(allow_dynamic_smem(fn, smem, "fugal_exact_lap: shared memory"));
             fn<<<1, kExactThreads, smem, stream>>>(P, ldp, nn, maximize ? 1 : 0, max_steps, w, cols, steps, status_out);
         } else {
             exact_lap_kernel<<<1, kExactThreads, 0, stream>>>(P, ldp, nn, maximize ? 1 : 0, max_steps, w, cols, steps,

@@ -42,6 +42,16 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // Number of SMs of the current device (cached per device).
 int sm_count();
 
+// Allow `fn` the largest dynamic shared memory the device gives a CTA next to its static arrays
+// (an error if `bytes` is more).  The limit belongs to the function, not to a launch, and launches
+// of several host threads may lie between a call and its own launch: a limit of the call's own
+// size would take away what a larger one has asked for.
+fugal_status allow_dynamic_smem(const void* fn, size_t bytes, const char* what);
+template <typename... Args>
+fugal_status allow_dynamic_smem(void (*fn)(Args...), size_t bytes, const char* what) {
+    return allow_dynamic_smem(reinterpret_cast<const void*>(fn), bytes, what);
+}
+
 }  // namespace fugal
 
 #define FUGAL_TRY(expr)                              \

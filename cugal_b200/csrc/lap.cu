@@ -488,9 +488,7 @@ extern "C" fugal_status fugal_sampled_lap(float* P, int64_t ldp, int64_t n, cons
     if (ldp < n) return fail(FUGAL_BAD_SHAPE, "fugal_sampled_lap: ldp < n");
     const size_t nch = static_cast<size_t>((n + 31) / 32);
     const size_t smem = nch * (sizeof(double) + sizeof(unsigned));
-    FUGAL_TRY(cuda_check(cudaFuncSetAttribute(sampled_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              static_cast<int>(smem)),
-                         "fugal_sampled_lap: shared memory"));
+    FUGAL_TRY(allow_dynamic_smem(sampled_walk_kernel, smem, "fugal_sampled_lap: shared memory"));
     LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
     sampled_walk_kernel<<<1, kSampleThreads, smem, stream>>>(P, ldp, static_cast<int>(n),
                                                              reinterpret_cast<const long long*>(order), uniforms,
@@ -562,9 +560,7 @@ extern "C" fugal_status fugal_greedy_lap(float* P, int64_t ldp, int64_t n, int m
                    method == FUGAL_LAP_PARALLEL_GREEDY ? 1 : 0, reinterpret_cast<long long*>(columns_out), w.pos,
                    w.owner_pos};
         const size_t smem = walk_smem_bytes(n, K);
-        FUGAL_TRY(cuda_check(cudaFuncSetAttribute(walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  static_cast<int>(smem)),
-                             "fugal_greedy_lap: walk shared memory"));
+        FUGAL_TRY(allow_dynamic_smem(walk_kernel, smem, "fugal_greedy_lap: walk shared memory"));
         LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
         walk_kernel<<<1, kWalkThreads, smem, stream>>>(a);
         FUGAL_TRY(launch_check("fugal_greedy_lap: walk"));

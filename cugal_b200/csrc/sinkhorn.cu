@@ -1436,8 +1436,7 @@ fugal_status make_plan(int64_t n, int dt, int kind, SweepPlan& pl, bool query_oc
         pl.smem = fixed + stages * stage_bytes;
         int clusters = sms * 4;  // upper bound for workspace sizing
         if (query_occupancy) {
-            FUGAL_TRY(cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem),
-                                 "sinkhorn: set dynamic shared memory"));
+            FUGAL_TRY(allow_dynamic_smem(fn, pl.smem, "sinkhorn: set dynamic shared memory"));
             // all of the unified L1 / shared memory as shared memory, so two CTAs fit per SM
             FUGAL_TRY(cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
                                                       cudaSharedmemCarveoutMaxShared),
@@ -1573,8 +1572,7 @@ fugal_status make_row_plan(int64_t n, int dt, int64_t n_pad, RowPlan& rp, bool s
     int groups = static_cast<int>(std::min<int64_t>(sm_count() / rp.cl, n));
     RowKernelFn fn = row_kernel_for(dt, rp.bt, rp.poly, rp.cl);
     if (set_attributes) {
-        FUGAL_TRY(cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rp.smem),
-                             "sinkhorn: row sweep shared memory"));
+        FUGAL_TRY(allow_dynamic_smem(fn, rp.smem, "sinkhorn: row sweep shared memory"));
         if (rp.cl > 1) {
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute attr[1];

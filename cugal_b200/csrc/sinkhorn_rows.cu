@@ -592,8 +592,7 @@ fugal_status make_rows_plan(int64_t n, int dt, RowsPlan& pl, bool device) {
         cudaGetDevice(&dev);
         if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return FUGAL_OK;
         RowsFn fn = rows_fn(pl);
-        FUGAL_TRY(cuda_check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem),
-                             "sinkhorn rows: shared memory"));
+        FUGAL_TRY(allow_dynamic_smem(fn, pl.smem, "sinkhorn rows: shared memory"));
         FUGAL_TRY(cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, kRowsThreads, pl.smem),
                              "sinkhorn rows: occupancy"));
         if (blocks < 1) return FUGAL_OK;

@@ -632,7 +632,7 @@ StdRowsPlan std_rows_plan(int64_t n, int64_t ldk, const float* K) {
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return pl;
     StdRowsFn fn = std_rows_fn(pl);
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem) != cudaSuccess ||
+    if (allow_dynamic_smem(fn, pl.smem, "sinkhorn standard: shared memory") != FUGAL_OK ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, kRowsThreads, pl.smem) != cudaSuccess || blocks < 1) {
         (void)cudaGetLastError();
         return pl;

@@ -661,9 +661,7 @@ template <int R>
 fugal_status launch_transposed_rows(int64_t n, const int* rp, const int* col, const float* Q, int64_t ldq, float* outT,
                                     int64_t ldo, float sign, cudaStream_t stream) {
     const size_t smem = static_cast<size_t>(n) * R * sizeof(float);
-    FUGAL_TRY(cuda_check(cudaFuncSetAttribute(spmm_transposed_rows_kernel<R>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-                         "fugal_adjacency_matmul: shared memory"));
+    FUGAL_TRY(allow_dynamic_smem(spmm_transposed_rows_kernel<R>, smem, "fugal_adjacency_matmul: shared memory"));
     spmm_transposed_rows_kernel<R><<<static_cast<unsigned>((n + R - 1) / R), kTransposedThreads, smem, stream>>>(
         rp, col, Q, ldq, static_cast<int>(n), outT, ldo, sign);
     return launch_check("fugal_adjacency_matmul");
