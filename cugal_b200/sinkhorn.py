@@ -205,6 +205,8 @@ class SinkhornState:
         start = TimeStamp(config.device)
         n = self.n
         N.require_cuda(C, "C")
+        if C.device != self.U.device:  # the duals are handed over as pointers
+            raise RuntimeError(f"solve: C is on {C.device}, the state on {self.U.device}")
         reg = config.sinkhorn_regularization
         rows = C.dim() == 2 and C.stride(1) == 1 and C.stride(0) >= C.shape[1]
         if C.dtype == torch.float32 and rows and not (C.requires_grad and torch.is_grad_enabled()):

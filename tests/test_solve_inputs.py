@@ -1,0 +1,75 @@
+"""What ``SinkhornState.solve`` takes as a cost, on the CPU: the kernel that forms the absorbed cost is
+replaced by its arithmetic on the pointers that it is given, the solve itself by nothing."""
+
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from cugal_b200 import _native as N
+from cugal_b200 import sinkhorn
+from cugal_b200.config import Config, SinkhornMethod
+
+REG = 0.25  # a power of two: a division and a product with its reciprocal round alike
+
+
+def _array(pointer, ctype, shape):
+    return np.ctypeslib.as_array(ctypes.cast(pointer, ctypes.POINTER(ctype)), shape=shape)
+
+
+def _absorb(name, C, ldc, n, scale, U, V, K, ldk, cost, ld, stream):
+    assert name == "fugal_absorb_cost"
+    k = np.float32(scale) * _array(C, ctypes.c_float, (n, ldc))[:, :n]
+    if K is not None:
+        _array(K, ctypes.c_float, (n, ldk))[:, :n] = k
+    out = _array(cost, ctypes.c_float, (n, ld))
+    out[:, :n] = k.astype(np.float64) + _array(U, ctypes.c_double, (n, 1)) + _array(V, ctypes.c_double, (n,))
+    out[:, n:] = 0.0
+
+
+class _NoSolve:
+    def solve(self, *args):
+        pass
+
+
+@pytest.fixture
+def state(monkeypatch):
+    """A state of 5 nodes with its duals on the CPU, zero increments, and no kernels."""
+    n = 5
+    s = object.__new__(sinkhorn.SinkhornState)
+    s.n, s.method = n, SinkhornMethod.LOG
+    s.config = Config(device="cpu", dtype=torch.float32, sinkhorn_method=SinkhornMethod.LOG,
+                      sinkhorn_regularization=REG)
+    s.U = torch.linspace(-1, 1, n, dtype=torch.float64)
+    s.V = torch.linspace(3, -2, n, dtype=torch.float64)
+    s._solver, s._rec = _NoSolve(), torch.empty(0)
+    s._du, s._dv = torch.zeros(n), torch.zeros(n)
+    monkeypatch.setattr(N, "require_cuda", lambda *args: None)
+    monkeypatch.setattr(N, "stream_handle", lambda *args: 0)
+    monkeypatch.setattr(N, "call", _absorb)
+    return s
+
+
+def _expected(C, s):
+    K = -C / REG
+    return K, (K.double() + s.U[:, None] + s.V[None, :]).float().expand(s.n, s.n)
+
+
+def _check(s, C, K):
+    expected, cost = _expected(C, s)
+    assert K.dtype == torch.float32 and torch.equal(K.detach(), expected.detach().float())
+    assert torch.equal(s._cost32[:, :s.n], cost)
+
+
+def test_row_major_cost(state):
+    C = torch.rand(5, 5)
+    K, u, v = state.solve(C)
+    _check(state, C, K)
+
+
+def test_cost_on_another_device_is_refused(state, monkeypatch):
+    state.U = state.U.to("meta")
+    monkeypatch.setattr(N, "call", lambda *args: pytest.fail("a kernel was given another device's pointers"))
+    with pytest.raises(RuntimeError):
+        state.solve(torch.rand(5, 5))
