@@ -19,6 +19,7 @@ import ctypes
 
 import numpy as np
 import torch
+from torch.autograd import forward_ad
 
 from . import _native as N
 from .config import Config, SinkhornMethod
@@ -209,7 +210,9 @@ class SinkhornState:
             raise RuntimeError(f"solve: C is on {C.device}, the state on {self.U.device}")
         reg = config.sinkhorn_regularization
         rows = C.dim() == 2 and C.stride(1) == 1 and C.stride(0) >= C.shape[1]
-        if C.dtype == torch.float32 and rows and not (C.requires_grad and torch.is_grad_enabled()):
+        # the returned K = -C / reg carries the derivatives of C: then torch forms it
+        derived = (C.requires_grad and torch.is_grad_enabled()) or forward_ad.unpack_dual(C).tangent is not None
+        if C.dtype == torch.float32 and rows and not derived:
             K = torch.empty((n, n), dtype=torch.float32, device=C.device)
             # -C / reg as torch divides a float32 tensor by a number: times the FP32 reciprocal
             src, scale, K_out = C, -float(np.float32(1.0) / np.float32(reg)), K

@@ -6,6 +6,7 @@ import ctypes
 import numpy as np
 import pytest
 import torch
+from torch.autograd import forward_ad
 
 from cugal_b200 import _native as N
 from cugal_b200 import sinkhorn
@@ -73,3 +74,22 @@ def test_cost_on_another_device_is_refused(state, monkeypatch):
     monkeypatch.setattr(N, "call", lambda *args: pytest.fail("a kernel was given another device's pointers"))
     with pytest.raises(RuntimeError):
         state.solve(torch.rand(5, 5))
+
+
+def test_returned_kernel_keeps_the_tangent_of_the_cost(state):
+    C, dC = torch.rand(5, 5), torch.rand(5, 5)
+    with forward_ad.dual_level():
+        K, _, _ = state.solve(forward_ad.make_dual(C, dC))
+        tangent = forward_ad.unpack_dual(K).tangent
+        assert tangent is not None and torch.equal(tangent, -dC / REG)
+    _check(state, C, K)
+
+
+def test_returned_kernel_keeps_the_graph_of_the_cost(state):
+    C = torch.rand(5, 5, requires_grad=True)
+    K, _, _ = state.solve(C)
+    _check(state, C, K)
+    (g,) = torch.autograd.grad(K.sum(), C)
+    assert torch.equal(g, torch.full((5, 5), -1 / REG))
+    with torch.no_grad():
+        assert not state.solve(C)[0].requires_grad
