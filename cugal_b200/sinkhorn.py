@@ -209,7 +209,7 @@ class SinkhornState:
         if C.device != self.U.device:  # the duals are handed over as pointers
             raise RuntimeError(f"solve: C is on {C.device}, the state on {self.U.device}")
         reg = config.sinkhorn_regularization
-        rows = C.dim() == 2 and C.stride(1) == 1 and C.stride(0) >= C.shape[1]
+        rows = C.shape == (n, n) and C.stride(1) == 1 and C.stride(0) >= n
         # the returned K = -C / reg carries the derivatives of C: then torch forms it
         derived = (C.requires_grad and torch.is_grad_enabled()) or forward_ad.unpack_dual(C).tangent is not None
         if C.dtype == torch.float32 and rows and not derived:
@@ -218,9 +218,9 @@ class SinkhornState:
             src, scale, K_out = C, -float(np.float32(1.0) / np.float32(reg)), K
         else:
             K = (-C / reg).to(torch.float32)
-            src, scale, K_out = K.detach().contiguous(), 1.0, None
-        if src.shape[0] != n or src.shape[1] != n:
-            raise ValueError(f"solve: C must be {n} x {n}")
+            # any shape that broadcasts to n x n (1 x n: one row for all; leading dimensions of 1)
+            src = K.detach().reshape(K.shape[-2:] if K.shape[:-2].numel() == 1 else K.shape)
+            src, scale, K_out = src.expand(n, n).contiguous(), 1.0, None
         cost32 = torch.empty((n, padded_ld(n)), dtype=torch.float32, device=C.device)
         N.call("fugal_absorb_cost", src.data_ptr(), N.matrix_ld(src, "C"), n, scale, self.U.data_ptr(),
                self.V.data_ptr(), N.ptr(K_out), n, cost32.data_ptr(), cost32.stride(0), N.stream_handle(C.device))

@@ -54,7 +54,9 @@ def state(monkeypatch):
 
 def _expected(C, s):
     K = -C / REG
-    return K, (K.double() + s.U[:, None] + s.V[None, :]).float().expand(s.n, s.n)
+    cost = torch.zeros(s.n, s.n)
+    cost[:] = (K.double() + s.U[:, None] + s.V[None, :]).float().detach()
+    return K, cost
 
 
 def _check(s, C, K):
@@ -93,3 +95,29 @@ def test_returned_kernel_keeps_the_graph_of_the_cost(state):
     assert torch.equal(g, torch.full((5, 5), -1 / REG))
     with torch.no_grad():
         assert not state.solve(C)[0].requires_grad
+
+
+@pytest.mark.parametrize("shape", [(5, 5), (1, 5), (5, 1), (5,), (1,), (), (1, 5, 5), (1, 1, 5, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_costs_that_broadcast(state, shape, dtype):
+    """What K + u_i + v_j broadcasts to n x n is a cost, as in the reference's arithmetic; K keeps its shape."""
+    C = torch.rand(shape).to(dtype)
+    K, _, _ = state.solve(C)
+    assert K.shape == torch.Size(shape)
+    _check(state, C.float(), K)
+
+
+@pytest.mark.parametrize("shape", [(4, 4), (5, 4), (2, 5, 5), (5, 5, 1), (6,)])
+def test_other_shapes_are_refused(state, shape, monkeypatch):
+    monkeypatch.setattr(N, "call", lambda *args: pytest.fail("a kernel was given a cost of another size"))
+    with pytest.raises(RuntimeError):
+        state.solve(torch.rand(shape))
+
+
+@pytest.mark.parametrize("order", ["transposed", "columns", "steps", "repeated"])
+def test_strides(state, order):
+    base = torch.rand(10, 10)
+    C = {"transposed": base[:5, :5].t(), "columns": base[:5, 2:7], "steps": base[::2, ::2],
+         "repeated": base[0, :5].expand(5, 5)}[order]
+    K, _, _ = state.solve(C)
+    _check(state, C, K)
