@@ -212,7 +212,8 @@ class SinkhornState:
         rows = C.shape == (n, n) and C.stride(1) == 1 and C.stride(0) >= n
         # the returned K = -C / reg carries the derivatives of C: then torch forms it
         derived = (C.requires_grad and torch.is_grad_enabled()) or forward_ad.unpack_dual(C).tangent is not None
-        if C.dtype == torch.float32 and rows and not derived:
+        plain = type(C) in (torch.Tensor, torch.nn.Parameter) and not C.is_neg() and isinstance(reg, (int, float))
+        if C.dtype == torch.float32 and rows and plain and not derived:
             K = torch.empty((n, n), dtype=torch.float32, device=C.device)
             # -C / reg as torch divides a float32 tensor by a number: times the FP32 reciprocal
             src, scale, K_out = C, -float(np.float32(1.0) / np.float32(reg)), K

@@ -2,6 +2,7 @@
 replaced by its arithmetic on the pointers that it is given, the solve itself by nothing."""
 
 import ctypes
+import dataclasses
 
 import numpy as np
 import pytest
@@ -121,3 +122,20 @@ def test_strides(state, order):
          "repeated": base[0, :5].expand(5, 5)}[order]
     K, _, _ = state.solve(C)
     _check(state, C, K)
+
+
+def test_negated_view(state):
+    C = torch._neg_view(torch.rand(5, 5))
+    K, _, _ = state.solve(C)
+    _check(state, C.resolve_neg(), K)
+
+
+def test_subclass_and_regularization_of_another_type(state):
+    class Cost(torch.Tensor):
+        pass
+    C = torch.rand(5, 5).as_subclass(Cost)
+    assert type(state.solve(C)[0]) is Cost
+    C = torch.rand(5, 5)
+    for reg in (torch.tensor(REG), np.float32(REG), torch.full((5, 1), REG)):
+        K, _, _ = state.solve(C, dataclasses.replace(state.config, sinkhorn_regularization=reg))
+        _check(state, C, K)
