@@ -190,7 +190,7 @@ class SinkhornPlanUnrolled(torch.autograd.Function):
         dev = K.device
         stream = N.stream_handle(dev)
         mv = _Matvec(n, dev)
-        ws = mv.ws
+        ws = torch.empty(N.workspace_size("fugal_sinkhorn_unrolled_workspace_size", n), dtype=torch.uint8, device=dev)
         ones = torch.ones(n, dtype=torch.float64, device=dev)
         G = G.to(torch.float32).contiguous()
         gK = (G * P).contiguous()

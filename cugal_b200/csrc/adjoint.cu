@@ -112,22 +112,22 @@ __global__ void adjoint_kernel(const float* __restrict__ P, long long ldp, const
 //     gK_ij -= g_i E_ij,   g_other_j -= sum_i g_i E_ij        (column partials)
 // axis 0 (column half, out_j = -LSE_i(K_ij + other_i)): E_ij = exp(K_ij + other_i + out_j),
 //     gK_ij -= g_j E_ij,   g_other_i -= sum_j g_j E_ij        (row partials)
-// A block covers kUnRows rows x 1024 columns (4 consecutive columns per thread): at
-// n = 1024 128 blocks, where blocks of 64 rows made 16 (89 us a half step, bound by
-// their FP64 exponentials; 10 us here).
-constexpr int kUnRows = 8;
+// A block covers ROWS rows x 1024 columns (4 consecutive columns per thread), bound by the
+// chain of its FP64 exponentials and gK updates where blocks are few: at n = 1024 128 blocks of
+// 8 rows, 16 of 64 (see unrolled_rows for the times).
+template <int ROWS>
 __global__ void __launch_bounds__(kMvThreads) unrolled_step_kernel(const float* __restrict__ K, long long ldk, int n,
                                                                    const float* __restrict__ out_dual,
                                                                    const float* __restrict__ other_dual,
                                                                    const double* __restrict__ g, int axis,
                                                                    float* __restrict__ gK, long long ldg,
                                                                    double* row_part, double* col_part) {
-    __shared__ double red[kMvThreads / 32][kUnRows];
+    __shared__ double red[kMvThreads / 32][ROWS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int r0 = blockIdx.y * kUnRows;
+    const int r0 = blockIdx.y * ROWS;
     const int j0 = blockIdx.x * kMvCols + threadIdx.x * 4;
     double cs[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int r = 0; r < kUnRows; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
         const int i = r0 + r;
         double rs = 0.0;
         if (i < n) {
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kMvThreads) unrolled_step_kernel(const float* 
     }
     if (axis == 0) {
         __syncthreads();
-        if (threadIdx.x < kUnRows) {
+        if (threadIdx.x < ROWS) {
             const int i = r0 + threadIdx.x;
             double s = 0.0;
 #pragma unroll
@@ -464,13 +464,29 @@ extern "C" fugal_status fugal_sinkhorn_plan(const float* cost32, int64_t ld32, i
     return launch_check("fugal_sinkhorn_plan");
 }
 
+namespace {
+// Row partials of every column block and column partials of every row block of `rows` rows.
+size_t partials_bytes(int64_t n, int rows) {
+    const int64_t cb = (n + kMvCols - 1) / kMvCols, rb = (n + rows - 1) / rows;
+    return static_cast<size_t>((cb + rb) * n) * 8 + 256;
+}
+
+// Rows of an unrolled step's block: the fewest of 8, 16, 32, 64 that leave at most 512 partial
+// rows.  Small n needs the blocks, large n fewer partials to write and read (and to hold: n^2
+// bytes with blocks of 8).  A row and a column half step together, us: n = 1024 41 with 8, 191
+// with 64; 4096 163, 273; 8192 504 with 16, 537 with 8, 653 with 64; 16384 1942 with 32, 1970
+// with 8, 1992 with 64.
+int unrolled_rows(int64_t n) {
+    int rows = 8;
+    while (rows < kMvRows && n > 512 * rows) rows *= 2;
+    return rows;
+}
+}  // namespace
+
 extern "C" fugal_status fugal_plan_matvec_workspace_size(int64_t n, size_t* bytes) {
     if (bytes == nullptr) return fail(FUGAL_BAD_ARGUMENT, "fugal_plan_matvec_workspace_size: null output");
     if (n <= 0 || n > (1ll << 30)) return fail(FUGAL_BAD_SHAPE, "fugal_plan_matvec_workspace_size: bad n");
-    // row partials of every column block, column partials of every row block (the
-    // unrolled step's blocks are the smaller ones)
-    const int64_t cb = (n + kMvCols - 1) / kMvCols, rb = (n + kUnRows - 1) / kUnRows;
-    *bytes = static_cast<size_t>((cb + rb) * n) * 8 + 256;
+    *bytes = partials_bytes(n, kMvRows);
     return FUGAL_OK;
 }
 
@@ -588,6 +604,13 @@ extern "C" fugal_status fugal_sinkhorn_adjoint_solve(const float* P, int64_t ldp
     return cuda_check(cudaLaunchKernelEx(&cfg, fn, args), who);
 }
 
+extern "C" fugal_status fugal_sinkhorn_unrolled_workspace_size(int64_t n, size_t* bytes) {
+    if (bytes == nullptr) return fail(FUGAL_BAD_ARGUMENT, "fugal_sinkhorn_unrolled_workspace_size: null output");
+    if (n <= 0 || n > (1ll << 30)) return fail(FUGAL_BAD_SHAPE, "fugal_sinkhorn_unrolled_workspace_size: bad n");
+    *bytes = partials_bytes(n, unrolled_rows(n));
+    return FUGAL_OK;
+}
+
 extern "C" fugal_status fugal_sinkhorn_unrolled_step_backward(const float* K, int64_t ldk, int64_t n,
                                                               const float* out_dual, const float* other_dual,
                                                               const double* g, int axis, float* gK, int64_t ldg,
@@ -604,13 +627,19 @@ extern "C" fugal_status fugal_sinkhorn_unrolled_step_backward(const float* K, in
     if (workspace_bytes < need)
         return fail(FUGAL_WORKSPACE_TOO_SMALL, "fugal_sinkhorn_unrolled_step_backward: workspace too small");
     const int nn = static_cast<int>(n);
-    const int cb = static_cast<int>((n + kMvCols - 1) / kMvCols), rb = static_cast<int>((n + kUnRows - 1) / kUnRows);
+    int rows = unrolled_rows(n);  // larger blocks where the workspace holds fewer partials
+    while (rows < kMvRows && partials_bytes(n, rows) > workspace_bytes) rows *= 2;
+    const int cb = static_cast<int>((n + kMvCols - 1) / kMvCols), rb = static_cast<int>((n + rows - 1) / rows);
     double* row_part = static_cast<double*>(workspace);
     double* col_part = row_part + static_cast<size_t>(cb) * n;
     {
         LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-        unrolled_step_kernel<<<dim3(cb, rb), kMvThreads, 0, stream>>>(K, ldk, nn, out_dual, other_dual, g, axis, gK,
-                                                                      ldg, row_part, col_part);
+        auto kernel = rows == 8    ? unrolled_step_kernel<8>
+                      : rows == 16 ? unrolled_step_kernel<16>
+                      : rows == 32 ? unrolled_step_kernel<32>
+                                   : unrolled_step_kernel<kMvRows>;
+        kernel<<<dim3(cb, rb), kMvThreads, 0, stream>>>(K, ldk, nn, out_dual, other_dual, g, axis, gK, ldg, row_part,
+                                                        col_part);
         FUGAL_TRY(launch_check("fugal_sinkhorn_unrolled_step_backward"));
     }
     {

@@ -241,7 +241,9 @@ fugal_status fugal_sinkhorn_adjoint_solve(const float* P, int64_t ldp, int64_t n
  * (row update); axis 0: out = -LSE_i(K_ij + other_i) (column update).  With
  * E = exp(K + other + out) in that orientation and g = dL/d(out) (FP64):
  * gK -= g o E (FP32, in place) and g_other -= the reduction of g o E over the
- * LSE axis (FP64, accumulated).  Workspace as fugal_plan_matvec_workspace_size. */
+ * LSE axis (FP64, accumulated).  Workspace: at least fugal_plan_matvec_workspace_size;
+ * fugal_sinkhorn_unrolled_workspace_size where the step is to run at its fastest. */
+fugal_status fugal_sinkhorn_unrolled_workspace_size(int64_t n, size_t* bytes);
 fugal_status fugal_sinkhorn_unrolled_step_backward(const float* K, int64_t ldk, int64_t n, const float* out_dual,
                                                    const float* other_dual, const double* g, int axis, float* gK,
                                                    int64_t ldg, double* g_other, void* workspace,
