@@ -146,6 +146,13 @@ def sinkhorn_plan(C: torch.Tensor, config: Config, tol: float = 1e-7, max_iter: 
     return SinkhornPlan.apply(C, dataclasses.replace(config, stream_dtype=None), tol, max_iter)
 
 
+def _zero_vectors(count: int, n: int, ld: int, device, block: int = 32):
+    """``count`` FP64 zero vectors of n entries, ``block`` of them allocated (and cleared) at a time: a
+    step's gradient is not needed once the next one is there, however long the segment."""
+    for k in range(0, count, block):
+        yield from torch.zeros((min(block, count - k), ld), dtype=torch.float64, device=device)[:, :n]
+
+
 class SinkhornPlanUnrolled(torch.autograd.Function):
     """P after the reference's iteration (cugal/sinkhorn.py:108-115, no momentum)
     run from zero potentials, differentiated through the iterations: the duals
@@ -211,7 +218,7 @@ class SinkhornPlanUnrolled(torch.autograd.Function):
             states = [tuple(pair) for pair in duals]
             for mine, saved in zip(states[0], ctx.checkpoints[seg_start]):
                 mine.copy_(saved)
-            grads = iter(torch.zeros((2 * steps, ld), dtype=torch.float64, device=dev)[:, :n])
+            grads = _zero_vectors(2 * steps, n, ld, dev)
             for (u, _), (u_next, v_next) in zip(states, states[1:]):
                 N.call("fugal_sinkhorn_log_step", Kt.data_ptr(), n, n, n, u.data_ptr(), v_next.data_ptr(), 1.0, stream)
                 N.call("fugal_sinkhorn_log_step", K.data_ptr(), n, n, n, v_next.data_ptr(), u_next.data_ptr(), 1.0,

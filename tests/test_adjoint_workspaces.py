@@ -58,3 +58,15 @@ def test_unrolled_step_in_every_workspace(n):
             N.call("fugal_sinkhorn_unrolled_step_backward", K.data_ptr(), n, n, u.data_ptr(), v.data_ptr(),
                    grad.data_ptr(), axis, gK.data_ptr(), n, other.data_ptr(), ws.data_ptr(),
                    _partials(n, 64) - 1, N.stream_handle())
+
+
+def test_unrolled_gradient_vectors_come_in_blocks():
+    """A long segment between checkpoints holds a few gradient vectors at a time, each zero, its own, and on
+    a 256-byte boundary."""
+    from cugal_b200.autograd import _zero_vectors
+    k = -1
+    for k, g in enumerate(_zero_vectors(1000, 5, 64, "cpu")):
+        assert g.shape == (5,) and g.dtype == torch.float64 and not g.any() and g.storage_offset() * 8 % 256 == 0
+        g += 1.0
+        assert g.untyped_storage().nbytes() <= 32 * 64 * 8
+    assert k == 999
