@@ -1247,9 +1247,11 @@ __device__ int frame_snapshot(const FrameArgs& f, int t) {
     return ((t - f.warmup) / f.every) & 1;
 }
 
-// Move the final main-phase duals into the FP32 frame and open the polish phase.
+// Move the final main-phase duals into the FP32 frame and open the polish phase.  A solve in which a
+// wait ran out stays closed: the grid barrier of its sweeps may have been left half arrived at.
 __global__ void polish_begin_kernel(SolveState* st, float* a, float* b_buf, long long n_pad, float* logcs,
                                     const float* a_snap, const float* b_snap, int n, FrameArgs f) {
+    if (st->status != 0) return;
     const int fin = st->final_it;
     const int snap = frame_snapshot(f, fin);
     float* b = b_buf + (fin & 1) * n_pad;
