@@ -4,6 +4,7 @@
 
 #include <atomic>
 #include <cstdio>
+#include <cstdlib>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -114,6 +115,16 @@ int sm_count() {
         cached[dev] = v > 0 ? v : 148;
     }
     return cached[dev];
+}
+
+unsigned long long test_wait_limit_ns() {
+    const char* e = getenv("FUGAL_TEST_WAIT_LIMIT_NS");
+    return e != nullptr ? strtoull(e, nullptr, 10) : 0ull;
+}
+
+int test_fault_row(bool fp32) {
+    const char* e = getenv(fp32 ? "FUGAL_TEST_FAULT_ROW_FP32" : "FUGAL_TEST_FAULT_ROW");
+    return e != nullptr ? atoi(e) : -1;
 }
 
 fugal_status allow_dynamic_smem(const void* fn, size_t bytes, const char* what) {

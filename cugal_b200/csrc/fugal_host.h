@@ -42,6 +42,14 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // Number of SMs of the current device (cached per device).
 int sm_count();
 
+// Failure-detection test hooks, read from the environment at each solve:
+// FUGAL_TEST_WAIT_LIMIT_NS (limit of every bounded wait of a solve's kernels; unset: 0, the 2 s
+// default), and a local row of CTA 0 whose first copy is armed for 16 bytes that never arrive, so
+// that the waits on it run out (unset: -1, none): FUGAL_TEST_FAULT_ROW in sweeps over a 16-bit
+// cost, FUGAL_TEST_FAULT_ROW_FP32 in the persistent kernels over FP32 rows.
+unsigned long long test_wait_limit_ns();
+int test_fault_row(bool fp32);
+
 // Allow `fn` the largest dynamic shared memory the device gives a CTA next to its static arrays
 // (an error if `bytes` is more).  The limit belongs to the function, not to a launch, and launches
 // of several host threads may lie between a call and its own launch: a limit of the call's own

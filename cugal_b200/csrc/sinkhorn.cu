@@ -591,7 +591,7 @@ struct RowArgs {
     float* partials;     // [ctas][n_pad]
     long long n_pad;
     SolveState* st;
-    // Failure-detection test hooks (host environment, see make_row_args): the
+    // Failure-detection test hooks (host environment, see test_fault_row): the
     // limit of every bounded wait (0: the 2 s default), and a local row of CTA 0
     // whose first copy is armed for 16 bytes more than it delivers (-1: none),
     // so that the waits on it time out.
@@ -1523,19 +1523,6 @@ int row_poly() {
     return (v == 4 || v == 8) ? v : 0;
 }
 
-// Failure-detection test hooks of the row sweep, read from the environment at
-// each solve: FUGAL_TEST_WAIT_LIMIT_NS (limit of every bounded wait; unset: 2 s)
-// and FUGAL_TEST_FAULT_ROW (a local row of CTA 0 whose copy is armed for 16
-// bytes that never arrive, so the waits on it run out; unset: none).
-unsigned long long test_wait_limit_ns() {
-    const char* e = getenv("FUGAL_TEST_WAIT_LIMIT_NS");
-    return e != nullptr ? strtoull(e, nullptr, 10) : 0ull;
-}
-int test_fault_row() {
-    const char* e = getenv("FUGAL_TEST_FAULT_ROW");
-    return e != nullptr ? atoi(e) : -1;
-}
-
 // Column duals of the row sweep in TMEM (default) or shared memory
 // (FUGAL_ROW_DUALS_SMEM=1).
 bool row_duals_in_tmem() {
@@ -1867,7 +1854,7 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
         ra.n_pad = w.n_pad;
         ra.st = w.st;
         ra.wait_limit_ns = test_wait_limit_ns();
-        ra.fault_row = dt == FUGAL_F32 ? -1 : test_fault_row();
+        ra.fault_row = test_fault_row(dt == FUGAL_F32);
         return ra;
     };
     const int fin_grid = static_cast<int>((n + kFinCols - 1) / kFinCols);
@@ -1959,7 +1946,7 @@ extern "C" fugal_status fugal_sinkhorn_solve(const fugal_solve_params* prm, void
             ra.n_pad = w.n_pad;
             ra.st = w.st;
             ra.wait_limit_ns = test_wait_limit_ns();
-            ra.fault_row = test_fault_row();
+            ra.fault_row = test_fault_row(false);
             {
                 LaunchScope scope(FUGAL_KERNEL_SWEEP, stream);
                 RowKernelFn fn = row_kernel_for(p.stream_dtype, rowplan.bt, rowplan.poly, rowplan.cl);

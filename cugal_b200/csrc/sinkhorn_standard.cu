@@ -189,7 +189,13 @@ __global__ void __launch_bounds__(kStdThreads) std_rowdot_kernel(const float* __
     }
 }
 
-__global__ void std_record_kernel(const StdState* st, const unsigned* status, fugal_solve_record* rec) {
+// The record, if asked for.  A solve whose waits ran out has stopped anywhere in an iteration: its
+// u and v become NaN, so that it cannot pass for a result where no record is read.
+__global__ void std_end_kernel(const StdState* st, const unsigned* status, int n, float* u, float* v,
+                               fugal_solve_record* rec) {
+    if (*status != 0)
+        for (int j = threadIdx.x; j < n; j += blockDim.x) u[j] = v[j] = NAN;
+    if (rec == nullptr) return;
     if (threadIdx.x == 0) {
         rec->iteration_count = st->final_it + 1;
         rec->n_errors = min(st->n_err, FUGAL_MAX_RECORDED_ERRORS);
@@ -253,6 +259,8 @@ struct StdRowsArgs {
     StdState* st;
     unsigned* arrivals;
     int* status;
+    unsigned long long wait_limit_ns;  // test hooks (test_fault_row in fugal_host.h)
+    int fault_row;
 };
 
 // x^(1-w) y^w, the momentum update (w != 1)
@@ -358,9 +366,10 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
 
     // ring of whole rows: unit u (row u mod nrows) sits in stage u mod NST; see rows_kernel
     const uint32_t row_bytes = static_cast<uint32_t>(p.n_copy) * sizeof(float);
-    auto issue = [&](int row, int s, uint32_t phase) {
+    auto issue = [&](int row, int s, uint32_t phase, bool first) {
+        const uint32_t unmet = (first && blockIdx.x == 0 && row == p.fault_row) ? 16u : 0u;
         newest[s] = static_cast<int>(phase);
-        mbar_arrive_expect_tx(&full[s], row_bytes);
+        mbar_arrive_expect_tx(&full[s], row_bytes + unmet);
         bulk_load(ring + static_cast<size_t>(s) * COVER * sizeof(float),
                   p.K + static_cast<unsigned long long>(static_cast<unsigned>(row_begin + row)) *
                             static_cast<unsigned long long>(p.ldk),
@@ -369,7 +378,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
     if (tid == 0 && nrows > 0) {
         fence_proxy_async_smem();
         const int first = p.resident ? min(nrows, NST) : NST;
-        for (int k = 0; k < first; ++k) issue(k % nrows, k, 0u);
+        for (int k = 0; k < first; ++k) issue(k % nrows, k, 0u, k < nrows);
     }
     int sbase = 0;
     uint32_t phbase = 0u;
@@ -435,7 +444,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
             const int s = s_cur;
             const float* stage = reinterpret_cast<const float*>(ring) + static_cast<size_t>(s) * COVER;
             const bool ok = (p.resident && t > 0) ||
-                            mbar_wait<true>(&full[s], p.resident ? 0u : ph, p.status, p.suspend_ns);
+                            mbar_wait<true>(&full[s], p.resident ? 0u : ph, p.status, p.suspend_ns, p.wait_limit_ns);
             cols.settle();
             float2 s2 = make_float2(0.f, 0.f), t2 = make_float2(0.f, 0.f);
 #pragma unroll
@@ -469,7 +478,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
             if (gt == 0 && !p.resident) {
                 int row = r + ahead;
                 if (row >= nrows) row -= nrows;
-                issue(row, s, ph ^ 1u);
+                issue(row, s, ph ^ 1u, false);
             }
             if (t == 0) {
                 wp = u_s[r];
@@ -533,7 +542,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
             }
         }
         arrivals += gridDim.x;
-        if (!grid_barrier(p.arrivals, p.status, alive, arrivals, 0)) {
+        if (!grid_barrier(p.arrivals, p.status, alive, arrivals, p.wait_limit_ns)) {
             alive = false;
             break;
         }
@@ -547,7 +556,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
             if (tid < per && j < n) p.colsum[p.n_pad + j] = __ldcg(p.v + j);
         }
         arrivals += gridDim.x;
-        if (!grid_barrier(p.arrivals, p.status, true, arrivals, 0)) {
+        if (!grid_barrier(p.arrivals, p.status, true, arrivals, p.wait_limit_ns)) {
             alive = false;
             break;
         }
@@ -565,7 +574,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
     __syncthreads();
     if (tid == 0) {  // copies still in flight (bounded waits)
         for (int s = 0; s < NST; ++s)
-            if (newest[s] >= 0) mbar_wait<true>(&full[s], static_cast<uint32_t>(newest[s]), p.status, p.suspend_ns);
+            if (newest[s] >= 0)
+                mbar_wait<true>(&full[s], static_cast<uint32_t>(newest[s]), p.status, p.suspend_ns, p.wait_limit_ns);
     }
     if (blockIdx.x == 0) {
         if (tid == 0) {
@@ -708,6 +718,8 @@ extern "C" fugal_status fugal_sinkhorn_standard_solve(const float* K, int64_t ld
         ra.st = w.st;
         ra.arrivals = w.sync;
         ra.status = reinterpret_cast<int*>(w.sync + 1);
+        ra.wait_limit_ns = test_wait_limit_ns();
+        ra.fault_row = test_fault_row(true);
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         cfg.gridDim = dim3(plan.ctas, 1, 1);
@@ -722,12 +734,9 @@ extern "C" fugal_status fugal_sinkhorn_standard_solve(const float* K, int64_t ld
             LaunchScope scope(FUGAL_KERNEL_SWEEP_F32, stream);
             FUGAL_TRY(cuda_check(cudaLaunchKernelEx(&cfg, std_rows_fn(plan), ra), "sinkhorn standard: rows"));
         }
-        if (record != nullptr) {
-            LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-            std_record_kernel<<<1, 256, 0, stream>>>(w.st, w.sync + 1, static_cast<fugal_solve_record*>(record));
-            FUGAL_TRY(launch_check("sinkhorn standard: record"));
-        }
-        return FUGAL_OK;
+        LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
+        std_end_kernel<<<1, 256, 0, stream>>>(w.st, w.sync + 1, nn, u, v, static_cast<fugal_solve_record*>(record));
+        return launch_check("sinkhorn standard: record");
     }
     if (g_std_pinned == nullptr) {
         void* p = nullptr;
@@ -789,7 +798,7 @@ extern "C" fugal_status fugal_sinkhorn_standard_solve(const float* K, int64_t ld
     }
     if (status == FUGAL_OK && record != nullptr) {
         LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-        std_record_kernel<<<1, 256, 0, stream>>>(w.st, w.sync + 1, static_cast<fugal_solve_record*>(record));
+        std_end_kernel<<<1, 256, 0, stream>>>(w.st, w.sync + 1, nn, u, v, static_cast<fugal_solve_record*>(record));
         status = launch_check("sinkhorn standard: record");
     }
     cudaEventDestroy(ev[0]);

@@ -170,7 +170,8 @@ class SinkhornState:
         return self.V.to(self.config.dtype)
 
     def solve_standard(self, C: torch.Tensor, config: Config | None = None, profile: SinkhornProfile | None = None):
-        """``solve_standard`` (``cugal/sinkhorn.py:122-144``): returns (K, u, v), K = exp(-C/reg)."""
+        """``solve_standard`` (``cugal/sinkhorn.py:122-144``): returns (K, u, v), K = exp(-C/reg).
+        u and v are NaN after a solve whose bounded device waits ran out (with a profile it raises)."""
         config = config or self.config
         start = TimeStamp(config.device)
         N.require_cuda(C, "C")

@@ -196,7 +196,8 @@ fugal_status fugal_alignment_overlap(const int32_t* a_row_pointers, const int32_
  * eval_freq, 2 eval_freq, ... (stop below threshold, Lehmann momentum from
  * momentum_start, < 0 for none), at most max_iterations iterations.  u, v (FP32,
  * device) are read and written in place (warm start).  record: optional DEVICE
- * fugal_solve_record.  fugal_exp_scale writes out = exp(scale * C) (K from C with
+ * fugal_solve_record.  If a bounded wait of the device runs out, the record's status is
+ * FUGAL_DEVICE_TIMEOUT and u and v are NaN.  fugal_exp_scale writes out = exp(scale * C) (K from C with
  * scale = -1/reg); fugal_fw_update_standard is the update of cugal/pred.py:77-86
  * for this method: q = K v u, P += alpha (q - P), *gap = sum C (q - P) in FP64. */
 fugal_status fugal_sinkhorn_standard_workspace_size(int64_t n, size_t* bytes);
