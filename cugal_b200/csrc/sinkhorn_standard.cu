@@ -615,10 +615,12 @@ StdRowsFn std_rows_fn(const StdRowsPlan& pl) {
     }
 }
 
-// Rows are copied in 16-byte pieces: K's rows aligned, n rounded up to 4 within ldk.
-StdRowsPlan std_rows_plan(int64_t n, int64_t ldk, const float* K) {
+// Rows are copied in 16-byte pieces: K's rows aligned, n rounded up to 4 within ldk.  The vectors of
+// the workspace are read 16 bytes at a time; the launch form needs 8-byte boundaries only.
+StdRowsPlan std_rows_plan(int64_t n, int64_t ldk, const float* K, const void* workspace) {
     StdRowsPlan pl;
-    if (n > kStdRowsLimit || (ldk % 4) != 0 || ldk < (n + 3) / 4 * 4 || !aligned16(K)) return pl;
+    if (n > kStdRowsLimit || (ldk % 4) != 0 || ldk < (n + 3) / 4 * 4 || !aligned16(K) || !aligned16(workspace))
+        return pl;
     for (const auto& sh : kStdShapes)
         if (static_cast<int64_t>(kRowsThreads / sh[0]) * sh[1] >= n) {
             pl.streams = sh[0];
@@ -697,7 +699,7 @@ extern "C" fugal_status fugal_sinkhorn_standard_solve(const float* K, int64_t ld
         FUGAL_TRY(launch_check("sinkhorn standard: init"));
     }
     FUGAL_TRY(cuda_check(cudaMemsetAsync(w.sync, 0, 2 * sizeof(unsigned), stream), "sinkhorn standard: clear"));
-    const StdRowsPlan plan = std_rows_plan(n, ldk, K);
+    const StdRowsPlan plan = std_rows_plan(n, ldk, K, workspace);
     if (plan.use) {
         StdRowsArgs ra{};
         ra.K = K;
