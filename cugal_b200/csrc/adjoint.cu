@@ -236,6 +236,8 @@ struct CgArgs {
     double* dots;        // [2][CTAs]
     unsigned* arrivals;
     int* status;
+    unsigned long long wait_limit_ns;  // test hooks (test_wait_limit_ns, test_fault_barrier in fugal_host.h)
+    int fault_barrier;
 };
 
 // Sums of 8 values over the 32 lanes of a warp: on return lane l holds the sum of
@@ -296,16 +298,17 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_kernel(const __grid_constant
     const int own = max(0, min(n, o0 + p.own) - o0);
     const int span_n = (n + SPAN - 1) / SPAN * SPAN;
     unsigned arrivals = 0;
-    auto barrier = [&]() {
+    auto barrier = [&]() {  // false: a wait ran out; cg_end_kernel then leaves no result
         arrivals += gridDim.x;
-        return grid_barrier(p.arrivals, p.status, true, arrivals, 0);
+        bool ok = grid_barrier(p.arrivals, p.status, true, arrivals, p.wait_limit_ns);
+        if (p.fault_barrier > 0 && blockIdx.x == gridDim.x - 1 && arrivals == p.fault_barrier * gridDim.x) {
+            if (tid == 0) report_error(p.status, FUGAL_DEVICE_TIMEOUT);
+            ok = false;
+        }
+        return ok;
     };
     // column q of this thread in the span starting at c0
     auto column = [&](int c0, int q) { return VEC ? c0 + tid * 4 + q : c0 + q * kCgThreads + tid; };
-    auto give_up = [&]() {  // a wait ran out: no result
-        for (int k = tid; k < own; k += kCgThreads) p.alpha[o0 + k] = p.beta[o0 + k] = NAN;
-        if (blockIdx.x == 0 && tid == 0) p.info[2] = FUGAL_DEVICE_TIMEOUT;
-    };
 
     for (int j = tid; j < span_n; j += kCgThreads) y_s[j] = j < n ? p.b[j] : 0.0;
     double rr = 0.0;
@@ -317,7 +320,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_kernel(const __grid_constant
     }
     rr = block_sum(rr, scratch);
     if (tid == 0) p.dots[blockIdx.x] = rr;
-    if (!barrier()) return give_up();
+    if (!barrier()) return;
     double rs = grid_total(p.dots, scratch);
     const double norm = sqrt(rs);
     double rel = 0.0;
@@ -367,7 +370,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_kernel(const __grid_constant
                 for (int q = 0; q < 4; ++q)
                     if (column(c0, q) < n) cp[column(c0, q)] = cs[q];
             }
-            if (!barrier()) return give_up();
+            if (!barrier()) return;
             // ---- A p on the CTA's rows and columns, <p, A p>
             double dot = 0.0;
             for (int k = tid; k < own; k += kCgThreads) {
@@ -407,7 +410,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_kernel(const __grid_constant
             }
             dot = block_sum(dot, scratch);
             if (tid == 0) p.dots[gridDim.x + blockIdx.x] = dot;
-            if (!barrier()) return give_up();
+            if (!barrier()) return;
             const double step = rs / grid_total(p.dots + gridDim.x, scratch);
             // ---- solution and residual
             rr = 0.0;
@@ -422,7 +425,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_kernel(const __grid_constant
             }
             rr = block_sum(rr, scratch);
             if (tid == 0) p.dots[blockIdx.x] = rr;
-            if (!barrier()) return give_up();
+            if (!barrier()) return;
             const double rs_new = grid_total(p.dots, scratch);
             rel = sqrt(rs_new) / norm;
             if (rel < p.tol) break;
@@ -440,8 +443,20 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_kernel(const __grid_constant
     if (blockIdx.x == 0 && tid == 0) {
         p.info[0] = it;
         p.info[1] = rel;
-        p.info[2] = 0.0;
     }
+}
+
+// The status that all CTAs of the solve share: a CTA may pass the last barrier while another one's wait
+// on it runs out, so none of them can tell alone.
+__global__ void __launch_bounds__(256) cg_end_kernel(const int* status, int n, double* alpha, double* beta,
+                                                     double* info) {
+    const int s = *status;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k == 0) {
+        info[2] = s;
+        if (s != 0) info[0] = info[1] = NAN;
+    }
+    if (s != 0 && k < n) alpha[k] = beta[k] = NAN;
 }
 
 inline dim3 ew2d(int64_t n) {
@@ -583,6 +598,8 @@ extern "C" fugal_status fugal_sinkhorn_adjoint_solve(const float* P, int64_t ldp
     args.dots = reinterpret_cast<double*>(w + 256);
     args.r_cols = args.dots + 2 * cg_ctas(n);
     args.colpart = args.r_cols + n;
+    args.wait_limit_ns = test_wait_limit_ns();
+    args.fault_barrier = test_fault_barrier();
     FUGAL_TRY(cuda_check(cudaMemsetAsync(w, 0, 256, stream), who));
     // float4 rows: aligned, and whole quads (else one column per lane and load)
     const bool vec = (n % 4) == 0 && (ldp % 4) == 0 && aligned16(P);
@@ -600,8 +617,13 @@ extern "C" fugal_status fugal_sinkhorn_adjoint_solve(const float* P, int64_t ldp
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    {
+        LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
+        FUGAL_TRY(cuda_check(cudaLaunchKernelEx(&cfg, fn, args), who));
+    }
     LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-    return cuda_check(cudaLaunchKernelEx(&cfg, fn, args), who);
+    cg_end_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(args.status, args.n, alpha, beta, info);
+    return launch_check(who);
 }
 
 extern "C" fugal_status fugal_sinkhorn_unrolled_workspace_size(int64_t n, size_t* bytes) {

@@ -127,6 +127,11 @@ int test_fault_row(bool fp32) {
     return e != nullptr ? atoi(e) : -1;
 }
 
+int test_fault_barrier() {
+    const char* e = getenv("FUGAL_TEST_FAULT_BARRIER");
+    return e != nullptr ? atoi(e) : 0;
+}
+
 fugal_status allow_dynamic_smem(const void* fn, size_t bytes, const char* what) {
     static std::mutex mu;
     static std::map<std::pair<const void*, int>, int> limits;  // (function, device): bytes

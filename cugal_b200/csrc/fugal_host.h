@@ -49,6 +49,9 @@ int sm_count();
 // cost, FUGAL_TEST_FAULT_ROW_FP32 in the persistent kernels over FP32 rows.
 unsigned long long test_wait_limit_ns();
 int test_fault_row(bool fp32);
+// FUGAL_TEST_FAULT_BARRIER (unset: 0, none): the last CTA of the adjoint's solve takes its wait on this
+// barrier (counted from 1) as run out after it has arrived, so that the others may pass it.
+int test_fault_barrier();
 
 // Allow `fn` the largest dynamic shared memory the device gives a CTA next to its static arrays
 // (an error if `bytes` is more).  The limit belongs to the function, not to a launch, and launches

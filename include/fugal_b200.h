@@ -231,7 +231,7 @@ fugal_status fugal_sinkhorn_adjoint(const float* P, int64_t ldp, const float* G,
  * conjugate gradients from zero (all of it on the device, FP64 vectors), until the
  * residual is below tol * |[a; b]| or max_iter iterations.  info (DEVICE, 3
  * doubles): iterations, relative residual, status (FUGAL_OK or
- * FUGAL_DEVICE_TIMEOUT, alpha and beta then NaN).  No counterpart in the reference. */
+ * FUGAL_DEVICE_TIMEOUT, all the rest then NaN).  No counterpart in the reference. */
 #define FUGAL_ADJOINT_SOLVE_MAX_N 16384
 fugal_status fugal_sinkhorn_adjoint_solve_workspace_size(int64_t n, size_t* bytes);
 fugal_status fugal_sinkhorn_adjoint_solve(const float* P, int64_t ldp, int64_t n, const double* a, const double* b,

@@ -83,3 +83,27 @@ def test_16_bit_solve_after_fp32_sweeps_that_gave_up(unmet_copy):
     disarm()
     _, u1, v1 = SinkhornState(3000, cfg).solve(C)
     assert torch.equal(u0, u1) and torch.equal(v0, v1)
+
+
+@pytest.mark.parametrize("n", [100, 1000])
+@pytest.mark.parametrize("barrier", [1, 2, 3, 4, 7])
+def test_adjoint_solve(n, barrier, monkeypatch):
+    """The last CTA's wait on a barrier runs out (``FUGAL_TEST_FAULT_BARRIER``) after it has arrived.  An
+    iteration has three barriers, one comes before the first: with one iteration the fourth is the last, which
+    all other CTAs pass."""
+    from cugal_b200 import _native as N
+    from cugal_b200.autograd import sinkhorn_adjoint
+    P = torch.rand((n, n), generator=torch.Generator(device="cuda").manual_seed(n), device="cuda") / n
+    P += torch.eye(n, device="cuda") * 0.5
+    G = torch.rand((n, n), generator=torch.Generator(device="cuda").manual_seed(n + 1), device="cuda")
+    kw = dict(tol=0.0, max_iter=(barrier + 1) // 3)
+    dC, it, rel = sinkhorn_adjoint(P, G, 0.3, **kw)
+    assert it == kw["max_iter"] and dC.isfinite().all()
+    monkeypatch.setenv("FUGAL_TEST_FAULT_BARRIER", str(barrier))
+    monkeypatch.setenv("FUGAL_TEST_WAIT_LIMIT_NS", "1000000")
+    with pytest.raises(N.NativeError, match="device status 6"):
+        sinkhorn_adjoint(P, G, 0.3, **kw)
+    monkeypatch.delenv("FUGAL_TEST_FAULT_BARRIER")
+    monkeypatch.delenv("FUGAL_TEST_WAIT_LIMIT_NS")
+    again, _, _ = sinkhorn_adjoint(P, G, 0.3, **kw)
+    assert torch.equal(dC, again)
