@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kRowThreads) log_step_kernel(const float* K, l
         float piece = 0.f;
 #pragma unroll
         for (int q = 0; q < kRowThreads / 32; ++q) piece += sm_s[q];
-        S = (LONG && c0 > 0 && M != -INFINITY ? S * expf(M - base) : 0.f) + piece;
+        S = (LONG && c0 > 0 ? S * expf(M - base) : 0.f) + piece;  // (0 times 0 before any finite entry)
         M = Mp;
         if (LONG) __syncthreads();  // the next piece writes sm_m, sm_s
     }
