@@ -25,6 +25,7 @@ LAP_GREEDY, LAP_DOUBLE_GREEDY, LAP_PARALLEL_GREEDY, LAP_ORDERED = 0, 1, 2, 3
 KERNEL_FAMILY_NAMES = ["sweep16", "sweep32", "absorb", "finalize", "column_pass", "gradient", "update", "other"]
 MAX_RECORDED_ERRORS = 256
 ADJOINT_SOLVE_MAX_N = 16384
+STANDARD_ROWS_MAX_N = 16384
 
 STREAM_DTYPES = {None: FUGAL_F32, torch.float32: FUGAL_F32, torch.bfloat16: FUGAL_BF16, torch.float16: FUGAL_F16}
 

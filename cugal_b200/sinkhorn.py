@@ -177,8 +177,9 @@ class SinkhornState:
         N.require_cuda(C, "C")
         C32 = C.to(torch.float32).contiguous()
         n = C32.shape[0]
-        # the solve streams 16-byte rows; K itself is returned contiguous
-        rows = torch.empty((n, padded_ld(n)), dtype=torch.float32, device=C32.device)
+        # the persistent solve streams 16-byte rows; K itself is returned contiguous
+        ld = n if n % 4 == 0 or n > N.STANDARD_ROWS_MAX_N else padded_ld(n)
+        rows = torch.empty((n, ld), dtype=torch.float32, device=C32.device)
         exp_scale(C32, -1.0 / config.sinkhorn_regularization, rows)
         self._std.solve(rows, self.u_std, self.v_std, self._rec.data_ptr())
         K = rows[:, :n].contiguous()

@@ -199,7 +199,10 @@ fugal_status fugal_alignment_overlap(const int32_t* a_row_pointers, const int32_
  * fugal_solve_record.  If a bounded wait of the device runs out, the record's status is
  * FUGAL_DEVICE_TIMEOUT and u and v are NaN.  fugal_exp_scale writes out = exp(scale * C) (K from C with
  * scale = -1/reg); fugal_fw_update_standard is the update of cugal/pred.py:77-86
- * for this method: q = K v u, P += alpha (q - P), *gap = sum C (q - P) in FP64. */
+ * for this method: q = K v u, P += alpha (q - P), *gap = sum C (q - P) in FP64.
+ * Rows of up to FUGAL_STANDARD_ROWS_MAX_N columns on 16-byte boundaries (K, ldk, and n rounded
+ * up to 4 within ldk; the workspace too) take the faster of two forms. */
+#define FUGAL_STANDARD_ROWS_MAX_N 16384
 fugal_status fugal_sinkhorn_standard_workspace_size(int64_t n, size_t* bytes);
 fugal_status fugal_sinkhorn_standard_solve(const float* K, int64_t ldk, int64_t n, float* u, float* v,
                                            int max_iterations, double threshold, int eval_freq, int momentum_start,

@@ -25,3 +25,24 @@ def test_workspace_off_a_16_byte_boundary(n, offset):
         got.append((u, v))
     for a, b in zip(*got):
         assert torch.allclose(a, b, rtol=2e-5, atol=0)
+
+
+@pytest.mark.parametrize("n", [4, 7, 300, 2001, 16385])
+def test_solve_holds_k_once_where_its_rows_need_no_padding(n):
+    """Beside the cost a solve allocates K and, only where the persistent form needs 16-byte rows that K does not
+    have, one padded copy; K comes back contiguous."""
+    from cugal_b200.config import Config, SinkhornMethod
+    from cugal_b200.sinkhorn import SinkhornState
+    C = torch.rand((n, n), generator=torch.Generator(device="cuda").manual_seed(n), device="cuda")
+    state = SinkhornState(n, Config(device="cuda", dtype=torch.float32, sinkhorn_method=SinkhornMethod.STANDARD,
+                                    sinkhorn_regularization=0.5, sinkhorn_iterations=2))
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    K, _, _ = state.solve(C)
+    torch.cuda.synchronize()
+    peak = torch.cuda.max_memory_allocated() - before
+    copies = 2 if n % 4 and n <= 16384 else 1
+    assert peak <= copies * (n * (n + 7) * 4 + (1 << 21))  # torch rounds an allocation up by 2 MB at most
+    assert K.is_contiguous() and K.shape == (n, n)
+    assert torch.allclose(K, torch.exp(C * -2.0), rtol=1e-6, atol=0)
