@@ -99,6 +99,7 @@ SIGNATURES = {
     "fugal_sinkhorn_unrolled_step_backward": (_INT, [_P, _I64, _I64, _P, _P, _P, _INT, _P, _I64, _P, _P, _SZ, _P]),
     "fugal_sinkhorn_workspace_size": (_INT, [_I64, _INT, POINTER(c_size_t)]),
     "fugal_sinkhorn_plan_info": (_INT, [_I64, _INT, _P]),
+    "fugal_sinkhorn_sweep_kernel": (c_char_p, [_I64, _INT]),
     "fugal_sinkhorn_solve": (_INT, [POINTER(SolveParams), _P, _SZ, _P]),
     "fugal_gradient_column_chunks": (_INT, [_I64, POINTER(ctypes.c_int32)]),
     "fugal_fw_gradient_column_stats": (_INT, [_I64, _P, _P, _P, _P, _P, _I64, _P, _P, _P, _I64, _D, _D, _D, _P, _P,
@@ -201,7 +202,13 @@ def sinkhorn_plan(n: int, stream_dtype: int) -> dict:
     info = (ctypes.c_int32 * 6)()
     call("fugal_sinkhorn_plan_info", n, stream_dtype, ctypes.cast(info, c_void_p))
     keys = ["threads", "cluster", "clusters", "stages", "smem_bytes", "rows_per_batch"]
-    return dict(zip(keys, list(info)))
+    return dict(zip(keys, list(info)), kernel=sweep_kernel(n, stream_dtype))
+
+
+def sweep_kernel(n: int, stream_dtype: int) -> str | None:
+    """Name of the kernel that runs the sweeps for size n (None: bad arguments)."""
+    name = lib().fugal_sinkhorn_sweep_kernel(n, stream_dtype)
+    return None if name is None else name.decode()
 
 
 def launch_count() -> int:

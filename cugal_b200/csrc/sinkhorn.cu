@@ -1688,26 +1688,42 @@ extern "C" fugal_status fugal_sinkhorn_workspace_size(int64_t n, int stream_dtyp
     return FUGAL_OK;
 }
 
+namespace {
+// Which row-owned kernel runs the sweeps of a solve without a fixed order of sums (neither: the cluster kernel).
+fugal_status choose_row_owned(int64_t n, int stream_dtype, RowsPlan& rows, RowPlan& rp) {
+    if (stream_dtype == FUGAL_F32 ? getenv("FUGAL_SWEEP_SHAPE") == nullptr : row_sweep_on())
+        FUGAL_TRY(make_rows_plan(n, stream_dtype, rows, false));
+    if (!rows.use && row_sweep_on())
+        FUGAL_TRY(make_row_plan(n, stream_dtype, static_cast<int64_t>(align_up(static_cast<size_t>(n), 64)), rp, false));
+    return FUGAL_OK;
+}
+}  // namespace
+
+extern "C" const char* fugal_sinkhorn_sweep_kernel(int64_t n, int stream_dtype) {
+    RowsPlan rows;
+    RowPlan rp;
+    if (n <= 0 || stream_dtype < FUGAL_F32 || stream_dtype > FUGAL_F16 ||
+        choose_row_owned(n, stream_dtype, rows, rp) != FUGAL_OK)
+        return nullptr;
+    return rows.use ? "rows_kernel" : (rp.use ? "row_sweep_kernel" : "sweep_kernel");
+}
+
 extern "C" fugal_status fugal_sinkhorn_plan_info(int64_t n, int stream_dtype, int32_t* info) {
     if (info == nullptr) return fail(FUGAL_BAD_ARGUMENT, "fugal_sinkhorn_plan_info: null output");
     if (stream_dtype < FUGAL_F32 || stream_dtype > FUGAL_F16)
         return fail(FUGAL_BAD_ARGUMENT, "fugal_sinkhorn_plan_info: bad stream dtype");
-    if (stream_dtype == FUGAL_F32 ? getenv("FUGAL_SWEEP_SHAPE") == nullptr : row_sweep_on()) {
-        RowsPlan rows;
-        FUGAL_TRY(make_rows_plan(n, stream_dtype, rows, false));
-        if (rows.use) {  // row-owned persistent sweeps: one CTA per SM, no cluster
-            info[0] = 512;
-            info[1] = 1;
-            info[2] = rows.ctas;
-            info[3] = rows.stages;
-            info[4] = static_cast<int32_t>(rows.smem);
-            info[5] = rows.streams;
-            return FUGAL_OK;
-        }
-    }
+    RowsPlan rows;
     RowPlan rp;
-    if (row_sweep_on())
-        FUGAL_TRY(make_row_plan(n, stream_dtype, static_cast<int64_t>(align_up(static_cast<size_t>(n), 64)), rp, false));
+    FUGAL_TRY(choose_row_owned(n, stream_dtype, rows, rp));
+    if (rows.use) {  // row-owned persistent sweeps: one CTA per SM, no cluster
+        info[0] = 512;
+        info[1] = 1;
+        info[2] = rows.ctas;
+        info[3] = rows.stages;
+        info[4] = static_cast<int32_t>(rows.smem);
+        info[5] = rows.streams;
+        return FUGAL_OK;
+    }
     if (rp.use) {  // row-owned sweep: one CTA per SM, no cluster
         info[0] = rp.threads;
         info[1] = rp.cl;

@@ -377,6 +377,9 @@ fugal_status fugal_sinkhorn_workspace_size(int64_t n, int stream_dtype, size_t* 
  * current device: info = {threads per CTA, CTAs per cluster, clusters in the
  * grid, pipeline stages, dynamic shared memory bytes, rows per batch}. */
 fugal_status fugal_sinkhorn_plan_info(int64_t n, int stream_dtype, int32_t* info);
+/* The kernel of those sweeps: "rows_kernel" (persistent, row-owned), "row_sweep_kernel"
+ * (row-owned, a launch per sweep) or "sweep_kernel" (clusters); NULL for bad arguments. */
+const char* fugal_sinkhorn_sweep_kernel(int64_t n, int stream_dtype);
 fugal_status fugal_sinkhorn_solve(const fugal_solve_params* params, void* workspace, size_t workspace_bytes,
                                   fugal_stream_t stream);
 
