@@ -1712,6 +1712,7 @@ extern "C" fugal_status fugal_sinkhorn_plan_info(int64_t n, int stream_dtype, in
     if (info == nullptr) return fail(FUGAL_BAD_ARGUMENT, "fugal_sinkhorn_plan_info: null output");
     if (stream_dtype < FUGAL_F32 || stream_dtype > FUGAL_F16)
         return fail(FUGAL_BAD_ARGUMENT, "fugal_sinkhorn_plan_info: bad stream dtype");
+    if (n <= 0) return fail(FUGAL_BAD_SHAPE, "fugal_sinkhorn_plan_info: n must be positive");
     RowsPlan rows;
     RowPlan rp;
     FUGAL_TRY(choose_row_owned(n, stream_dtype, rows, rp));

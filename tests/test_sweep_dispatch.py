@@ -24,3 +24,10 @@ def test_environment_and_bad_arguments(monkeypatch):
     assert N.sweep_kernel(300, N.FUGAL_F32) == "rows_kernel"
     monkeypatch.setenv("FUGAL_SWEEP_SHAPE", "256x16")  # a shape of the cluster kernel asked for by name
     assert N.sweep_kernel(300, N.FUGAL_F32) == "sweep_kernel"
+
+
+@pytest.mark.parametrize("dtype", [N.FUGAL_F32, N.FUGAL_BF16, N.FUGAL_F16])
+@pytest.mark.parametrize("n", [0, -1])
+def test_plan_info_refuses_sizes_below_one(n, dtype):
+    with pytest.raises(N.NativeError, match="bad shape"):
+        N.sinkhorn_plan(n, dtype)
