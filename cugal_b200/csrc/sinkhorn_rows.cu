@@ -576,7 +576,6 @@ fugal_status make_rows_plan(int64_t n, int dt, RowsPlan& pl, bool device) {
     pl.ctas = static_cast<int>((n + pl.rows_per_cta - 1) / pl.rows_per_cta);
     const size_t stage = static_cast<size_t>(kRowsThreads / pl.streams) * pl.ept * es;
     const size_t dump = rows_dump_bytes(pl.streams, pl.ept);
-    pl.parts = pl.ctas;
     const size_t room = 227 * 1024 - kRowsStatic - dump;
     pl.stages = static_cast<int>(std::min<size_t>({room / stage, static_cast<size_t>(kRowsMaxStages),
                                                    static_cast<size_t>(pl.rows_per_cta)}));

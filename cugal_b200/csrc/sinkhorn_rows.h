@@ -29,7 +29,7 @@ struct RowsArgs {
     float* logcs;          // log column sums of the previous sweep
     float* b_next;         // b - log colsum: the next sweep's column duals without momentum
     float* a;              // row duals
-    float* partials;       // [CTAs or streams][n_pad]
+    float* partials;       // [CTAs][n_pad]
     double* errs;          // [CTAs] column error of a sweep
     float* corrs;          // [CTAs] largest |column correction|
     long long n_pad;
@@ -46,12 +46,11 @@ struct RowsPlan {
     int dt = 0;
     int ept = 0;           // columns per thread
     int streams = 0;       // row streams (groups of warps) per CTA
-    int ctas = 0;
+    int ctas = 0;          // each writes one row of column partials
     int rows_per_cta = 0;
     int stages = 0;
     int resident = 0;
     size_t smem = 0;
-    int parts = 0;         // rows of column partials a launch writes
 };
 
 // Plan for n columns of element type dt (FUGAL_F32, FUGAL_BF16, FUGAL_F16);
