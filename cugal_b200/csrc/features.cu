@@ -31,15 +31,24 @@ __device__ __forceinline__ int lower_bound(const int* __restrict__ col, int lo, 
     return lo;
 }
 
+// Vertices of up to this degree have counts below 2^32: a list of d entries meets d others, each in
+// at most d places.
+constexpr int kMaxDegree32 = 65535;
+
+__global__ void __launch_bounds__(256) clear_counts_kernel(int n, unsigned* tri, unsigned* carry) {
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) tri[v] = carry[v] = 0u;
+}
+
 // Adds to tri[v] the common neighbours of the edges (v, u) of one chunk of 32 edges.
-// Count: 64-bit counts (long long) or, where they cannot overflow, 32-bit ones.  Lists
+// Count: 64-bit counts (long long), or 32-bit ones with the wraps of rows longer than
+// kMaxDegree32 (parallel edges: a simple graph of 65536 vertices has none) in `carry`.  Lists
 // of up to 32 entries are intersected in registers (five shuffles a binary search);
 // longer ones are searched in memory by lanes that share the shorter list.  One warp
 // per vertex, lanes over its neighbours, left a power-law graph's hubs to single
 // warps: 904 us at 65536 vertices of mean degree 16.
 template <typename Count>
 __global__ void __launch_bounds__(256) triangle_kernel(const int* __restrict__ col, const int* __restrict__ rp, int n,
-                                                       Count* tri) {
+                                                       Count* tri, unsigned* carry) {
     const int lane = threadIdx.x & 31;
     const int nnz = rp[n];
     const long long chunk = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -89,18 +98,27 @@ __global__ void __launch_bounds__(256) triangle_kernel(const int* __restrict__ c
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
-            if (lane == 0 && count) atomicAdd(&tri[v], count);
+            if (lane == 0 && count) {
+                if (sizeof(Count) == 8 || d <= kMaxDegree32) {
+                    atomicAdd(&tri[v], count);
+                } else if (atomicAdd(&tri[v], count) > ~count) {
+                    atomicAdd(&carry[v], 1u);
+                }
+            }
             ++v;
         }
     }
 }
 
+// 32-bit counts lie in clustering, their carries in degrees (read as the floats that they are
+// overwritten with, so that the compiler keeps the order).
 template <typename Count>
 __global__ void clustering_kernel(const int* __restrict__ rp, int n, const Count* tri, float* clustering,
                                   float* degrees, int* degree_counts) {
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const int d = rp[v + 1] - rp[v];
-        const long long t = static_cast<long long>(tri[v]);
+        long long t = static_cast<long long>(tri[v]);
+        if (sizeof(Count) == 4 && d > kMaxDegree32) t += static_cast<long long>(__float_as_uint(degrees[v])) << 32;
         degrees[v] = static_cast<float>(d);
         if (degree_counts) degree_counts[v] = d;
         const float denom = static_cast<float>(static_cast<long long>(d) * (d - 1));
@@ -330,15 +348,15 @@ extern "C" fugal_status fugal_graph_features(const int32_t* col_indices, const i
     const int blocks = static_cast<int>(std::min<int64_t>((n * 32 + threads - 1) / threads, 32 * sm_count()));
     const int vec_blocks = static_cast<int>(std::min<int64_t>((n + threads - 1) / threads, 8 * sm_count()));
     const int chunk_blocks = static_cast<int>(std::min<int64_t>((n + 15) / 16 + 1, 16 * sm_count()));
-    // A count is at most d (d - 1) < n^2: with up to 65536 vertices it fits the 32 bits of
-    // a clustering entry, which holds it until the ratio is formed.
+    // Up to 65536 vertices a count is kept in 32 bits, in the vertex's clustering entry, until the
+    // ratio is formed, and what does not fit them in its degree entry.
     if (triangle_counts != nullptr) {
         long long* tri = reinterpret_cast<long long*>(triangle_counts);
         FUGAL_TRY(cuda_check(cudaMemsetAsync(tri, 0, static_cast<size_t>(n) * 8, stream), "fugal_graph_features"));
         {
             LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
             triangle_kernel<unsigned long long><<<chunk_blocks, threads, 0, stream>>>(
-                col_indices, row_pointers, ni, reinterpret_cast<unsigned long long*>(tri));
+                col_indices, row_pointers, ni, reinterpret_cast<unsigned long long*>(tri), nullptr);
             FUGAL_TRY(launch_check("fugal_graph_features: triangles"));
         }
         LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
@@ -348,10 +366,15 @@ extern "C" fugal_status fugal_graph_features(const int32_t* col_indices, const i
     }
     if (n <= 65536) {
         unsigned* tri = reinterpret_cast<unsigned*>(clustering);
-        FUGAL_TRY(cuda_check(cudaMemsetAsync(tri, 0, static_cast<size_t>(n) * 4, stream), "fugal_graph_features"));
+        unsigned* carry = reinterpret_cast<unsigned*>(degrees);
         {
             LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
-            triangle_kernel<unsigned><<<chunk_blocks, threads, 0, stream>>>(col_indices, row_pointers, ni, tri);
+            clear_counts_kernel<<<vec_blocks, threads, 0, stream>>>(ni, tri, carry);
+            FUGAL_TRY(launch_check("fugal_graph_features: clear"));
+        }
+        {
+            LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
+            triangle_kernel<unsigned><<<chunk_blocks, threads, 0, stream>>>(col_indices, row_pointers, ni, tri, carry);
             FUGAL_TRY(launch_check("fugal_graph_features: triangles"));
         }
         LaunchScope scope(FUGAL_KERNEL_OTHER, stream);
