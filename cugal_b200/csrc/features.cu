@@ -200,9 +200,9 @@ __global__ void count_rows_kernel(const int* edges, long long m, int n, int* cou
     }
 }
 
-// Exclusive scan of counts[0..n) into rp[0..n], 1024 counts per block; a block first
-// adds up all counts before its own (up to kScanBlocks blocks: at most 1 MB each, read
-// by all SMs at once).  51 us at n = 65536 when one block walked all counts.
+// Exclusive scan of counts[0..n) into rp[0..n], 1024 counts per block (more above 262144); a
+// block first adds up all counts before its own, 4 n bytes at most, read by all SMs at once.
+// 7 us at n = 65536, 51 when one block walked all counts.
 constexpr int kScanBlocks = 256;
 
 // Inclusive scan of one value per thread over a 1024-thread block; returns the block's total in `total`.

@@ -313,7 +313,6 @@ FUGAL_DEVICE void tmem_relinquish() {
 FUGAL_DEVICE void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// Ordering of tensor-memory operations around a thread barrier.
 // Programmatic dependent launch: the next kernel of the stream, if launched so, may start
 // once all blocks have called `launch_dependents` (or ended); its blocks read what this
 // kernel writes only after `wait_for_previous`, which returns when the previous kernel of
@@ -321,6 +320,8 @@ FUGAL_DEVICE void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 // ends of the kernels of such a chain stay in order.
 FUGAL_DEVICE void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 FUGAL_DEVICE void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Ordering of tensor-memory operations around a thread barrier, and of loads after stores of the
+// same thread (tmem_wait_st; nothing else orders those).
 FUGAL_DEVICE void tmem_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 FUGAL_DEVICE void tmem_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 FUGAL_DEVICE void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }

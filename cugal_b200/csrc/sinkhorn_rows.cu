@@ -539,7 +539,8 @@ RowsFn rows_fn(const RowsPlan& pl) {
 // n = 8192 41.1 us as {4, 64}, 51.2 as {2, 32}; n = 6000 28.2 as {4, 48}, 39.1 as
 // {2, 32}; n = 4096 18.6 as {4, 32}, 25.5 as {8, 64}.  FP32 rows of 6145 to 8192
 // columns take two streams, so that two stages of 32 KB are left for each.  Wider
-// rows: FP32 sweeps are at 85% of the copy peak in the cluster kernel; 16-bit ones of
+// rows: FP32 sweeps stay with the cluster kernel (an iteration takes 107 us at n = 8193, 145 at
+// 12000, 190 at 16384, 800 at 32768: 38, 61, 87 and 82% of the copy peak); 16-bit ones of
 // more than 24576 columns have too few stages left here (469 against 454 us at 32768).
 struct RowsShape {
     int streams, ept;

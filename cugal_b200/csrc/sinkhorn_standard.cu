@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(kStdThreads) std_update_kernel(float* P, long 
 // ------------------------------------------------------------- persistent form
 
 // Per iteration: one read of K (144 MB at n = 6000, 22 us at the copy peak) where the
-// four launches of the wider form read it twice (31 + 49 us) and paid their gaps: 92 us
+// four launches of the other form read it twice (31 + 49 us) and paid their gaps: 101 us
 // against 40 us an iteration at n = 6000.
 struct StdRowsArgs {
     const float* K;

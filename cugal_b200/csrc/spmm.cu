@@ -602,7 +602,9 @@ __global__ void __launch_bounds__(kStructThreads, 4) gradient_structural_kernel(
 // and one shared-memory access of 4 R bytes serve R outputs, each summed in CSR order.
 // With one row of Q per block and its values gathered from L1 the column indices were
 // read once per output row: 3.32 ms at n = 8192, mean degree 12, against 0.28 ms for
-// the other operand layout.  R = 4 up to 14000 columns, 2 and 1 up to 57000, by what
+// the other operand layout; 0.63 ms here, bound by the L1 / shared-memory data pipe (81% of its
+// peak: the gathers, two wavefronts in five of them bank conflicts, and the lanes' own column
+// indices).  R = 4 up to 14000 columns, 2 and 1 up to 57000, by what
 // shared memory holds; wider rows gather from global memory.
 constexpr int kTransposedThreads = 1024;
 template <int R>

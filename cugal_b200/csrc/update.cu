@@ -253,7 +253,7 @@ FUGAL_DEVICE float4 row_quad(const float* row, int k, int cols, float fill) {
 // One block per row, the row read once: QUADS float4 per thread stay in registers
 // between the maximum and the exponentials (rows up to
 // 8192), and longer rows (LONG) keep a running (max, sum) over pieces of 8192.
-// Bound by HBM: 172 us with two scalar passes over a row, 57 us here at n = 8192 (268
+// Bound by HBM: 172 us with two scalar passes over a row, 52 us here at n = 8192 (268
 // MB, 41 us at the copy peak).
 template <int QUADS, bool VEC, bool LONG>
 __global__ void __launch_bounds__(kRowThreads) log_step_kernel(const float* K, long long ldk, int cols,

@@ -375,7 +375,8 @@ typedef struct {
 fugal_status fugal_sinkhorn_workspace_size(int64_t n, int stream_dtype, size_t* bytes);
 /* Launch shape of the sweeps over an n-column cost of stream_dtype on the
  * current device: info = {threads per CTA, CTAs per cluster, clusters in the
- * grid, pipeline stages, dynamic shared memory bytes, rows per batch}. */
+ * grid, pipeline stages, dynamic shared memory bytes, rows per batch (the persistent
+ * kernel: row streams of a CTA)}. */
 fugal_status fugal_sinkhorn_plan_info(int64_t n, int stream_dtype, int32_t* info);
 /* The kernel of those sweeps: "rows_kernel" (persistent, row-owned), "row_sweep_kernel"
  * (row-owned, a launch per sweep) or "sweep_kernel" (clusters); NULL for bad arguments. */
