@@ -264,9 +264,11 @@ FUGAL_DEVICE double warp_sum8(const double (&v)[8]) {
     return w;
 }
 
-// The sum of one value per CTA, the same in every thread of every CTA.
-FUGAL_DEVICE double grid_total(const double* per_cta, double* scratch) {
-    __syncthreads();  // scratch is free
+// The sum of one value per CTA, the same in every thread of every CTA.  (`total` is not the scratch
+// of a block_sum: the first warp of one that follows would write it under a slower warp's read.)
+FUGAL_DEVICE double grid_total(const double* per_cta) {
+    __shared__ double total;
+    __syncthreads();  // the total before has been read
     if (threadIdx.x < 32) {
         double s = 0.0;
         const int ctas = static_cast<int>(gridDim.x);
@@ -278,10 +280,10 @@ FUGAL_DEVICE double grid_total(const double* per_cta, double* scratch) {
             for (int u = 0; u < 8; ++u) s += v[u];
         }
         s = warp_sum(s);
-        if (threadIdx.x == 0) scratch[0] = s;
+        if (threadIdx.x == 0) total = s;
     }
     __syncthreads();
-    return scratch[0];
+    return total;
 }
 
 template <bool VEC>
@@ -321,7 +323,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_kernel(const __grid_constant
     rr = block_sum(rr, scratch);
     if (tid == 0) p.dots[blockIdx.x] = rr;
     if (!barrier()) return;
-    double rs = grid_total(p.dots, scratch);
+    double rs = grid_total(p.dots);
     const double norm = sqrt(rs);
     double rel = 0.0;
     int it = 0;
@@ -411,7 +413,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_kernel(const __grid_constant
             dot = block_sum(dot, scratch);
             if (tid == 0) p.dots[gridDim.x + blockIdx.x] = dot;
             if (!barrier()) return;
-            const double step = rs / grid_total(p.dots + gridDim.x, scratch);
+            const double step = rs / grid_total(p.dots + gridDim.x);
             // ---- solution and residual
             rr = 0.0;
             for (int k = tid; k < own; k += kCgThreads) {
@@ -426,7 +428,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_kernel(const __grid_constant
             rr = block_sum(rr, scratch);
             if (tid == 0) p.dots[blockIdx.x] = rr;
             if (!barrier()) return;
-            const double rs_new = grid_total(p.dots, scratch);
+            const double rs_new = grid_total(p.dots);
             rel = sqrt(rs_new) / norm;
             if (rel < p.tol) break;
             const double ratio = rs_new / rs;
