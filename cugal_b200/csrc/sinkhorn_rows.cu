@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
                 if (gt == 0 && ubase + r + NST < units) {
                     int row = r + ahead;
                     if (row >= nrows) row -= nrows;
+                    fence_proxy_async_smem();  // the reads of the stage precede the copy into it
                     issue(row, s, ph ^ 1u, false);
                 }
             };

@@ -482,6 +482,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) std_rows_kernel(const __grid_
             if (gt == 0 && !p.resident) {
                 int row = r + ahead;
                 if (row >= nrows) row -= nrows;
+                fence_proxy_async_smem();  // the reads of the stage precede the copy into it
                 issue(row, s, ph ^ 1u, false);
             }
             if (t == 0) {
